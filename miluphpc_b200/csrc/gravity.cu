@@ -22,67 +22,263 @@ constexpr int kWalkBlock = 128;
 // pushed as a node by the reference and contributes nothing, which is kept.
 // r is formed with explicitly rounded products and sums like the
 // reference's -fmad=false build so that accept decisions match it exactly.
-__global__ void __launch_bounds__(kWalkBlock) k_grav_v2(const double4* __restrict__ com, const int2* __restrict__ link,
-                                                        const int* __restrict__ nodes_total, GravParams P,
-                                                        const double* __restrict__ sx, const double* __restrict__ sy,
-                                                        const double* __restrict__ sz, const double* __restrict__ sh,
-                                                        const int* __restrict__ perm, double* __restrict__ gax,
-                                                        double* __restrict__ gay, double* __restrict__ gaz,
-                                                        DevStatus* st) {
-    if (st->code) return;
-    const int M = *nodes_total;
-    const int lane = threadIdx.x & 31;
-    const long gwarp = ((long)blockIdx.x * kWalkBlock + threadIdx.x) >> 5;
-    const long ngroups = ((long)P.n + 31) >> 5;
-    if (gwarp >= ngroups) return;
-    const long s = gwarp * 32 + lane;
-    const bool valid = s < P.n;
-    double px = 0, py = 0, pz = 0, e2 = P.eps2;
-    if (valid) {
-        px = __ldg(sx + s); py = __ldg(sy + s); pz = __ldg(sz + s);
-        if (P.h_factor > 0.0) { double e = P.h_factor * __ldg(sh + s); e2 += e * e; }
+//
+// A block of W warps per 32 sorted particles (the reference's groups).  The
+// traversal is lane-parallel: a step pops up to 32 W nodes from a stack in
+// shared memory, one per thread, so their records arrive in one round trip (a
+// walk that takes one node at a time waits for each: 620-670 ns a node).  Most
+// cells are decided by their thread alone from the group's bounding box in
+// FP32 with a margin above its rounding (nearest point of the box farther
+// than dp: every particle accepts; farthest point nearer: every particle
+// refuses); the others are put to the exact vote of the 32 particles, spread
+// over the warps.  So the decisions, and the set of interactions, are those
+// of the reference's walk; only their order differs.  Accepted nodes go to a
+// list in shared memory; every warp holds the same 32 particles and evaluates
+// every W-th entry in FP64, and the warps' sums are added at the end.  The
+// stack bound is the list walk's (below): a pop of k nodes pushes at most 8k,
+// and k leaves room for a depth-first descent.
+// Bound: FP64 pipe (20 instructions an entry and warp) and, below ~500
+// groups, the round trips of the traversal.  Walk in us, Plummer theta 0.5:
+//   n                  1,000  4,000  20,011  50,000  131,072  300,000  1,000,000
+//   one node at a time   190               262               800
+//   W = 1                 93    170     223     267      418      793       2326
+//   W = 2                 58     98     134     177      369      748       2347
+//   W = 4                 38     57      84     161      352      772       2547
+//   W = 8                 31     40      89     176      436      989       3400
+__host__ __device__ constexpr int v2_stack(int W) { return 512 + 256 * (W - 1); }
+constexpr int kV2Reserve = 7 * 22 + 8;
+
+template <int W>
+struct V2Smem {
+    double2 la[64 * W], lb[64 * W];  // accepted: (x, y), (z, m)
+    double2 ua[32 * W], ub[32 * W];  // put to the vote: (x, y), (z, dp)
+    double part[W][3][32];           // the warps' sums
+    int stk[v2_stack(W)];
+    int defer[32 * W];
+    int cnt[W][4];                   // per warp: accepted, children, votes, buckets
+    unsigned char yes[32 * W];
+    int top;
+};
+
+// every W-th entry of the list from entry w on
+template <int W>
+__device__ __forceinline__ void eval_v2(const V2Smem<W>& S, int w, int count, double px, double py, double pz,
+                                        double e2, double& ax, double& ay, double& az) {
+#pragma unroll 4
+    for (int e = w; e < count; e += W) {
+        const double2 a = S.la[e], b = S.lb[e];
+        const double dx = a.x - px, dy = a.y - py, dz = b.x - pz;
+        const double r = fma(dx, dx, fma(dy, dy, fma(dz, dz, e2)));
+        const double ri = r > 0.0 ? rsqrt(r) : 0.0;
+        const double f = b.y * ri * (ri * ri);
+        ax = fma(f, dx, ax); ay = fma(f, dy, ay); az = fma(f, dz, az);
     }
+}
+
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, const double* __restrict__ sx,
+                                                    const double* __restrict__ sy, const double* __restrict__ sz,
+                                                    const double* __restrict__ sh, const int* __restrict__ perm,
+                                                    double* __restrict__ gax, double* __restrict__ gay,
+                                                    double* __restrict__ gaz, DevStatus* st) {
+    extern __shared__ __align__(16) unsigned char v2_raw[];
+    V2Smem<W>& S = *reinterpret_cast<V2Smem<W>*>(v2_raw);
+    if (__syncthreads_or(st->code)) return;
+    const int M = *T.nodes;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const long s = (long)blockIdx.x * 32 + lane;
+    const bool valid = s < P.n;
+    const long sl = valid ? s : (long)P.n - 1;
+    const double px = __ldg(sx + sl), py = __ldg(sy + sl), pz = __ldg(sz + sl);
+    double e2 = P.eps2;
+    if (P.h_factor > 0.0) { double e = P.h_factor * __ldg(sh + sl); e2 += e * e; }
+    // bounding box of the group: centre in FP64, half edges and the largest
+    // softening in FP32 rounded up
+    double lox = px, loy = py, loz = pz, hix = px, hiy = py, hiz = pz, emax = e2;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lox = fmin(lox, __shfl_xor_sync(MHPC_FULL, lox, o));
+        loy = fmin(loy, __shfl_xor_sync(MHPC_FULL, loy, o));
+        loz = fmin(loz, __shfl_xor_sync(MHPC_FULL, loz, o));
+        hix = fmax(hix, __shfl_xor_sync(MHPC_FULL, hix, o));
+        hiy = fmax(hiy, __shfl_xor_sync(MHPC_FULL, hiy, o));
+        hiz = fmax(hiz, __shfl_xor_sync(MHPC_FULL, hiz, o));
+        emax = fmax(emax, __shfl_xor_sync(MHPC_FULL, emax, o));
+    }
+    const double cx = 0.5 * (lox + hix), cy = 0.5 * (loy + hiy), cz = 0.5 * (loz + hiz);
+    // the margin of 1e-6 is several times the FP32 roundings of the offsets and
+    // squares below (a few 2^-24 each)
+    constexpr float kUp = 1.f + 1e-6f, kDown = 1.f - 1e-6f;
+    const float bx = kUp * (float)fmax(hix - cx, cx - lox), by = kUp * (float)fmax(hiy - cy, cy - loy),
+                bz = kUp * (float)fmax(hiz - cz, cz - loz), ef = kUp * (float)emax;
     // dp(L) = (radius^2 / theta) * 0.25^(L-1); powers of two scale exactly,
     // so this equals the reference's repeated 0.25 * depth products.
     const double radius = 0.5 * (ord_to_dbl(P.ord[1]) - ord_to_dbl(P.ord[0]));
     const double depth1 = radius * radius / P.theta;
     double ax = 0, ay = 0, az = 0;
     unsigned long long ninter = 0, nvisit = 0;
-    int nd = 0;
-    while (nd < M) {
-        const int2 lk = __ldg(link + nd);
-        const int L = lk.y & 0xff;
-        const bool leaf = lk.y & ND_LEAF;
-        ++nvisit;
-        if (L == 1) {  // root child
-            nd = leaf ? lk.x : nd + 1;
-            continue;
-        }
-        const double4 c = ldg_d4(com + nd);
-        const double dx = c.x - px, dy = c.y - py, dz = c.z - pz;
-        double r = __dadd_rn(__dmul_rn(dx, dx), e2);
-        r = __dadd_rn(r, __dmul_rn(dy, dy));
-        r = __dadd_rn(r, __dmul_rn(dz, dz));
-        bool acc = leaf;
-        if (!leaf) acc = __all_sync(MHPC_FULL, !valid || ldexp(depth1, -2 * (L - 1)) <= r);
-        if (acc) {
-            double f = 0.0;
-            if (r > 0.0) {
-                const double ri = rsqrt(r);
-                f = c.w * ri * ri * ri;
+    // the root's children: node 0 and its skip chain
+    if (threadIdx.x == 0) {
+        int c = 0, q = 0;
+        while (c < M && q < 8) { S.stk[q++] = c; c = __ldg(&T.link[c].x); }
+        if (c < M) set_status(st, MHPC_ERR_DEPTH, 9);
+        S.top = q;
+    }
+    __syncthreads();
+    int top = S.top, nlist = 0;  // block-uniform
+    while (top > 0) {
+        const int room = (v2_stack(W) - kV2Reserve - top) / 7;
+        int k = top < 32 * W ? top : 32 * W;
+        if (k > room) k = room > 1 ? room : 1;
+        const bool act = (int)threadIdx.x < k;
+        const int nd = act ? S.stk[top - 1 - threadIdx.x] : 0;
+        top -= k;
+        nvisit += k;
+        bool acc = false, open = false, vote = false;
+        double4 c = make_double4(0, 0, 0, 0);
+        double dp = 0;
+        int mask = 0;
+        if (act) {
+            const int2 lk = __ldg(T.link + nd);
+            c = ldg_d4(T.com + nd);
+            mask = __ldg(T.kmask + nd);
+            const int L = lk.y & 0xff;
+            if (lk.y & ND_LEAF) {
+                acc = L > 1;
+            } else if (L == 1) {
+                open = true;
+            } else {
+                dp = depth1 * __longlong_as_double((long long)(1023 - 2 * (L - 1)) << 52);
+                const float nx = fabsf((float)(c.x - cx)), ny = fabsf((float)(c.y - cy)), nz = fabsf((float)(c.z - cz));
+                const float x0 = fmaxf(fmaf(kDown, nx, -bx), 0.f), x1 = fmaf(kUp, nx, bx);
+                const float y0 = fmaxf(fmaf(kDown, ny, -by), 0.f), y1 = fmaf(kUp, ny, by);
+                const float z0 = fmaxf(fmaf(kDown, nz, -bz), 0.f), z1 = fmaf(kUp, nz, bz);
+                const float near2 = fmaf(x0, x0, fmaf(y0, y0, z0 * z0));
+                const float far2 = fmaf(x1, x1, fmaf(y1, y1, fmaf(z1, z1, ef)));
+                acc = near2 * kDown > __double2float_ru(dp);
+                open = far2 * kUp < __double2float_rd(dp);
+                vote = !acc && !open;
             }
-            ax += f * dx; ay += f * dy; az += f * dz;
-            ++ninter;
-            nd = lk.x;
-        } else {
-            ++nd;
+        }
+        const unsigned bv = __ballot_sync(MHPC_FULL, vote);
+        if (lane == 0) S.cnt[w][2] = __popc(bv);
+        __syncthreads();
+        int vbase = 0, nvote = 0;
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            if (q == w) vbase = nvote;
+            nvote += S.cnt[q][2];
+        }
+        if (nvote) {
+            const int mine = vbase + __popc(bv & lt);
+            if (vote) {
+                S.ua[mine] = make_double2(c.x, c.y);
+                S.ub[mine] = make_double2(c.z, dp);
+            }
+            __syncthreads();
+#pragma unroll 2
+            for (int i = w; i < nvote; i += W) {
+                const double2 a = S.ua[i], b = S.ub[i];
+                const double dx = a.x - px, dy = a.y - py, dz = b.x - pz;
+                double r = __dadd_rn(__dmul_rn(dx, dx), e2);
+                r = __dadd_rn(r, __dmul_rn(dy, dy));
+                r = __dadd_rn(r, __dmul_rn(dz, dz));
+                const int all = __all_sync(MHPC_FULL, !valid || b.y <= r);
+                if (lane == 0) S.yes[i] = (unsigned char)all;
+            }
+            __syncthreads();
+            if (vote) {
+                acc = S.yes[mine] != 0;
+                open = !acc;
+            }
+        }
+        // accepted nodes to the list, opened cells' children to the stack;
+        // shared-key buckets wait (their children have no slots)
+        const unsigned ba = __ballot_sync(MHPC_FULL, acc);
+        const bool bucket = open && (mask & 0x100);
+        const unsigned bb = __ballot_sync(MHPC_FULL, bucket);
+        const int nkid = (open && !bucket) ? __popc(mask & 0xff) : 0;
+        int incl = nkid;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(MHPC_FULL, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) { S.cnt[w][0] = __popc(ba); S.cnt[w][1] = incl; S.cnt[w][3] = __popc(bb); }
+        __syncthreads();
+        int nacc = 0, total = 0, ndefer = 0, abase = 0, kbase = 0, dbase = 0;
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            if (q == w) { abase = nacc; kbase = total; dbase = ndefer; }
+            nacc += S.cnt[q][0]; total += S.cnt[q][1]; ndefer += S.cnt[q][3];
+        }
+        if (acc) {
+            const int i = nlist + abase + __popc(ba & lt);
+            S.la[i] = make_double2(c.x, c.y);
+            S.lb[i] = make_double2(c.z, c.w);
+        }
+        if (bucket) S.defer[dbase + __popc(bb & lt)] = nd;
+        nlist += nacc;
+        if (top + total > v2_stack(W)) {
+            // unreachable by the bound on k; stop instead of overrunning
+            if (threadIdx.x == 0) set_status(st, MHPC_ERR_DEPTH, 10);
+            return;
+        }
+        if (nkid) {
+            const int4 k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
+            const int4 k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
+            const int all[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+            int pos = top + kbase + incl - nkid;
+#pragma unroll
+            for (int d = 0; d < 8; ++d)
+                if ((mask >> d) & 1) S.stk[pos++] = all[d];
+        }
+        top += total;
+        __syncthreads();
+        // (the list holds at most 64 W entries: fewer than 32 W before a step)
+        if (nlist >= 32 * W) {
+            eval_v2<W>(S, w, nlist, px, py, pz, e2, ax, ay, az);
+            ninter += nlist;
+            nlist = 0;
+            __syncthreads();
+        }
+        // shared-key buckets: their children are consecutive leaves
+        for (int d = 0; d < ndefer; ++d) {
+            const int b = S.defer[d];
+            const int end = __ldg(&T.link[b].x);
+            for (int c0 = b + 1; c0 < end; c0 += 32 * W) {
+                const int l = c0 + (int)threadIdx.x;
+                if (l < end) {
+                    const double4 q = ldg_d4(T.com + l);
+                    S.la[nlist + threadIdx.x] = make_double2(q.x, q.y);
+                    S.lb[nlist + threadIdx.x] = make_double2(q.z, q.w);
+                }
+                const int got = min(32 * W, end - c0);
+                nlist += got;
+                nvisit += got;
+                __syncthreads();
+                if (nlist >= 32 * W) {
+                    eval_v2<W>(S, w, nlist, px, py, pz, e2, ax, ay, az);
+                    ninter += nlist;
+                    nlist = 0;
+                    __syncthreads();
+                }
+            }
         }
     }
+    eval_v2<W>(S, w, nlist, px, py, pz, e2, ax, ay, az);
+    ninter += nlist;
+    S.part[w][0][lane] = ax; S.part[w][1][lane] = ay; S.part[w][2][lane] = az;
+    __syncthreads();
+    if (w > 0) return;
+#pragma unroll
+    for (int q = 1; q < W; ++q) { ax += S.part[q][0][lane]; ay += S.part[q][1][lane]; az += S.part[q][2][lane]; }
     if (valid) {
         const int o = __ldg(perm + s);
         gax[o] = P.G * ax; gay[o] = P.G * ay; gaz[o] = P.G * az;
     }
-    // statistics: accepted interactions (lanes x nodes) and node visits per warp
+    // statistics: accepted interactions (lanes x nodes) and node visits per group
     unsigned nv = __popc(__ballot_sync(MHPC_FULL, valid));
     if (lane == 0) {
         atomicAdd(&st->interactions, ninter * nv);
@@ -837,9 +1033,16 @@ int gravity_v2(const TreeDev& T, const GravParams& P, const double* sx, const do
                const double* sh, const int* perm, double* gax, double* gay, double* gaz, DevStatus* st,
                cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
-    long groups = ((long)P.n + 31) / 32;
-    long blocks = (groups * 32 + kWalkBlock - 1) / kWalkBlock;
-    k_grav_v2<<<(int)blocks, kWalkBlock, 0, s>>>(T.com, T.link, T.nodes, P, sx, sy, sz, sh, perm, gax, gay, gaz, st);
+    const long groups = ((long)P.n + 31) / 32;
+#define MHPC_V2(W_) \
+    k_grav_v2<W_><<<(int)groups, 32 * W_, sizeof(V2Smem<W_>), s>>>(T, P, sx, sy, sz, sh, perm, gax, gay, gaz, st)
+    // warps per group: the walk of one group is a chain of memory round trips
+    // and FP64 sums, so more warps pay until the groups alone fill the SMs
+    // (measured at either side of each line beside k_grav_v2)
+    if (groups <= 148 * 2) MHPC_V2(8);
+    else if (groups <= 148 * 32) MHPC_V2(4);
+    else MHPC_V2(2);
+#undef MHPC_V2
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
 }
