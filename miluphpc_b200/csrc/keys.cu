@@ -76,6 +76,42 @@ __device__ __forceinline__ uint32_t axis_bits(double v, double lo, double hi) {
     return bits;
 }
 
+// The same bits without the chain where that is safe.  In exact arithmetic the
+// midpoints are the inner points of a grid of 2^21 cells, and the bits are the
+// complement of the cell index.  A computed midpoint is off the grid point by at
+// most one rounding (2^-53 M, M = max(|lo|, |hi|)) per level, 21 in all; in
+// cells that is 21 * 2^-32 M / edge = 4.9e-9 M / edge, and u below is off by
+// 2^21 * 4 roundings, 1.9e-9.  A coordinate whose u lies farther than `eps`
+// (more than twice the sum) from every grid point is on the same side of every
+// computed midpoint as of the grid point, so the comparisons of the chain are
+// known.  Everything else takes the chain: coordinates next to a grid point
+// (about 3e-8 of them), outside the box, not finite, or in a box too small,
+// too large or too far from the origin for the bound.
+struct AxisGrid {
+    double lo, scale, eps;
+};
+
+__device__ __forceinline__ AxisGrid axis_grid(double lo, double hi) {
+    AxisGrid G;
+    const double edge = hi - lo, m = fmax(fabs(lo), fabs(hi));
+    const bool ok = edge > 1e-280 && m < 1e300;
+    G.lo = lo;
+    G.scale = ok ? 2097152.0 / edge : 0.0;
+    G.eps = ok ? 4e-9 + 1.2e-8 * (m / edge) : 1.0;
+    return G;
+}
+
+__device__ __forceinline__ uint32_t axis_bits(const AxisGrid& G, double v, double hi) {
+    constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+    const double u = (v - G.lo) * G.scale;
+    const double r = u + kRound, t = u - (r - kRound);  // t: u minus the nearest grid point
+    if (fabs(t) > G.eps && u > 0.0 && u < 2097152.0) {
+        const int k = (int)(uint32_t)__double_as_longlong(r) - (t < 0.0 ? 1 : 0);
+        return 0x1fffffu ^ (uint32_t)k;
+    }
+    return axis_bits(v, G.lo, hi);
+}
+
 // Interleave: axis bit b of level l goes to key bit 3*(20-l) + axis.
 __device__ __forceinline__ uint64_t spread3(uint32_t v) {
     uint64_t x = v & 0x1fffffULL;
@@ -105,10 +141,11 @@ __global__ void __launch_bounds__(256) k_keys(const double* __restrict__ x, cons
     }
     __syncthreads();
     const double lo = bb ? bb[0] : ord_to_dbl(ord[0]), hi = bb ? bb[1] : ord_to_dbl(ord[1]);
+    const AxisGrid G = axis_grid(lo, hi);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t bx = axis_bits(__ldg(x + i), lo, hi);
-        uint32_t by = axis_bits(__ldg(y + i), lo, hi);
-        uint32_t bz = axis_bits(__ldg(z + i), lo, hi);
+        uint32_t bx = axis_bits(G, __ldg(x + i), hi);
+        uint32_t by = axis_bits(G, __ldg(y + i), hi);
+        uint32_t bz = axis_bits(G, __ldg(z + i), hi);
         uint64_t key = spread3(bx) | (spread3(by) << 1) | (spread3(bz) << 2);
         if (curve == 1) {
             // levels 21..2 in pairs, then level 1

@@ -1,14 +1,21 @@
 """Kernel variants that are chosen by size or input range, at the edges of
 those ranges, against the FP64 oracle."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
-from miluphpc_b200 import ics
+from miluphpc_b200 import _lib, ics
 from miluphpc_b200.miluphpc import Miluphpc
 from oracle import oracle as O
 from tests.helpers import gravity_cfg, rel_err
 
 pytestmark = pytest.mark.gpu
+
+
+def dptr(t):
+    return ctypes.c_void_p(t.data_ptr())
 
 
 # ---------------------------------------------------------------- v2 walk
@@ -46,3 +53,38 @@ def test_v2_walk_shared_keys(n, cuda):
     g = [sim.numpy(f)[tg] for f in ("g_ax", "g_ay", "g_az")]
     assert rel_err(*g, *o).max() < 1e-9
     sim.close()
+
+
+# -------------------------------------------------------------------- keys
+def box_keys(x, y, z, lo, hi, curve):
+    dev = torch.device("cuda:0")
+    t = [torch.as_tensor(np.ascontiguousarray(a), device=dev) for a in (x, y, z)]
+    bb = torch.tensor([lo, hi] * 3, dtype=torch.float64, device=dev)
+    keys = torch.zeros(len(x), dtype=torch.int64, device=dev)
+    _lib.check(_lib.load().mhpc_keys(*(dptr(a) for a in t), len(x), dptr(bb), curve, dptr(keys),
+                                     ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "keys")
+    return keys.cpu().numpy().view(np.uint64)
+
+
+@pytest.mark.parametrize("curve", [0, 1])
+@pytest.mark.parametrize("lo,hi", [(-1.0, 1.0), (-3.7, 11.3), (0.0, 1.0), (-1e-3, 0.0), (1e6, 1e6 + 1.0),
+                                   (-1e9 - 1e-3, -1e9 + 1e-3), (-1e-290, 1e-290), (0.0, 5e-324 * 1e6),
+                                   (-1e307, 1.2e308), (-1e200, 1e210), (2.0, 2.0)])
+def test_keys_near_grid_points(lo, hi, curve, cuda):
+    """Keys bit-equal to the oracle's bisection for coordinates on, next to (1 to
+    3 ulp) and far from the 2^21 grid points of boxes around, beside and far
+    from the origin, tiny, huge and empty boxes, and coordinates outside."""
+    rng = np.random.default_rng(5)
+    n = 60_000
+    f = rng.integers(0, 2 ** 21 + 1, n) / 2.0 ** 21
+    f[::3] = rng.uniform(0.0, 1.0, len(f[::3]))
+    f[::50] = np.round(f[::50] * 64) / 64
+    f[:4] = (0.0, 1.0, -0.01, 1.01)
+    with np.errstate(over="ignore", invalid="ignore"):
+        v = lo * (1.0 - f) + hi * f
+        for k in range(3):
+            m = rng.integers(0, 4, n) > k
+            v = np.where(m, np.nextafter(v, rng.choice([lo - 1.0, hi + 1.0], n)), v)
+    v = np.where(np.isfinite(v), v, lo)
+    x, y, z = v[: n // 3], v[n // 3: 2 * (n // 3)], v[2 * (n // 3): 3 * (n // 3)]
+    assert np.array_equal(box_keys(x, y, z, lo, hi, curve), O.keys(x, y, z, np.array([lo, hi] * 3), curve))
