@@ -212,19 +212,37 @@ __global__ void __launch_bounds__(256) k_dt_blocks(mhpc_particles p, int gravity
 
 __global__ void k_max_sml(int n, const double* h, double* part);
 
-// search radius from the per-block h maxima, then the final combine
-__global__ void k_dt_final_sr(int blocks, const double* hmax_part, const double* part, int int_rho, double time_left,
-                              double dt_max, double* dt_out) {
+// search radius from the per-block h maxima, then the final combine, in one
+// block (minima and maxima do not depend on the order).  One thread reading
+// the 296 blocks' values one after the other took 82 us.
+__global__ void __launch_bounds__(256) k_dt_final_sr(int blocks, const double* hmax_part, const double* part,
+                                                     int int_rho, double time_left, double dt_max, double* dt_out) {
     double hmax = 0.0;
-    for (int b = 0; b < blocks; ++b) hmax = fmax(hmax, hmax_part[b]);
-    double forces = 1.7976931348623157e308, courant = forces, dtrho = forces, visc = forces, vmax = 0.0;
-    for (int b = 0; b < blocks; ++b) {
-        forces = fmin(forces, part[5 * b]);
-        courant = fmin(courant, part[5 * b + 1]);
-        dtrho = fmin(dtrho, part[5 * b + 2]);
-        visc = fmin(visc, part[5 * b + 3]);
-        vmax = b == 0 ? part[5 * b + 4] : fmin(vmax, part[5 * b + 4]);
+    double v[5] = {1.7976931348623157e308, 1.7976931348623157e308, 1.7976931348623157e308, 1.7976931348623157e308,
+                   part[4]};
+    for (int b = threadIdx.x; b < blocks; b += 256) {
+        hmax = fmax(hmax, hmax_part[b]);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) v[k] = fmin(v[k], part[5 * b + k]);
     }
+    __shared__ double red[8][6];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        hmax = fmax(hmax, __shfl_xor_sync(MHPC_FULL, hmax, o));
+#pragma unroll
+        for (int k = 0; k < 5; ++k) v[k] = fmin(v[k], __shfl_xor_sync(MHPC_FULL, v[k], o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        for (int k = 0; k < 5; ++k) red[threadIdx.x >> 5][k] = v[k];
+        red[threadIdx.x >> 5][5] = hmax;
+    }
+    __syncthreads();
+    if (threadIdx.x > 0) return;
+    for (int w = 1; w < 8; ++w) {
+        for (int k = 0; k < 5; ++k) v[k] = fmin(v[k], red[w][k]);
+        hmax = fmax(hmax, red[w][5]);
+    }
+    const double forces = v[0], courant = v[1], dtrho = v[2], visc = v[3], vmax = v[4];
     const double search_radius = 2.0 * hmax;
     double dt = fmin(0.4 * courant, 0.2 * forces);
     if (vmax > 0. && search_radius > 0.) dt = fmin(dt, search_radius / (2 * vmax));
@@ -505,7 +523,7 @@ int launch_set_time_step(const mhpc_particles& p, int gravity, int sph, double a
     // search radius = 2 max(h) (Miluphpc::parallel_sph, src/miluphpc.cpp:2430-2433)
     k_max_sml<<<blocks, 256, 0, s>>>(p.n, p.sml, part);
     k_dt_blocks<<<blocks, 256, 0, s>>>(p, gravity, sph, alpha, beta, int_rho, part + blocks);
-    k_dt_final_sr<<<1, 1, 0, s>>>(blocks, part, part + blocks, int_rho, time_left, dt_max, dt_out);
+    k_dt_final_sr<<<1, 256, 0, s>>>(blocks, part, part + blocks, int_rho, time_left, dt_max, dt_out);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
 }
