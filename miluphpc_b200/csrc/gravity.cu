@@ -542,20 +542,29 @@ constexpr int kEvalUnroll = kPPL == 2 ? 8 : 4;
 constexpr int kListSub = 8;
 constexpr int kListStack = 1024;
 constexpr int kListReserve = 7 * 22 + 8;
-constexpr int kListCap = 64;
 
+// of one group, served by a team of W warps
+template <int W>
 struct ListSmem {
     int stk[kListStack];
-    float4 cpos[kListCap];  // cell: x, y, z (group frame), m
-    float4 cq0[kListCap];   // cell: Qxx Qxy Qxz Qyy
-    float2 cq1[kListCap];   // cell: Qyz Qzz
-    float4 lpos[kListCap];  // leaf: x, y, z, m
+    float4 cpos[64 * W];  // cell: x, y, z (group frame), m
+    float4 cq0[64 * W];   // cell: Qxx Qxy Qxz Qyy
+    float2 cq1[64 * W];   // cell: Qyz Qzz
+    float4 lpos[64 * W];  // leaf: x, y, z, m
     // sub-boxes, one array per component so that sub-boxes b, b+1 load as a
     // float2: lower corner, NEGATED upper corner, alpha |a|_min, quad_alpha |a|_min
     float bx0[kListSub], by0[kListSub], bz0[kListSub], bw0[kListSub];
     float nbx1[kListSub], nby1[kListSub], nbz1[kListSub], bw1[kListSub];
-    int defer[32];
+    int defer[32 * W];
+    int top;
+    int cnt[W > 1 ? W : 1][4];                            // per warp: leaf entries, cells, children, buckets
+    double part[W > 1 ? W : 1][W > 1 ? 4 * kPPL : 1][32]; // the warps' sums
 };
+template <int W>
+__device__ __forceinline__ void team_sync() {
+    if (W == 1) __syncwarp();
+    else __syncthreads();
+}
 
 // kGuard: some softened distance may be 0 (eps2 = 0), so 1/r is guarded; with
 // eps2 >= 1e-20 every r^2 >= eps2 keeps 1/r^3 finite and the guard is dropped
@@ -575,8 +584,8 @@ __device__ __forceinline__ float2 rsqrt2(float2 r2) {
     return ri;
 }
 
-template <bool kGuard>
-__device__ __forceinline__ void eval_cells_x2(const ListSmem& S, int count, const float (&rx)[kPPL],
+template <int W, bool kGuard>
+__device__ __forceinline__ void eval_cells_x2(const ListSmem<W>& S, int w, int count, const float (&rx)[kPPL],
                                               const float (&ry)[kPPL], const float (&rz)[kPPL],
                                               const float (&e2)[kPPL], double (&ax)[kPPL], double (&ay)[kPPL],
                                               double (&az)[kPPL]) {
@@ -588,7 +597,7 @@ __device__ __forceinline__ void eval_cells_x2(const ListSmem& S, int count, cons
         fx[q] = bc2(0.f); fy[q] = bc2(0.f); fz[q] = bc2(0.f);
     }
 #pragma unroll kEvalUnroll
-    for (int e = 0; e < count; ++e) {
+    for (int e = w; e < count; e += W) {
         const float4 c = S.cpos[e];
         const float4 a0 = S.cq0[e];
         const float2 a1 = S.cq1[e];
@@ -620,8 +629,8 @@ __device__ __forceinline__ void eval_cells_x2(const ListSmem& S, int count, cons
     }
 }
 
-template <bool kGuard>
-__device__ __forceinline__ void eval_leaves_x2(const ListSmem& S, int count, const float (&rx)[kPPL],
+template <int W, bool kGuard>
+__device__ __forceinline__ void eval_leaves_x2(const ListSmem<W>& S, int w, int count, const float (&rx)[kPPL],
                                                const float (&ry)[kPPL], const float (&rz)[kPPL],
                                                const float (&e2)[kPPL], double (&ax)[kPPL], double (&ay)[kPPL],
                                                double (&az)[kPPL]) {
@@ -633,7 +642,7 @@ __device__ __forceinline__ void eval_leaves_x2(const ListSmem& S, int count, con
         fx[q] = bc2(0.f); fy[q] = bc2(0.f); fz[q] = bc2(0.f);
     }
 #pragma unroll kEvalUnroll
-    for (int e = 0; e < count; ++e) {
+    for (int e = w; e < count; e += W) {
         const float4 c = S.lpos[e];
 #pragma unroll
         for (int q = 0; q < kNP; ++q) {
@@ -656,13 +665,13 @@ __device__ __forceinline__ void eval_leaves_x2(const ListSmem& S, int count, con
 
 // kPot: also the potential, -(m/r + RQR/(2 r^5)) per cell and -m/r per leaf,
 // leaving out the particle's own leaf (R = 0 exactly).
-template <bool kGuard, bool kPot>
-__device__ __forceinline__ void eval_cells(const ListSmem& S, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
+template <int W, bool kGuard, bool kPot>
+__device__ __forceinline__ void eval_cells(const ListSmem<W>& S, int w, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
                                            const float (&rz)[kPPL], const float (&e2)[kPPL], double (&ax)[kPPL],
                                            double (&ay)[kPPL], double (&az)[kPPL], double (&ph)[kPPL]) {
     float fx[kPPL] = {}, fy[kPPL] = {}, fz[kPPL] = {}, fp[kPPL] = {};
 #pragma unroll kEvalUnroll
-    for (int e = 0; e < count; ++e) {
+    for (int e = w; e < count; e += W) {
         const float4 c = S.cpos[e];
         const float4 a0 = S.cq0[e];
         const float2 a1 = S.cq1[e];
@@ -693,13 +702,13 @@ __device__ __forceinline__ void eval_cells(const ListSmem& S, int count, const f
     }
 }
 
-template <bool kGuard, bool kPot>
-__device__ __forceinline__ void eval_leaves(const ListSmem& S, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
+template <int W, bool kGuard, bool kPot>
+__device__ __forceinline__ void eval_leaves(const ListSmem<W>& S, int w, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
                                             const float (&rz)[kPPL], const float (&e2)[kPPL], double (&ax)[kPPL],
                                             double (&ay)[kPPL], double (&az)[kPPL], double (&ph)[kPPL]) {
     float fx[kPPL] = {}, fy[kPPL] = {}, fz[kPPL] = {}, fp[kPPL] = {};
 #pragma unroll kEvalUnroll
-    for (int e = 0; e < count; ++e) {
+    for (int e = w; e < count; e += W) {
         const float4 c = S.lpos[e];
 #pragma unroll
         for (int k = 0; k < kPPL; ++k) {
@@ -722,25 +731,32 @@ __device__ __forceinline__ void eval_leaves(const ListSmem& S, int count, const 
 
 // the packed forms for the force walk, the scalar forms when the potential is wanted
 constexpr bool kPackedEval = true;
-template <bool kGuard, bool kPot>
-__device__ __forceinline__ void eval_cells_sel(const ListSmem& S, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
+template <int W, bool kGuard, bool kPot>
+__device__ __forceinline__ void eval_cells_sel(const ListSmem<W>& S, int w, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
                                                const float (&rz)[kPPL], const float (&e2)[kPPL], double (&ax)[kPPL],
                                                double (&ay)[kPPL], double (&az)[kPPL], double (&ph)[kPPL]) {
-    if (kPackedEval && !kPot) eval_cells_x2<kGuard>(S, count, rx, ry, rz, e2, ax, ay, az);
-    else eval_cells<kGuard, kPot>(S, count, rx, ry, rz, e2, ax, ay, az, ph);
+    if (kPackedEval && !kPot) eval_cells_x2<W, kGuard>(S, w, count, rx, ry, rz, e2, ax, ay, az);
+    else eval_cells<W, kGuard, kPot>(S, w, count, rx, ry, rz, e2, ax, ay, az, ph);
 }
-template <bool kGuard, bool kPot>
-__device__ __forceinline__ void eval_leaves_sel(const ListSmem& S, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
+template <int W, bool kGuard, bool kPot>
+__device__ __forceinline__ void eval_leaves_sel(const ListSmem<W>& S, int w, int count, const float (&rx)[kPPL], const float (&ry)[kPPL],
                                                 const float (&rz)[kPPL], const float (&e2)[kPPL], double (&ax)[kPPL],
                                                 double (&ay)[kPPL], double (&az)[kPPL], double (&ph)[kPPL]) {
-    if (kPackedEval && !kPot) eval_leaves_x2<kGuard>(S, count, rx, ry, rz, e2, ax, ay, az);
-    else eval_leaves<kGuard, kPot>(S, count, rx, ry, rz, e2, ax, ay, az, ph);
+    if (kPackedEval && !kPot) eval_leaves_x2<W, kGuard>(S, w, count, rx, ry, rz, e2, ax, ay, az);
+    else eval_leaves<W, kGuard, kPot>(S, w, count, rx, ry, rz, e2, ax, ay, az, ph);
 }
 
 constexpr int kListBlock = 128;
 // relative rule: a sub-box's smallest previous |a| is taken as at least this
 // fraction of its largest (the oracle's statement uses the same floor)
 constexpr float kRelFloor = 0.1f;
+// Groups up to which a group gets a team of kListBlock / 32 warps: they test
+// kListBlock nodes a step and share the evaluation of the lists.  Walk in
+// us, Plummer (relative rule), one warp a group / teams of four:
+//   n        1,000   4,000   20,011   50,000   100,003   200,000   400,000   1,000,000
+//   1 warp      80     201      287      428       508       697      1047        1786
+//   4 warps     43      90      127      209       301       516       883        1923
+constexpr long kTeamGroups = 148 * 64;
 // Resident blocks per SM the list walk is compiled for: 5 (96 registers, no
 // spills in the force walk) measured 3 % faster at 16.7 M than the
 // unconstrained 116 registers (4 blocks); 6 blocks (80 registers) spill and
@@ -749,7 +765,7 @@ constexpr float kRelFloor = 0.1f;
 #define MHPC_LISTS_MIN_BLOCKS 5
 #endif
 
-template <bool kGuard, bool kRel, bool kPot>
+template <int W, bool kGuard, bool kRel, bool kPot>
 __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_lists(TreeDev T, GravParams P,
                                                                                  const double* __restrict__ sx,
                                                            const double* __restrict__ sy,
@@ -758,16 +774,19 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
                                                            const int* __restrict__ perm, double* __restrict__ gax,
                                                            double* __restrict__ gay, double* __restrict__ gaz,
                                                            DevStatus* st) {
-    __shared__ ListSmem smem[kListBlock / 32];
-    if (st->code) return;
+    static_assert(W == 1 || 32 * W == kListBlock, "a team is a warp or the whole block");
+    __shared__ ListSmem<W> smem[kListBlock / (32 * W)];
+    if (W == 1 ? st->code : __syncthreads_or(st->code)) return;
     const int M = *T.nodes;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    ListSmem& S = smem[threadIdx.x >> 5];
-    const long gwarp = ((long)blockIdx.x * kListBlock + threadIdx.x) >> 5;
+    const int w = W == 1 ? 0 : threadIdx.x >> 5;            // warp of the team
+    const int tt = W == 1 ? lane : threadIdx.x;             // thread of the team
+    ListSmem<W>& S = smem[W == 1 ? threadIdx.x >> 5 : 0];
+    const long group = W == 1 ? ((long)blockIdx.x * kListBlock + threadIdx.x) >> 5 : (long)blockIdx.x;
     const long ngroups = ((long)P.n + kListGroup - 1) / kListGroup;
-    if (gwarp >= ngroups) return;
-    const long s0 = gwarp * kListGroup;
+    if (group >= ngroups) return;
+    const long s0 = group * kListGroup;
     long s[kPPL];
     bool valid[kPPL];
     int sl[kPPL];
@@ -848,24 +867,24 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
     const double edge0 = ord_to_dbl(P.ord[1]) - ord_to_dbl(P.ord[0]);
     const float edge2 = (float)(edge0 * edge0);
     // the root's children: node 0 and its skip chain
-    int top = 0;
-    if (lane == 0) {
-        int c = 0;
-        while (c < M && top < 8) { S.stk[top++] = c; c = __ldg(&T.link[c].x); }
+    if (tt == 0) {
+        int c = 0, q = 0;
+        while (c < M && q < 8) { S.stk[q++] = c; c = __ldg(&T.link[c].x); }
         if (c < M) set_status(st, MHPC_ERR_DEPTH, 1);
+        S.top = q;
     }
-    top = __shfl_sync(MHPC_FULL, top, 0);
-    __syncwarp();
+    team_sync<W>();  // (also the sub-boxes, which every warp writes alike)
+    int top = S.top;
     double ax[kPPL] = {}, ay[kPPL] = {}, az[kPPL] = {}, ph[kPPL] = {};
     int ncell = 0, nleaf = 0;
     unsigned long long tested = 0, ncell_tot = 0, nleaf_tot = 0;
     while (top > 0) {
         int room = (kListStack - kListReserve - top) / 7;
-        int k = top < 32 ? top : 32;
+        int k = top < 32 * W ? top : 32 * W;
         if (k > room) k = room > 1 ? room : 1;
-        const bool act = lane < k;
-        const int nd = act ? S.stk[top - 1 - lane] : 0;
-        __syncwarp();
+        const bool act = tt < k;
+        const int nd = act ? S.stk[top - 1 - tt] : 0;
+        if (W == 1) __syncwarp();
         top -= k;
         tested += k;
         bool acc_leaf = false, acc_cell = false, open = false;
@@ -926,21 +945,10 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
                 open = !ok;
             }
         }
-        const unsigned bl = __ballot_sync(MHPC_FULL, acc_leaf);
-        if (acc_leaf) S.lpos[nleaf + __popc(bl & lt)] = make_float4(nx, ny, nz, m);
-        nleaf += __popc(bl);
-        const unsigned bc = __ballot_sync(MHPC_FULL, acc_cell);
-        if (acc_cell) {
-            const int i = ncell + __popc(bc & lt);
-            S.cpos[i] = make_float4(nx, ny, nz, m);
-            S.cq0[i] = w2;
-            S.cq1[i] = make_float2(w3.x, w3.y);
-        }
-        ncell += __popc(bc);
+        const unsigned bl = __ballot_sync(MHPC_FULL, acc_leaf), bc = __ballot_sync(MHPC_FULL, acc_cell);
         const int mask = open ? (__float_as_int(w3.z) >> 9) : 0;
         const bool bucket = open && (mask & 0x100);
         const unsigned bb = __ballot_sync(MHPC_FULL, bucket);
-        if (bucket) S.defer[__popc(bb & lt)] = nd;
         const int nkid = (open && !bucket) ? __popc(mask & 0xff) : 0;
         int incl = nkid;
 #pragma unroll
@@ -948,68 +956,105 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
             const int v = __shfl_up_sync(MHPC_FULL, incl, o);
             if (lane >= o) incl += v;
         }
-        const int total = __shfl_sync(MHPC_FULL, incl, 31);
+        // places in the lists and on the stack: this warp's, after the warps before it
+        int nl = __popc(bl), nc = __popc(bc), ndefer = __popc(bb), total = 0;
+        int lbase = nleaf, cbase = ncell, kbase = top, dbase = 0;
+        if (W == 1) {
+            total = __shfl_sync(MHPC_FULL, incl, 31);
+        } else {
+            if (lane == 31) { S.cnt[w][0] = nl; S.cnt[w][1] = nc; S.cnt[w][2] = incl; S.cnt[w][3] = ndefer; }
+            __syncthreads();
+            nl = nc = ndefer = 0;
+#pragma unroll
+            for (int q = 0; q < W; ++q) {
+                if (q == w) { lbase += nl; cbase += nc; kbase += total; dbase = ndefer; }
+                nl += S.cnt[q][0]; nc += S.cnt[q][1]; total += S.cnt[q][2]; ndefer += S.cnt[q][3];
+            }
+        }
+        if (acc_leaf) S.lpos[lbase + __popc(bl & lt)] = make_float4(nx, ny, nz, m);
+        nleaf += nl;
+        if (acc_cell) {
+            const int i = cbase + __popc(bc & lt);
+            S.cpos[i] = make_float4(nx, ny, nz, m);
+            S.cq0[i] = w2;
+            S.cq1[i] = make_float2(w3.x, w3.y);
+        }
+        ncell += nc;
+        if (bucket) S.defer[dbase + __popc(bb & lt)] = nd;
         if (top + total > kListStack) {
             // unreachable by the bound on k; stop instead of overrunning
-            if (lane == 0) set_status(st, MHPC_ERR_DEPTH, 2);
+            if (tt == 0) set_status(st, MHPC_ERR_DEPTH, 2);
             return;
         }
         if (nkid) {
             const int4 k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
             const int4 k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
             const int all[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-            int w = top + incl - nkid;
+            int pos = kbase + incl - nkid;
 #pragma unroll
             for (int d = 0; d < 8; ++d)
-                if ((mask >> d) & 1) S.stk[w++] = all[d];
+                if ((mask >> d) & 1) S.stk[pos++] = all[d];
         }
         top += total;
-        __syncwarp();
-        if (ncell >= 32) {
-            eval_cells_sel<kGuard, kPot>(S, ncell, rx, ry, rz, e2, ax, ay, az, ph);
+        team_sync<W>();
+        if (ncell >= 32 * W) {
+            eval_cells_sel<W, kGuard, kPot>(S, w, ncell, rx, ry, rz, e2, ax, ay, az, ph);
             ncell_tot += ncell;
             ncell = 0;
-            __syncwarp();
+            team_sync<W>();
         }
-        if (nleaf >= 32) {
-            eval_leaves_sel<kGuard, kPot>(S, nleaf, rx, ry, rz, e2, ax, ay, az, ph);
+        if (nleaf >= 32 * W) {
+            eval_leaves_sel<W, kGuard, kPot>(S, w, nleaf, rx, ry, rz, e2, ax, ay, az, ph);
             nleaf_tot += nleaf;
             nleaf = 0;
-            __syncwarp();
+            team_sync<W>();
         }
-        // shared-key buckets: their children are consecutive leaves (the
-        // leaf list holds fewer than 32 entries here, at most 63 after a round)
-        const int ndefer = __popc(bb);
+        // shared-key buckets: their children are consecutive leaves (the leaf
+        // list holds fewer than 32 W entries here, at most 64 W - 1 after a round)
         for (int d = 0; d < ndefer; ++d) {
             const int b = S.defer[d];
             const int end = __ldg(&T.link[b].x);
-            for (int c0 = b + 1; c0 < end; c0 += 32) {
-                const int c = c0 + lane;
-                const bool a = c < end;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (a) {
+            for (int c0 = b + 1; c0 < end; c0 += 32 * W) {
+                const int c = c0 + tt;
+                if (c < end) {
                     const float4 hp = __ldg(T.wrec + 4 * (size_t)c);
                     const float4 lp = __ldg(T.wrec + 4 * (size_t)c + 1);
-                    v = make_float4((hp.x - chx) + (lp.x - clx), (hp.y - chy) + (lp.y - cly),
-                                    (hp.z - chz) + (lp.z - clz), hp.w);
+                    S.lpos[nleaf + tt] = make_float4((hp.x - chx) + (lp.x - clx), (hp.y - chy) + (lp.y - cly),
+                                                     (hp.z - chz) + (lp.z - clz), hp.w);
                 }
-                const unsigned ba = __ballot_sync(MHPC_FULL, a);
-                if (a) S.lpos[nleaf + __popc(ba & lt)] = v;
-                nleaf += __popc(ba);
-                __syncwarp();
-                if (nleaf >= 32) {
-                    eval_leaves_sel<kGuard, kPot>(S, nleaf, rx, ry, rz, e2, ax, ay, az, ph);
+                nleaf += min(32 * W, end - c0);
+                team_sync<W>();
+                if (nleaf >= 32 * W) {
+                    eval_leaves_sel<W, kGuard, kPot>(S, w, nleaf, rx, ry, rz, e2, ax, ay, az, ph);
                     nleaf_tot += nleaf;
                     nleaf = 0;
-                    __syncwarp();
+                    team_sync<W>();
                 }
             }
         }
     }
-    if (ncell) eval_cells_sel<kGuard, kPot>(S, ncell, rx, ry, rz, e2, ax, ay, az, ph);
-    if (nleaf) eval_leaves_sel<kGuard, kPot>(S, nleaf, rx, ry, rz, e2, ax, ay, az, ph);
+    if (ncell) eval_cells_sel<W, kGuard, kPot>(S, w, ncell, rx, ry, rz, e2, ax, ay, az, ph);
+    if (nleaf) eval_leaves_sel<W, kGuard, kPot>(S, w, nleaf, rx, ry, rz, e2, ax, ay, az, ph);
     ncell_tot += ncell;
     nleaf_tot += nleaf;
+    if (W > 1) {
+        // the team's sums, added by its first warp in warp order
+#pragma unroll
+        for (int q = 0; q < kPPL; ++q) {
+            S.part[w][4 * q][lane] = ax[q]; S.part[w][4 * q + 1][lane] = ay[q]; S.part[w][4 * q + 2][lane] = az[q];
+            if (kPot) S.part[w][4 * q + 3][lane] = ph[q];
+        }
+        __syncthreads();
+        if (w > 0) return;
+#pragma unroll
+        for (int v = 1; v < W; ++v)
+#pragma unroll
+            for (int q = 0; q < kPPL; ++q) {
+                ax[q] += S.part[v][4 * q][lane]; ay[q] += S.part[v][4 * q + 1][lane];
+                az[q] += S.part[v][4 * q + 2][lane];
+                if (kPot) ph[q] += S.part[v][4 * q + 3][lane];
+            }
+    }
     unsigned nv = 0;
 #pragma unroll
     for (int k = 0; k < kPPL; ++k) {
@@ -1074,12 +1119,20 @@ int gravity_lists(const TreeDev& T, const GravParams& P, const double* sx, const
                   cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
     const long groups = ((long)P.n + kListGroup - 1) / kListGroup;
-    const long blocks = (groups * 32 + kListBlock - 1) / kListBlock;
+    const bool team = groups <= kTeamGroups;
+    const long blocks = team ? groups : (groups * 32 + kListBlock - 1) / kListBlock;
     // the self-interaction has R = 0 and r^2 = eps2: 1/r^3 stays finite in
     // FP32 for eps2 >= 1e-20
     const bool guard = !(P.eps2 >= 1e-20) && !(P.h_factor > 0.0), rel = P.rel_alpha > 0.0;
-#define MHPC_LISTS(G_, R_, P_) \
-    k_grav_lists<G_, R_, P_><<<(int)blocks, kListBlock, 0, s>>>(T, P, sx, sy, sz, sh, perm, gax, gay, gaz, st)
+#define MHPC_LISTS(G_, R_, P_)                                                                                     \
+    do {                                                                                                           \
+        if (team)                                                                                                  \
+            k_grav_lists<kListBlock / 32, G_, R_, P_>                                                              \
+                <<<(int)blocks, kListBlock, 0, s>>>(T, P, sx, sy, sz, sh, perm, gax, gay, gaz, st);                \
+        else                                                                                                       \
+            k_grav_lists<1, G_, R_, P_>                                                                            \
+                <<<(int)blocks, kListBlock, 0, s>>>(T, P, sx, sy, sz, sh, perm, gax, gay, gaz, st);                \
+    } while (0)
     if (P.pot) {
         // potential (diagnostics): separate instantiations, the force walk stays as it is
         if (!guard && !rel) MHPC_LISTS(false, false, true);
