@@ -228,34 +228,63 @@ __device__ __forceinline__ void leaf_moments(const TreeDev& T, int a, int leaf, 
 
 // Cell p from its completed children.  Centres of mass use explicitly
 // rounded products and sums in slot order, so the result is bit-identical to
-// the level-wise sums of the reference.  With `local` the first pass over the
-// children also brings their quadrupoles into L1 for the second.
+// the level-wise sums of the reference.  The children's loads are issued kB
+// slots at a time (an empty slot reads cell p itself) before the ordered sums:
+// a load behind each slot's test waits for the one before it.  With `local`
+// the first pass over the children also brings their quadrupoles into L1 for
+// the second.
+template <int kB>
 __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids& K, int want_quad, int want_box,
                                              double edge0, double inv_theta, bool local) {
     double m = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
     float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
     float4 hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-    auto add_com = [&](int c) {
-        const double4 cc = ld_up_d4(&T.com[c], local);
-        if (local && want_quad) prefetch_l1(T.wrec + 4 * (size_t)c + 2);
+    auto add_com = [&](const double4& cc) {
         mx = __dadd_rn(mx, __dmul_rn(cc.x, cc.w));
         my = __dadd_rn(my, __dmul_rn(cc.y, cc.w));
         mz = __dadd_rn(mz, __dmul_rn(cc.z, cc.w));
         m = __dadd_rn(m, cc.w);
-        if (want_box) {
-            const float4 bl = ld_up(&T.bmin[c], local), bh = ld_up(&T.bmax[c], local);
-            lo.x = fminf(lo.x, bl.x); lo.y = fminf(lo.y, bl.y); lo.z = fminf(lo.z, bl.z);
-            hi.x = fmaxf(hi.x, bh.x); hi.y = fmaxf(hi.y, bh.y); hi.z = fmaxf(hi.z, bh.z);
-        }
+    };
+    auto add_box = [&](const float4& bl, const float4& bh) {
+        lo.x = fminf(lo.x, bl.x); lo.y = fminf(lo.y, bl.y); lo.z = fminf(lo.z, bl.z);
+        hi.x = fmaxf(hi.x, bh.x); hi.y = fmaxf(hi.y, bh.y); hi.z = fmaxf(hi.z, bh.z);
     };
     const int2 lkp = __ldg(&T.link[p]);
     const int end = lkp.x;
     if (K.mask & 0x100) {
-        for (int c = p + 1; c < end; c = __ldg(&T.link[c].x)) add_com(c);
+        for (int c = p + 1; c < end; c = __ldg(&T.link[c].x)) {
+            add_com(ld_up_d4(&T.com[c], local));
+            if (want_box) add_box(ld_up(&T.bmin[c], local), ld_up(&T.bmax[c], local));
+        }
     } else {
 #pragma unroll
-        for (int d = 0; d < 8; ++d)
-            if ((K.mask >> d) & 1) add_com(K.id[d]);
+        for (int d0 = 0; d0 < 8; d0 += kB) {
+            const int part = (K.mask >> d0) & ((1 << kB) - 1);
+            if (!part) continue;
+            double4 cc[kB];
+#pragma unroll
+            for (int d = 0; d < kB; ++d) cc[d] = ld_up_d4(&T.com[(part >> d) & 1 ? K.id[d0 + d] : p], local);
+            if (local && want_quad) {
+#pragma unroll
+                for (int d = 0; d < kB; ++d)
+                    if ((part >> d) & 1) prefetch_l1(T.wrec + 4 * (size_t)K.id[d0 + d] + 2);
+            }
+#pragma unroll
+            for (int d = 0; d < kB; ++d)
+                if ((part >> d) & 1) add_com(cc[d]);
+            if (want_box) {
+                float4 bl[kB], bh[kB];
+#pragma unroll
+                for (int d = 0; d < kB; ++d) {
+                    const int c = (part >> d) & 1 ? K.id[d0 + d] : p;
+                    bl[d] = ld_up(&T.bmin[c], local);
+                    bh[d] = ld_up(&T.bmax[c], local);
+                }
+#pragma unroll
+                for (int d = 0; d < kB; ++d)
+                    if ((part >> d) & 1) add_box(bl[d], bh[d]);
+            }
+        }
     }
     if (m > 0.0) {
         mx = __ddiv_rn(mx, m);
@@ -269,8 +298,8 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
     }
     if (want_quad) {
         double q[6] = {0, 0, 0, 0, 0, 0};
-        auto add_quad = [&](int c) {
-            const double4 cc = ld_up_d4(&T.com[c], local);
+        // a0, a1: the child's quadrupole from its walk record (one 32-byte sector)
+        auto add_quad = [&](const double4& cc, const float4& a0, const float4& a1) {
             const double s0 = cc.x - mx, s1 = cc.y - my, s2 = cc.z - mz;
             const double ss = s0 * s0 + s1 * s1 + s2 * s2;
             const double w = cc.w;
@@ -280,19 +309,33 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
             q[3] += w * (3.0 * s1 * s1 - ss);
             q[4] += w * 3.0 * s1 * s2;
             q[5] += w * (3.0 * s2 * s2 - ss);
-            // the child's quadrupole from its walk record (one 32-byte sector)
-            const float4 a0 = ld_up(T.wrec + 4 * (size_t)c + 2, local);
-            const float4 a1 = ld_up(T.wrec + 4 * (size_t)c + 3, local);
             if (!(__float_as_int(a1.z) & ND_LEAF)) {
                 q[0] += a0.x; q[1] += a0.y; q[2] += a0.z; q[3] += a0.w; q[4] += a1.x; q[5] += a1.y;
             }
         };
         if (K.mask & 0x100) {
-            for (int c = p + 1; c < end; c = __ldg(&T.link[c].x)) add_quad(c);
+            for (int c = p + 1; c < end; c = __ldg(&T.link[c].x))
+                add_quad(ld_up_d4(&T.com[c], local), ld_up(T.wrec + 4 * (size_t)c + 2, local),
+                         ld_up(T.wrec + 4 * (size_t)c + 3, local));
         } else {
+            constexpr int kQ = kB > 2 ? kB / 2 : kB;
 #pragma unroll
-            for (int d = 0; d < 8; ++d)
-                if ((K.mask >> d) & 1) add_quad(K.id[d]);
+            for (int d0 = 0; d0 < 8; d0 += kQ) {
+                const int part = (K.mask >> d0) & ((1 << kQ) - 1);
+                if (!part) continue;
+                double4 cc[kQ];
+                float4 a0[kQ], a1[kQ];
+#pragma unroll
+                for (int d = 0; d < kQ; ++d) {
+                    const int c = (part >> d) & 1 ? K.id[d0 + d] : p;
+                    cc[d] = ld_up_d4(&T.com[c], local);
+                    a0[d] = ld_up(T.wrec + 4 * (size_t)c + 2, local);
+                    a1[d] = ld_up(T.wrec + 4 * (size_t)c + 3, local);
+                }
+#pragma unroll
+                for (int d = 0; d < kQ; ++d)
+                    if ((part >> d) & 1) add_quad(cc[d], a0[d], a1[d]);
+            }
         }
         const float4 q0 = make_float4((float)q[0], (float)q[1], (float)q[2], (float)q[3]);
         const float2 q1 = make_float2((float)q[4], (float)q[5]);
@@ -320,12 +363,28 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
 // clears the count for the next pass over the same tree.  Crossing cells are
 // the common ancestors of the two particles at a range boundary, at most 21
 // per boundary, so counted hand-offs are rare.
-// 256 threads x 8 positions; 4 resident blocks per SM (64 registers) measured
-// faster than 2 (86 registers); 16 positions per thread measured slower
+// 256 threads; 3 resident blocks per SM (80 registers, four children's loads in
+// flight) measured faster than 2 or 4.
 constexpr int kUpBlock = 256;
-constexpr int kUpPer = 8;  // positions per thread
-constexpr int kUpChunk = kUpPer * kUpBlock;
 constexpr int kUpHand = 1024;
+
+// Positions per thread.  A block works through its levels one round trip after
+// the other, so a small n takes few positions per block to have many blocks;
+// a large n fills the SMs anyway, and longer ranges have fewer cells that
+// cross a boundary.  Upward pass with walk records in us (the 8-position form
+// with one child's loads at a time was the only one before):
+//   n         1,000   20,011   100,003   300,000   1,000,000   4,000,000   2^24
+//   before       74      158       160       180         266         742   2604
+//   1            66       77        87       176         447
+//   2            68       79        90       141         313
+//   4            55       93        97       120         262
+//   8                                        136         283         682   2504
+inline int up_per(int n) {
+    if (n <= 8192) return 4;
+    if (n <= 65536) return 1;
+    if (n <= 200000) return 2;
+    return n <= 2000000 ? 4 : 8;
+}
 
 __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
@@ -374,8 +433,9 @@ __device__ __forceinline__ void block_min_scans(int agg, int* wtot, int& pre, in
     suf = min(right, lane < 31 ? qe : 255);
 }
 
-template <typename Leaf, typename Combine>
+template <int kUpPer, typename Leaf, typename Combine>
 __device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, Combine&& combine) {
+    constexpr int kUpChunk = kUpPer * kUpBlock;
     __shared__ int queue[kUpBlock / 32][32 * kUpPer];             // cell
     __shared__ unsigned short qpos[kUpBlock / 32][32 * kUpPer];   // its first position - a0
     __shared__ int hand[kUpHand];
@@ -485,25 +545,27 @@ __device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, C
     for (int k = threadIdx.x; k < nh; k += kUpBlock) hand_off(T, hand[k], combine);
 }
 
-__global__ void __launch_bounds__(kUpBlock, 4) k_upward(TreeDev T, const double* __restrict__ sx,
+template <int kUpPer>
+__global__ void __launch_bounds__(kUpBlock, 3) k_upward(TreeDev T, const double* __restrict__ sx,
                                                      const double* __restrict__ sy, const double* __restrict__ sz,
                                                      const double* __restrict__ sm, int want_quad, int want_box,
                                                      const long long* __restrict__ ord, double inv_theta,
                                                      const DevStatus* st) {
     if (st->code) return;
     const double edge0 = want_quad ? ord_to_dbl(ord[1]) - ord_to_dbl(ord[0]) : 0.0;
-    upward_chunk(
+    upward_chunk<kUpPer>(
         T, [&](int a, int leaf) { leaf_moments(T, a, leaf, sx, sy, sz, sm, want_quad, want_box, edge0, inv_theta); },
         [&](int p, bool local) {
-            cell_moments(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta, local);
+            cell_moments<4>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta, local);
         });
 }
 
 
 // Bottom-up maximum of the smoothing lengths, in one launch like the moments.
+template <int kUpPer>
 __global__ void __launch_bounds__(kUpBlock, 4) k_hmax(TreeDev T, const double* __restrict__ h, const DevStatus* st) {
     if (st->code) return;
-    upward_chunk(
+    upward_chunk<kUpPer>(
         T, [&](int a, int leaf) { T.hmax[leaf] = __double2float_ru(h[a]); },
         [&](int p, bool local) {
             const int km = __ldg(T.kmask + p);
@@ -513,9 +575,12 @@ __global__ void __launch_bounds__(kUpBlock, 4) k_hmax(TreeDev T, const double* _
                 for (int c = p + 1; c < end; c = __ldg(&T.link[c].x)) m = fmaxf(m, ld_up(&T.hmax[c], local));
             } else {
                 const Kids K = cell_kids(T, p);
+                float v[8];
+#pragma unroll
+                for (int d = 0; d < 8; ++d) v[d] = ld_up(&T.hmax[(K.mask >> d) & 1 ? K.id[d] : p], local);
 #pragma unroll
                 for (int d = 0; d < 8; ++d)
-                    if ((K.mask >> d) & 1) m = fmaxf(m, ld_up(&T.hmax[K.id[d]], local));
+                    if ((K.mask >> d) & 1) m = fmaxf(m, v[d]);
             }
             T.hmax[p] = m;
         });
@@ -543,14 +608,29 @@ int tree_build(TreeDev& T, const uint64_t* skey, void* scan_scratch, DevStatus* 
 int tree_upward(TreeDev& T, const double* sx, const double* sy, const double* sz, const double* sm,
                 int want_quad, int want_box, const long long* ord, double theta, DevStatus* st, cudaStream_t s) {
     const double inv_theta = want_quad ? 1.0 / theta : 0.0;
-    k_upward<<<(T.n + kUpChunk - 1) / kUpChunk, kUpBlock, 0, s>>>(T, sx, sy, sz, sm, want_quad, want_box, ord,
-                                                                  inv_theta, st);
+#define MHPC_UP(P_)                                                                                              \
+    k_upward<P_><<<(T.n + P_ * kUpBlock - 1) / (P_ * kUpBlock), kUpBlock, 0, s>>>(T, sx, sy, sz, sm, want_quad, \
+                                                                                 want_box, ord, inv_theta, st)
+    switch (up_per(T.n)) {
+        case 1: MHPC_UP(1); break;
+        case 2: MHPC_UP(2); break;
+        case 4: MHPC_UP(4); break;
+        default: MHPC_UP(8); break;
+    }
+#undef MHPC_UP
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
 }
 
 int tree_node_hmax(const TreeDev& T, const double* h, const DevStatus* st, cudaStream_t s) {
-    k_hmax<<<(T.n + kUpChunk - 1) / kUpChunk, kUpBlock, 0, s>>>(T, h, st);
+#define MHPC_UP(P_) k_hmax<P_><<<(T.n + P_ * kUpBlock - 1) / (P_ * kUpBlock), kUpBlock, 0, s>>>(T, h, st)
+    switch (up_per(T.n)) {
+        case 1: MHPC_UP(1); break;
+        case 2: MHPC_UP(2); break;
+        case 4: MHPC_UP(4); break;
+        default: MHPC_UP(8); break;
+    }
+#undef MHPC_UP
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
 }
