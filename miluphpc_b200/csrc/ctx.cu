@@ -42,8 +42,7 @@ struct mhpc_ctx {
     double *sx = nullptr, *sy = nullptr, *sz = nullptr, *sm = nullptr, *sh = nullptr;
     double *svx = nullptr, *svy = nullptr, *svz = nullptr, *se = nullptr, *srho = nullptr, *sp = nullptr,
            *scs = nullptr, *sbal = nullptr;
-    float4 *sf0 = nullptr, *sf1 = nullptr, *sf2 = nullptr;  // FP32 pair-sum views (mixed SPH)
-    float2* sf3 = nullptr;
+    double4 *ra = nullptr, *rb = nullptr, *rc = nullptr;  // 32-byte records of the SPH pair sums
     int* smat = nullptr;
     TreeDev T;
     int* nbr = nullptr;
@@ -310,7 +309,7 @@ SphSorted sph_sorted(mhpc_ctx* c, const mhpc_particles* p) {
     S.vx = c->svx; S.vy = c->svy; S.vz = c->svz; S.e = c->se;
     S.mat = p->material_id ? c->smat : nullptr;
     S.rho = c->srho; S.p = c->sp; S.cs = c->scs; S.bal = c->sbal;
-    S.f0 = c->sf0; S.f1 = c->sf1; S.f2 = c->sf2; S.f3 = c->sf3;
+    S.ra = c->ra; S.rb = c->rb; S.rc = c->rc;
     return S;
 }
 
@@ -414,7 +413,7 @@ int stage_forces(mhpc_ctx* c, const mhpc_particles* p) {
     SphSorted S = sph_sorted(c, p);
     const int target = sph_target(c);
     const bool learned = c->frnn_learned;
-    TRY(sph_forces(P, S, c->nbr, c->noi, c->perm, p->ax, p->ay, p->az, p->drhodt, p->dedt, p->dsmldt, c->st, s));
+    TRY(sph_forces(P, S, c->dens_ready, c->nbr, c->noi, c->perm, p->ax, p->ay, p->az, p->drhodt, p->dedt, p->dsmldt, c->st, s));
     if (p->nnl || p->noi) TRY(sph_export_nnl(P, c->nbr, c->noi, c->perm, p->nnl, p->noi, s));
     if (c->cfg.variable_sml) TRY(sph_band_stats(P, c->noi, target, c->cfg.nb_tolerance, c->st, s));
     record(c, EV_FORCES);
@@ -598,7 +597,7 @@ int mhpc_ctx_create(mhpc_ctx** out, int capacity, const mhpc_config* cfg, const 
     if (cfg->sph) {
         A(c->svx, n); A(c->svy, n); A(c->svz, n); A(c->se, n); A(c->srho, n); A(c->sp, n); A(c->scs, n);
         A(c->sbal, n);
-        A(c->sf0, n); A(c->sf1, n); A(c->sf2, n); A(c->sf3, n);
+        A(c->ra, n); A(c->rb, n); A(c->rc, n);
         A(c->smat, n);
         size_t groups = (n + 31) / 32;
         A(c->nbr, groups * 32 * (size_t)c->maxnb);

@@ -1,5 +1,5 @@
-// SPH: fixed-radius neighbour search, variable smoothing length, density /
-// sound speed / pressure, and internal (hydro) forces.
+// SPH: fixed-radius neighbour search and variable smoothing length (the pair
+// sums over the neighbour lists are in sph_pairs.cu).
 //
 // Neighbour search: the reference walks the tree once per particle with a
 // per-thread stack (SPH::fixedRadiusNN, src/sph/sph.cu:93-281).  Here a warp
@@ -18,114 +18,6 @@ namespace {
 constexpr int kBlock = 128;
 constexpr int kWarps = kBlock / 32;
 constexpr int kSmall = 16;    // cells with at most this many particles are staged whole
-
-// ------------------------------------------------------------ kernels W
-// SmoothingKernel::{spiky, cubicSpline, wendlandc2, wendlandc4, wendlandc6}
-// (src/sph/kernel.cu:14-183), 3-D forms, support radius = h.
-__device__ __forceinline__ void skernel(int type, double r, double h, double& W, double& dWdr) {
-    const double q = r / h;
-    W = 0.0;
-    dWdr = 0.0;
-    switch (type) {
-        case 0: {  // spiky
-            if (q <= 1.0 && q >= 0.0) {
-                const double a = 1.0 - q;
-                W = 15. / (M_PI * h * h * h) * a * a * a;
-                dWdr = -45 / (M_PI * h * h * h * h) * a * a;
-            }
-        } break;
-        case 1: {  // cubic spline
-            const double f = 8. / M_PI * 1. / (h * h * h);
-            if (q > 1) {
-            } else if (q > 0.5) {
-                const double a = 1. - q;
-                W = 2. * f * a * a * a;
-                dWdr = -6. * f * 1. / h * a * a;
-            } else {
-                W = f * (6. * q * q * q - 6. * q * q + 1.);
-                dWdr = 6. * f / h * (3 * q * q - 2 * q);
-            }
-        } break;
-        case 2: {  // Wendland C2
-            if (r <= h) {
-                const double a = 1 - q;
-                W = 21. / (2 * M_PI * h * h * h) * a * a * a * a * (1 + 4 * q) * (q < 1);
-                dWdr = -210. / (M_PI * h * h * h * h) * q * a * a * a * (q < 1);
-            }
-        } break;
-        case 3: {  // Wendland C4 (derivative as written in the reference)
-            if (r <= h) {
-                const double a = 1 - q, a5 = a * a * a * a * a;
-                W = 495. / (32. * M_PI * h * h * h) * a5 * a * (1. + 6. * q + 35. / 3. * q * q) * (q < 1);
-                dWdr = -1485. / (16. * M_PI * h * h * h * h) * a5 * (1. - 35. * q * q + 105. * q * q * q) * (q < 1);
-            }
-        } break;
-        default: {  // Wendland C6
-            if (r <= h) {
-                const double a = 1 - q, a7 = a * a * a * a * a * a * a;
-                W = 1365. / (64. * M_PI * h * h * h) * a7 * a * (1. + 8. * q + 25. * q * q + 32 * q * q * q) * (q < 1);
-                dWdr = -15015. / (32. * M_PI * h * h * h * h) * q * a7 * (1. + 7 * q + 16 * q * q) * (q < 1);
-            }
-        } break;
-    }
-}
-
-// FP32 forms of the same kernels for the mixed-precision pair sums (one
-// reciprocal of h, the rest products).
-__device__ __forceinline__ void skernel_f(int type, float r, float h, float& W, float& dWdr) {
-    const float ih = __frcp_rn(h);
-    const float q = r * ih, ih3 = ih * ih * ih, ih4 = ih3 * ih;
-    constexpr float kPi = 3.14159265358979f;
-    W = 0.f;
-    dWdr = 0.f;
-    switch (type) {
-        case 0: {
-            if (q <= 1.f && q >= 0.f) {
-                const float a = 1.f - q;
-                W = 15.f / kPi * ih3 * a * a * a;
-                dWdr = -45.f / kPi * ih4 * a * a;
-            }
-        } break;
-        case 1: {
-            const float f = 8.f / kPi * ih3;
-            if (q > 1.f) {
-            } else if (q > 0.5f) {
-                const float a = 1.f - q;
-                W = 2.f * f * a * a * a;
-                dWdr = -6.f * f * ih * a * a;
-            } else {
-                W = f * (6.f * q * q * q - 6.f * q * q + 1.f);
-                dWdr = 6.f * f * ih * (3.f * q * q - 2.f * q);
-            }
-        } break;
-        case 2: {
-            if (q < 1.f) {
-                const float a = 1.f - q;
-                W = 21.f / (2.f * kPi) * ih3 * a * a * a * a * (1.f + 4.f * q);
-                dWdr = -210.f / kPi * ih4 * q * a * a * a;
-            }
-        } break;
-        case 3: {
-            if (q < 1.f) {
-                const float a = 1.f - q, a5 = a * a * a * a * a;
-                W = 495.f / (32.f * kPi) * ih3 * a5 * a * (1.f + 6.f * q + 35.f / 3.f * q * q);
-                dWdr = -1485.f / (16.f * kPi) * ih4 * a5 * (1.f - 35.f * q * q + 105.f * q * q * q);
-            }
-        } break;
-        default: {
-            if (q < 1.f) {
-                const float a = 1.f - q, a7 = a * a * a * a * a * a * a;
-                W = 1365.f / (64.f * kPi) * ih3 * a7 * a * (1.f + 8.f * q + 25.f * q * q + 32.f * q * q * q);
-                dWdr = -15015.f / (32.f * kPi) * ih4 * q * a7 * (1.f + 7.f * q + 16.f * q * q);
-            }
-        } break;
-    }
-}
-
-// FP32 difference of two positions held as FP32 hi/lo splits of FP64 values
-__device__ __forceinline__ float3 rel_f(const float4& ah, const float4& al, const float4& bh, const float4& bl) {
-    return make_float3((ah.x - bh.x) + (al.x - bl.x), (ah.y - bh.y) + (al.y - bl.y), (ah.z - bh.z) + (al.z - bl.z));
-}
 
 // ------------------------------------------------------------ FRNN walk
 // One warp per 32 consecutive (sorted or listed) particles, lane = particle,
@@ -585,294 +477,6 @@ __global__ void k_noi_stats(int n, int maxnb, const int* __restrict__ noi, DevSt
     }
 }
 
-// --------------------------------------------------- density + EOS (fused)
-// calculateDensity (src/sph/density.cu:8-72), then calculateSoundSpeed
-// (src/sph/soundspeed.cu:38-97) and calculatePressure (src/sph/pressure.cu:5-87)
-// in the reference's order: the ideal-gas sound speed uses the pressure of
-// the previous call.
-__global__ void __launch_bounds__(kBlock) k_density_eos(SphParams P, SphSorted S, const int* __restrict__ nbr,
-                                                        const int* __restrict__ noi, const int* __restrict__ perm,
-                                                        double* rho_out, double* p_out, double* cs_out,
-                                                        DevStatus* st) {
-    if (st->code) return;
-    const long s = (long)blockIdx.x * kBlock + threadIdx.x;
-    if (s >= P.n) return;
-    const double xi = S.x[s], yi = S.y[s], zi = S.z[s], hi = S.h[s];
-    double rho;
-    if (P.integrate_density) {
-        rho = S.rho[s];
-    } else {
-        double W, dWdr;
-        skernel(P.kernel, 0.0, hi, W, dWdr);
-        rho = S.m[s] * W;
-        const int k = min(noi[s], P.maxnb);
-        for (int q = 0; q < k; ++q) {
-            const int j = nbr[nb_index(s, q, P.maxnb)];
-            const double hb = P.avg_h ? 0.5 * (hi + __ldg(S.h + j)) : hi;
-            const double dx = xi - __ldg(S.x + j), dy = yi - __ldg(S.y + j), dz = zi - __ldg(S.z + j);
-            const double r = sqrt(dx * dx + dy * dy + dz * dz);
-            skernel(P.kernel, r, hb, W, dWdr);
-            rho += __ldg(S.m + j) * W;
-        }
-        if (!(rho > 0.0)) set_status(st, MHPC_ERR_NAN, (int)s);
-    }
-    const int mid = S.mat ? S.mat[s] : 0;
-    const MatDev& M = P.mat[mid];
-    double p = S.p[s], cs = S.cs[s];
-    switch (M.eos_type) {
-        case 0: cs = sqrt(M.K * pow(rho, M.gamma - 1.0)); break;
-        case 1: case 3: cs = M.cs_init; break;  // constant: initializeSoundSpeed (soundspeed.cu:4-36)
-        case 9: cs = sqrt(M.gamma * p / rho); break;
-        case 12: cs = 0.0; break;
-        default: break;
-    }
-    switch (M.eos_type) {
-        case 0: p = M.K * pow(rho, M.gamma); break;
-        case 1: p = (M.bulk / M.n_exp) * (pow(rho / M.rho0, M.n_exp) - 1.0); break;
-        case 3: p = 41255.407 * rho; break;
-        case 9: p = (M.gamma - 1) * rho * S.e[s]; break;
-        case 12: p = cs * cs * rho; break;
-        default: break;
-    }
-    S.rho[s] = rho;
-    S.p[s] = p;
-    S.cs[s] = cs;
-    const int o = perm[s];
-    rho_out[o] = rho;
-    p_out[o] = p;
-    cs_out[o] = cs;
-}
-
-// ------------------------------------------------------------- Balsara
-// SPH::Kernel::CalcDivvandCurlv (src/sph/kernel.cu:223-342) and the factor of
-// internalForces (src/sph/internal_forces.cu:210-217):
-//   div v_i = sum_j m_j / rho_j (v_j - v_i) . grad W,
-//   curl v_i = sum_j m_j / rho_i (v_i - v_j) x grad W,
-//   f_i = |div v_i| / (|div v_i| + |curl v_i| + 1e-4 c_s,i / h_i),
-// grad W at h_i (h_bar only under VARIABLE_SML, as in the reference).
-__global__ void __launch_bounds__(kBlock) k_balsara(SphParams P, SphSorted S, const int* __restrict__ nbr,
-                                                    const int* __restrict__ noi, DevStatus* st) {
-    if (st->code) return;
-    const long s = (long)blockIdx.x * kBlock + threadIdx.x;
-    if (s >= P.n) return;
-    const double xi = S.x[s], yi = S.y[s], zi = S.z[s], hi = S.h[s];
-    const double vxi = S.vx[s], vyi = S.vy[s], vzi = S.vz[s], rhoi = S.rho[s];
-    double divv = 0.0, c0 = 0.0, c1 = 0.0, c2 = 0.0;
-    const int k = min(noi[s], P.maxnb);
-    for (int q = 0; q < k; ++q) {
-        const int j = nbr[nb_index(s, q, P.maxnb)];
-        const double hb = P.variable_sml ? 0.5 * (hi + __ldg(S.h + j)) : hi;
-        const double dx = xi - __ldg(S.x + j), dy = yi - __ldg(S.y + j), dz = zi - __ldg(S.z + j);
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        double W, dWdr;
-        skernel(P.kernel, r, hb, W, dWdr);
-        const double g = dWdr / r;
-        const double gx = g * dx, gy = g * dy, gz = g * dz;
-        const double dvx = vxi - __ldg(S.vx + j), dvy = vyi - __ldg(S.vy + j), dvz = vzi - __ldg(S.vz + j);
-        const double mj = __ldg(S.m + j);
-        divv += mj / __ldg(S.rho + j) * (-dvx * gx - dvy * gy - dvz * gz);
-        const double w = mj / rhoi;
-        c0 += w * (dvy * gz - dvz * gy);
-        c1 += w * (dvz * gx - dvx * gz);
-        c2 += w * (dvx * gy - dvy * gx);
-    }
-    const double curl = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-    S.bal[s] = fabs(divv) / (fabs(divv) + curl + 1e-4 * S.cs[s] / hi);
-}
-
-// ------------------------------------------------------------- forces
-// SPH::Kernel::internalForces, hydro part, SPH_EQU_VERSION 1
-// (src/sph/internal_forces.cu:372-552).
-__global__ void __launch_bounds__(kBlock) k_forces(SphParams P, SphSorted S, const int* __restrict__ nbr,
-                                                   const int* __restrict__ noi, const int* __restrict__ perm,
-                                                   double* ax_o, double* ay_o, double* az_o, double* drhodt_o,
-                                                   double* dedt_o, double* dsmldt_o, DevStatus* st) {
-    if (st->code) return;
-    const long s = (long)blockIdx.x * kBlock + threadIdx.x;
-    if (s >= P.n) return;
-    const double xi = S.x[s], yi = S.y[s], zi = S.z[s], hi = S.h[s];
-    const double vxi = S.vx[s], vyi = S.vy[s], vzi = S.vz[s];
-    const double rhoi = S.rho[s], pi = S.p[s], csi = S.cs[s];
-    const int mid = S.mat ? S.mat[s] : 0;
-    const double alpha = P.mat[mid].alpha, beta = P.mat[mid].beta;
-    const double pri = pi / (rhoi * rhoi);
-    double a0 = 0, a1 = 0, a2 = 0, drho = 0, de = 0, dh = 0;
-    const int k = min(noi[s], P.maxnb);
-    for (int q = 0; q < k; ++q) {
-        const int j = nbr[nb_index(s, q, P.maxnb)];
-        const double hj = __ldg(S.h + j);
-        const double hb = P.avg_h ? 0.5 * (hi + hj) : hi;
-        const double dx = xi - __ldg(S.x + j), dy = yi - __ldg(S.y + j), dz = zi - __ldg(S.z + j);
-        const double rr = dx * dx + dy * dy + dz * dz;
-        const double r = sqrt(rr);
-        double W, dWdr;
-        skernel(P.kernel, r, hb, W, dWdr);
-        const double g = dWdr / r;
-        const double gx = g * dx, gy = g * dy, gz = g * dz;
-        const double dvx = vxi - __ldg(S.vx + j), dvy = vyi - __ldg(S.vy + j), dvz = vzi - __ldg(S.vz + j);
-        const double vvnablaW = dvx * gx + dvy * gy + dvz * gz;
-        const double vr = dvx * dx + dvy * dy + dvz * dz;
-        const double rhoj = __ldg(S.rho + j), mj = __ldg(S.m + j);
-        double pij = 0.0;
-        if (vr < 0) {
-            const double csbar = 0.5 * (csi + __ldg(S.cs + j));
-            const double smooth = 0.5 * (hi + hj);
-            double mu = smooth * vr / (rr + smooth * smooth * 1e-2);
-            const double rhobar = 0.5 * (rhoi + rhoj);
-            if (P.balsara) mu *= (S.bal[s] + __ldg(S.bal + j)) / 2.;
-            pij = (beta * mu - alpha * csbar) * mu / rhobar;
-        }
-        const double pf = -mj * (pri + __ldg(S.p + j) / (rhoj * rhoj));
-        const double ajx = pf * gx, ajy = pf * gy, ajz = pf * gz;
-        const double vf = mj * (-pij);
-        a0 += ajx + vf * gx;
-        a1 += ajy + vf * gy;
-        a2 += ajz + vf * gz;
-        drho += rhoi / rhoj * mj * vvnablaW;
-        if (P.integrate_sml) dh -= 1. / 3. * hi * mj / rhoj * vvnablaW;
-        if (P.integrate_energy) de += 0.5 * mj * pij * vvnablaW - 0.5 * (ajx * dvx + ajy * dvy + ajz * dvz);
-    }
-    const int o = perm[s];
-    ax_o[o] = a0;
-    ay_o[o] = a1;
-    az_o[o] = a2;
-    if (drhodt_o) drhodt_o[o] = drho;
-    if (dedt_o) dedt_o[o] = P.integrate_energy ? de : 0.0;
-    if (dsmldt_o) dsmldt_o[o] = P.integrate_sml ? dh : 0.0;
-}
-
-// ----------------------------------------------- mixed precision (FP32 pairs)
-// Positions as FP32 hi/lo splits: x_hi = (float)x, x_lo = (float)(x - x_hi), so
-// that a neighbour difference (x_hi,i - x_hi,j) + (x_lo,i - x_lo,j) keeps FP32
-// relative accuracy of the difference itself at any distance from the origin.
-__global__ void k_pack_pos(SphSorted S, int n) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const double x = S.x[s], y = S.y[s], z = S.z[s];
-        const float hx = (float)x, hy = (float)y, hz = (float)z;
-        S.f0[s] = make_float4(hx, hy, hz, (float)S.h[s]);
-        S.f1[s] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz), (float)S.m[s]);
-    }
-}
-
-// EOS of one particle (calculateSoundSpeed, then calculatePressure, in the
-// reference's order: the ideal-gas sound speed uses the previous pressure)
-__device__ __forceinline__ void eos(const MatDev& M, double rho, double e, double& p, double& cs) {
-    switch (M.eos_type) {
-        case 0: cs = sqrt(M.K * pow(rho, M.gamma - 1.0)); break;
-        case 1: case 3: cs = M.cs_init; break;  // constant: initializeSoundSpeed (soundspeed.cu:4-36)
-        case 9: cs = sqrt(M.gamma * p / rho); break;
-        case 12: cs = 0.0; break;
-        default: break;
-    }
-    switch (M.eos_type) {
-        case 0: p = M.K * pow(rho, M.gamma); break;
-        case 1: p = (M.bulk / M.n_exp) * (pow(rho / M.rho0, M.n_exp) - 1.0); break;
-        case 3: p = 41255.407 * rho; break;
-        case 9: p = (M.gamma - 1) * rho * e; break;
-        case 12: p = cs * cs * rho; break;
-        default: break;
-    }
-}
-
-__global__ void __launch_bounds__(kBlock) k_density_eos_f32(SphParams P, SphSorted S, const int* __restrict__ nbr,
-                                                            const int* __restrict__ noi, const int* __restrict__ perm,
-                                                            double* rho_out, double* p_out, double* cs_out,
-                                                            DevStatus* st) {
-    if (st->code) return;
-    const long s = (long)blockIdx.x * kBlock + threadIdx.x;
-    if (s >= P.n) return;
-    double rho;
-    if (P.integrate_density) {
-        rho = S.rho[s];
-    } else {
-        const float4 a0 = S.f0[s], a1 = S.f1[s];
-        const float hi = a0.w;
-        float W, dWdr;
-        skernel_f(P.kernel, 0.f, hi, W, dWdr);
-        rho = (double)(a1.w * W);
-        const int k = min(noi[s], P.maxnb);
-        for (int q = 0; q < k; ++q) {
-            const int j = nbr[nb_index(s, q, P.maxnb)];
-            const float4 b0 = __ldg(S.f0 + j), b1 = __ldg(S.f1 + j);
-            const float3 d = rel_f(a0, a1, b0, b1);
-            const float r = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
-            skernel_f(P.kernel, r, P.avg_h ? 0.5f * (hi + b0.w) : hi, W, dWdr);
-            rho += (double)(b1.w * W);
-        }
-        if (!(rho > 0.0)) set_status(st, MHPC_ERR_NAN, (int)s);
-    }
-    const int mid = S.mat ? S.mat[s] : 0;
-    double p = S.p[s], cs = S.cs[s];
-    eos(P.mat[mid], rho, S.e[s], p, cs);
-    S.rho[s] = rho;
-    S.p[s] = p;
-    S.cs[s] = cs;
-    S.f2[s] = make_float4((float)S.vx[s], (float)S.vy[s], (float)S.vz[s], (float)cs);
-    S.f3[s] = make_float2((float)rho, (float)(p / (rho * rho)));
-    const int o = perm[s];
-    rho_out[o] = rho;
-    p_out[o] = p;
-    cs_out[o] = cs;
-}
-
-__global__ void __launch_bounds__(kBlock) k_forces_f32(SphParams P, SphSorted S, const int* __restrict__ nbr,
-                                                       const int* __restrict__ noi, const int* __restrict__ perm,
-                                                       double* ax_o, double* ay_o, double* az_o, double* drhodt_o,
-                                                       double* dedt_o, double* dsmldt_o, DevStatus* st) {
-    if (st->code) return;
-    const long s = (long)blockIdx.x * kBlock + threadIdx.x;
-    if (s >= P.n) return;
-    const float4 a0 = S.f0[s], a1 = S.f1[s], v = S.f2[s];
-    const float2 rp = S.f3[s];
-    const float hi = a0.w, csi = v.w, rhoi = rp.x, pri = rp.y;
-    const int mid = S.mat ? S.mat[s] : 0;
-    const float alpha = (float)P.mat[mid].alpha, beta = (float)P.mat[mid].beta;
-    const float bali = P.balsara ? (float)S.bal[s] : 1.f;
-    double a0x = 0, a0y = 0, a0z = 0, drho = 0, de = 0, dh = 0;
-    const int k = min(noi[s], P.maxnb);
-    for (int q = 0; q < k; ++q) {
-        const int j = nbr[nb_index(s, q, P.maxnb)];
-        const float4 b0 = __ldg(S.f0 + j), b1 = __ldg(S.f1 + j), w = __ldg(S.f2 + j);
-        const float2 rpj = __ldg(S.f3 + j);
-        const float hj = b0.w, mj = b1.w, rhoj = rpj.x;
-        const float3 d = rel_f(a0, a1, b0, b1);
-        const float rr = d.x * d.x + d.y * d.y + d.z * d.z;
-        const float r = sqrtf(rr);
-        float W, dWdr;
-        skernel_f(P.kernel, r, P.avg_h ? 0.5f * (hi + hj) : hi, W, dWdr);
-        const float g = __fdividef(dWdr, r);
-        const float gx = g * d.x, gy = g * d.y, gz = g * d.z;
-        const float dvx = v.x - w.x, dvy = v.y - w.y, dvz = v.z - w.z;
-        const float vvnablaW = dvx * gx + dvy * gy + dvz * gz;
-        const float vr = dvx * d.x + dvy * d.y + dvz * d.z;
-        float pij = 0.f;
-        if (vr < 0.f) {
-            const float csbar = 0.5f * (csi + w.w);
-            const float smooth = 0.5f * (hi + hj);
-            float mu = __fdividef(smooth * vr, rr + smooth * smooth * 1e-2f);
-            if (P.balsara) mu *= 0.5f * (bali + (float)__ldg(S.bal + j));
-            pij = __fdividef((beta * mu - alpha * csbar) * mu, 0.5f * (rhoi + rhoj));
-        }
-        const float pf = -mj * (pri + rpj.y);
-        const float ajx = pf * gx, ajy = pf * gy, ajz = pf * gz;
-        const float vf = -mj * pij;
-        a0x += (double)(ajx + vf * gx);
-        a0y += (double)(ajy + vf * gy);
-        a0z += (double)(ajz + vf * gz);
-        const float mv = __fdividef(mj, rhoj) * vvnablaW;
-        drho += (double)(rhoi * mv);
-        if (P.integrate_sml) dh -= (double)(1.f / 3.f * hi * mv);
-        if (P.integrate_energy) de += (double)(0.5f * mj * pij * vvnablaW - 0.5f * (ajx * dvx + ajy * dvy + ajz * dvz));
-    }
-    const int o = perm[s];
-    ax_o[o] = a0x;
-    ay_o[o] = a0y;
-    az_o[o] = a0z;
-    if (drhodt_o) drhodt_o[o] = drho;
-    if (dedt_o) dedt_o[o] = P.integrate_energy ? de : 0.0;
-    if (dsmldt_o) dsmldt_o[o] = P.integrate_sml ? dh : 0.0;
-}
-
 __global__ void k_export_nnl(int n, int maxnb, const int* __restrict__ nbr, const int* __restrict__ noi,
                              const int* __restrict__ perm, int* nnl, int* noi_out) {
     for (long s = blockIdx.x * (long)blockDim.x + threadIdx.x; s < n; s += (long)gridDim.x * blockDim.x) {
@@ -1000,46 +604,6 @@ int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, 
     rc = sph_sort_appended(P, nbr, noi, B.appended, s);
     if (rc) return rc;
     k_noi_stats<<<g, 256, 0, s>>>(P.n, P.maxnb, noi, st);
-    CUDA_TRY(cudaGetLastError());
-    return MHPC_OK;
-}
-
-int sph_density_eos(const SphParams& P, const SphSorted& S, const int* nbr, const int* noi, const int* perm,
-                    double* rho_out, double* p_out, double* cs_out, DevStatus* st, cudaStream_t s) {
-    if (P.n <= 0) return MHPC_OK;
-    if (P.mixed) {
-        if (!S.f0 || !S.f1 || !S.f2 || !S.f3) return MHPC_ERR_ARG;
-        k_pack_pos<<<grid_for(P.n, 256, 148 * 8), 256, 0, s>>>(S, P.n);
-        k_density_eos_f32<<<(P.n + kBlock - 1) / kBlock, kBlock, 0, s>>>(P, S, nbr, noi, perm, rho_out, p_out,
-                                                                        cs_out, st);
-        CUDA_TRY(cudaGetLastError());
-        return MHPC_OK;
-    }
-    k_density_eos<<<(P.n + kBlock - 1) / kBlock, kBlock, 0, s>>>(P, S, nbr, noi, perm, rho_out, p_out, cs_out, st);
-    CUDA_TRY(cudaGetLastError());
-    return MHPC_OK;
-}
-
-int sph_balsara(const SphParams& P, const SphSorted& S, const int* nbr, const int* noi, DevStatus* st,
-                cudaStream_t s) {
-    if (P.n <= 0) return MHPC_OK;
-    k_balsara<<<(P.n + kBlock - 1) / kBlock, kBlock, 0, s>>>(P, S, nbr, noi, st);
-    CUDA_TRY(cudaGetLastError());
-    return MHPC_OK;
-}
-
-int sph_forces(const SphParams& P, const SphSorted& S, const int* nbr, const int* noi, const int* perm, double* ax,
-               double* ay, double* az, double* drhodt, double* dedt, double* dsmldt, DevStatus* st, cudaStream_t s) {
-    if (P.n <= 0) return MHPC_OK;
-    if (P.mixed) {
-        if (!S.f0 || !S.f1 || !S.f2 || !S.f3) return MHPC_ERR_ARG;
-        k_forces_f32<<<(P.n + kBlock - 1) / kBlock, kBlock, 0, s>>>(P, S, nbr, noi, perm, ax, ay, az, drhodt, dedt,
-                                                                   dsmldt, st);
-        CUDA_TRY(cudaGetLastError());
-        return MHPC_OK;
-    }
-    k_forces<<<(P.n + kBlock - 1) / kBlock, kBlock, 0, s>>>(P, S, nbr, noi, perm, ax, ay, az, drhodt, dedt, dsmldt,
-                                                           st);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
 }

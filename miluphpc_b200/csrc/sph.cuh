@@ -34,11 +34,9 @@ struct SphSorted {
     const int* mat;        // may be null
     double *rho, *p, *cs;  // sorted outputs of the density/EOS pass (p, cs hold previous values on entry)
     double* bal;           // sorted Balsara factors (written by sph_balsara, read by sph_forces)
-    // FP32 pair-sum views (mixed precision), written by sph_density_eos:
-    // f0 = (x_hi, y_hi, z_hi, h), f1 = (x_lo, y_lo, z_lo, m) with x = x_hi + x_lo
-    // (FP32 split of the FP64 position), f2 = (vx, vy, vz, c_s), f3 = (rho, p/rho^2)
-    float4 *f0, *f1, *f2;
-    float2* f3;
+    // [n] 32-byte records of the pair sums (sph_pairs.cu), written by
+    // sph_density_eos, or by sph_forces on rho, p and c_s that it did not compute
+    void *ra, *rb, *rc;
 };
 
 // Squared distance without FMA contraction, summed in the reference's order
@@ -76,7 +74,7 @@ int sph_variable_h(const TreeDev& T, const SphParams& P, const double* x, const 
                    double* h, const VhBuffers& B, int target, int tol, int max_iter, int sweeps, DevStatus* st,
                    cudaStream_t s);
 // Density (kernel sum over the lists) + EOS.  P.mixed: the pair sums in FP32 on
-// hi/lo-split relative positions with FP64 accumulation (and the FP32 views
+// hi/lo-split relative positions with FP64 accumulation (and the records
 // of S filled for sph_forces); otherwise FP64 throughout.
 int sph_density_eos(const SphParams& P, const SphSorted& S, const int* nbr, const int* noi, const int* perm,
                     double* rho_out, double* p_out, double* cs_out, DevStatus* st, cudaStream_t s);
@@ -85,9 +83,9 @@ int sph_density_eos(const SphParams& P, const SphSorted& S, const int* nbr, cons
 // curl v from the neighbour lists, f_i into S.bal; after sph_density_eos.
 int sph_balsara(const SphParams& P, const SphSorted& S, const int* nbr, const int* noi, DevStatus* st,
                 cudaStream_t s);
-// Internal forces; P.mixed: pair terms in FP32 from the views sph_density_eos
-// filled, FP64 accumulation.
-int sph_forces(const SphParams& P, const SphSorted& S, const int* nbr, const int* noi, const int* perm,
+// Internal forces; P.mixed: pair terms in FP32, FP64 accumulation.  packed: the
+// records of S are those of the density pass of this tree and lists.
+int sph_forces(const SphParams& P, const SphSorted& S, bool packed, const int* nbr, const int* noi, const int* perm,
                double* ax, double* ay, double* az, double* drhodt, double* dedt, double* dsmldt, DevStatus* st,
                cudaStream_t s);
 // Scatter the sorted neighbour lists into the reference layout
