@@ -104,6 +104,51 @@ def test_keys_near_grid_points(lo, hi, curve, cuda):
     assert np.array_equal(box_keys(x, y, z, lo, hi, curve), O.keys(x, y, z, np.array([lo, hi] * 3), curve))
 
 
+# -------------------------------------------------------------------- sort
+def gpu_sort(keys, vals=None):
+    dev = torch.device("cuda:0")
+    n, L = len(keys), _lib.load()
+    kin = torch.as_tensor(keys.view(np.int64), device=dev)
+    vin = torch.as_tensor(vals, device=dev) if vals is not None else None
+    kout = torch.zeros(n, dtype=torch.int64, device=dev)
+    vout = torch.zeros(n, dtype=torch.int32, device=dev)
+    nb = L.mhpc_sort_scratch_bytes(n)
+    scratch = torch.zeros(nb, dtype=torch.uint8, device=dev)
+    _lib.check(L.mhpc_sort_pairs(dptr(kin), dptr(vin) if vin is not None else None, dptr(kout), dptr(vout), n,
+                                 dptr(scratch), nb, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "sort")
+    assert int(scratch[nb - 256:nb - 252].view(torch.int32).item()) == 0
+    return kout.cpu().numpy().view(np.uint64), vout.cpu().numpy()
+
+
+# one block up to 1024 and 4096 keys, look-back with tiles of 1024 up to 200,000 and
+# of 4096 up to 600,000, counted tiles of 2048 up to 6,000,000 and of 3072 above
+@pytest.mark.parametrize("n", [1, 2, 33, 1023, 1024, 1025, 4095, 4096, 4097, 5121, 199_999, 200_000, 200_001, 600_000,
+                               600_001, 1_000_003, 6_000_001])
+def test_sort_sizes(n, cuda):
+    """Stable ascending order over all 64 key bits, with and without values:
+    random keys, few distinct keys, keys equal to the largest, descending."""
+    rng = np.random.default_rng(n)
+    kinds = [rng.integers(0, 2 ** 64 - 1, n, dtype=np.uint64, endpoint=True),
+             rng.integers(0, 5, n).astype(np.uint64) << np.uint64(61),
+             np.where(rng.random(n) < 0.5, np.uint64(2 ** 64 - 1), rng.integers(0, 2 ** 63, n).astype(np.uint64)),
+             np.arange(n, 0, -1).astype(np.uint64) * np.uint64(3)]
+    for i, keys in enumerate(kinds):
+        vals = rng.permutation(n).astype(np.int32) if i % 2 else None
+        order = np.argsort(keys, kind="stable")
+        ks, vs = gpu_sort(keys, vals)
+        assert np.array_equal(ks, keys[order])
+        assert np.array_equal(vs, order.astype(np.int32) if vals is None else vals[order])
+
+
+def test_sort_scratch_serves_smaller_n(cuda):
+    """Scratch made for n keys is large enough for every smaller number."""
+    L = _lib.load()
+    sizes = sorted({1, 1000, 4096, 4097, 199_999, 200_000, 200_001, 300_000, 599_999, 600_000, 600_001, 1 << 20, 6_000_000,
+                    6_000_001, 1 << 24, 2_000_000_000})
+    b = [L.mhpc_sort_scratch_bytes(n) for n in sizes]
+    assert b == sorted(b)
+
+
 # ------------------------------------------------------------- upward pass
 # 4 positions per thread up to 8,192, 1 up to 65,536, 2 up to 200,000, 4 up to 2,000,000,
 # then 8; nodes are counted in one block up to 16,384
