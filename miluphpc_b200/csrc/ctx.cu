@@ -32,7 +32,6 @@ struct mhpc_ctx {
     DevStatus* st = nullptr;
     DevStatus* h_st = nullptr;
     long long* ord = nullptr;
-    double* bbox = nullptr;
     uint64_t* keys = nullptr;
     uint64_t* skey = nullptr;
     int* perm = nullptr;
@@ -198,7 +197,6 @@ int stage_tree_build(mhpc_ctx* c, const mhpc_particles* p) {
     const int n = p->n;
     cudaStream_t s = c->stream;
     TRY(launch_bbox(p->x, p->y, p->z, n, c->ord, c->st, s));
-    TRY(launch_bbox_finish(c->ord, c->bbox, s));
     TRY(launch_keys(p->x, p->y, p->z, n, c->ord, c->cfg.sfc, c->keys, nullptr, s));
     record(c, EV_KEYS);
     TRY(sort_pairs_u64(c->keys, nullptr, c->skey, c->perm, n, c->sort_scratch, c->sort_bytes, c->st, s));
@@ -569,7 +567,6 @@ int mhpc_ctx_create(mhpc_ctx** out, int capacity, const mhpc_config* cfg, const 
     A(c->st, 1);
     A(c->run, 1);
     A(c->ord, 2);
-    A(c->bbox, 6);
     A(c->keys, n);
     A(c->skey, n);
     A(c->perm, n);
@@ -1208,7 +1205,13 @@ int mhpc_get_stats(mhpc_ctx* c, mhpc_stats* o) {
         int total = 0;
         CUDA_TRY(cudaMemcpy(&total, c->T.nodes, sizeof(int), cudaMemcpyDeviceToHost));
         o->cells = total - c->last_n;
-        CUDA_TRY(cudaMemcpy(o->bbox, c->bbox, sizeof(double) * 6, cudaMemcpyDeviceToHost));
+        // the cubic box: one ordered (min, max) pair for all axes
+        long long ord[2];
+        CUDA_TRY(cudaMemcpy(ord, c->ord, sizeof(ord), cudaMemcpyDeviceToHost));
+        for (int d = 0; d < 3; ++d) {
+            o->bbox[2 * d] = ord_to_dbl(ord[0]);
+            o->bbox[2 * d + 1] = ord_to_dbl(ord[1]);
+        }
         o->radius = 0.5 * (o->bbox[1] - o->bbox[0]);
     }
     DevStatus& h = *c->h_st;

@@ -476,7 +476,8 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(const int* __restric
     if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_bsum(int* bsum, int nb) {
+// (also the scan's total)
+__global__ void __launch_bounds__(1024) k_scan_bsum(int* bsum, int nb, int* total) {
     __shared__ int sw[32];
     int carry = 0;
     for (int b0 = 0; b0 < nb; b0 += 1024) {
@@ -487,6 +488,7 @@ __global__ void __launch_bounds__(1024) k_scan_bsum(int* bsum, int nb) {
         if (i < nb) bsum[i] = carry + e;
         carry += tot;
     }
+    if (threadIdx.x == 0) *total = carry;
 }
 
 __global__ void __launch_bounds__(kScanBlock) k_scan_down(const int* __restrict__ in, int* out, int n,
@@ -516,12 +518,6 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_down(const int* __restrict_
         long idx = base + i * kScanBlock + threadIdx.x;
         if (idx < n) out[idx] = tile[i * kScanBlock + threadIdx.x];
     }
-}
-
-__global__ void k_scan_total(const int* __restrict__ in, int* out, int n) {
-    // out[n] = out[n-1] + in[n-1]
-    if (n > 0) out[n] = out[n - 1] + in[n - 1];
-    else out[0] = 0;
 }
 
 constexpr size_t align256c(size_t b) { return (b + 255) & ~size_t(255); }
@@ -671,9 +667,8 @@ int scan_exclusive_i32(const int* in, int* out, int n, void* scratch, cudaStream
     int nb = (int)(((long)n + kScanChunk - 1) / kScanChunk);
     int* bsum = (int*)scratch;
     k_scan_reduce<<<nb, kScanBlock, 0, s>>>(in, n, bsum);
-    k_scan_bsum<<<1, 1024, 0, s>>>(bsum, nb);
+    k_scan_bsum<<<1, 1024, 0, s>>>(bsum, nb, out + n);
     k_scan_down<<<nb, kScanBlock, 0, s>>>(in, out, n, bsum);
-    k_scan_total<<<1, 1, 0, s>>>(in, out, n);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
 }

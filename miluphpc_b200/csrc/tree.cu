@@ -19,24 +19,79 @@ namespace {
 
 __device__ __forceinline__ int dl_at(const unsigned char* dl, int i) { return i >= 0 ? (int)dl[i] : 0; }
 
-__global__ void __launch_bounds__(256) k_lcp(const uint64_t* __restrict__ k, int n, unsigned char* dl, int* cnt,
-                                             DevStatus* st) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int d = 0;
-        if (i + 1 < n) {
-            uint64_t x = __ldg(k + i) ^ __ldg(k + i + 1);
-            d = x == 0 ? MHPC_MAX_LEVEL : (__clzll((long long)x) - 1) / 3;
-            if (d > MHPC_MAX_LEVEL) d = MHPC_MAX_LEVEL;
-            if (x == 0) atomicAdd(&st->key_collisions, 1);
-        }
-        dl[i] = (unsigned char)d;
-    }
+// octal digits that sorted keys i and i + 1 share (0 past the ends)
+__device__ __forceinline__ int common_digits(uint64_t ka, uint64_t kb) {
+    const uint64_t x = ka ^ kb;
+    return x == 0 ? MHPC_MAX_LEVEL : min((__clzll((long long)x) - 1) / 3, MHPC_MAX_LEVEL);
 }
 
-__global__ void __launch_bounds__(256) k_count(const unsigned char* __restrict__ dl, int n, int* cnt) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int dp = dl_at(dl, i - 1), dc = dl[i];
-        cnt[i] = (dc > dp ? dc - dp : 0) + 1;
+// dl and the number of nodes (cells, then the leaf) that start at position i
+__device__ __forceinline__ int count_nodes(const uint64_t* __restrict__ k, int n, int i, unsigned char* dl,
+                                           DevStatus* st) {
+    const uint64_t ki = __ldg(k + i);
+    int d = 0;
+    if (i + 1 < n) {
+        const uint64_t kn = __ldg(k + i + 1);
+        d = common_digits(ki, kn);
+        if (ki == kn) atomicAdd(&st->key_collisions, 1);
+    }
+    const int dp = i > 0 ? common_digits(__ldg(k + i - 1), ki) : 0;
+    dl[i] = (unsigned char)d;
+    return (d > dp ? d - dp : 0) + 1;
+}
+
+__global__ void __launch_bounds__(256) k_lcp(const uint64_t* __restrict__ k, int n, unsigned char* dl, int* cnt,
+                                             DevStatus* st) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        cnt[i] = count_nodes(k, n, i, dl, st);
+}
+
+// The counts, their scan and the clearing of the nodes' child masks in one
+// block, for an n whose five launches (count, three of the scan, clear) take
+// longer than the work.
+constexpr int kSmallTreeN = 16384;
+constexpr int kSmallTreeBlock = 1024, kSmallTreePer = 4;
+
+__global__ void __launch_bounds__(kSmallTreeBlock) k_count_scan_small(TreeDev T, const uint64_t* __restrict__ k,
+                                                                      DevStatus* st) {
+    __shared__ int ws[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n = T.n;
+    int carry = 0;
+    for (int b0 = 0; b0 < n; b0 += kSmallTreeBlock * kSmallTreePer) {
+        const int i0 = b0 + threadIdx.x * kSmallTreePer;
+        int c[kSmallTreePer], sum = 0;
+#pragma unroll
+        for (int q = 0; q < kSmallTreePer; ++q) {
+            c[q] = i0 + q < n ? count_nodes(k, n, i0 + q, T.dl, st) : 0;
+            sum += c[q];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(MHPC_FULL, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) ws[w] = incl;
+        __syncthreads();
+        int v = ws[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(MHPC_FULL, v, o);
+            if (lane >= o) v += u;
+        }
+        int at = carry + incl - sum + (w > 0 ? __shfl_sync(MHPC_FULL, v, w - 1) : 0);
+        carry += __shfl_sync(MHPC_FULL, v, 31);
+#pragma unroll
+        for (int q = 0; q < kSmallTreePer; ++q) {
+            if (i0 + q < n) T.off[i0 + q] = at;
+            at += c[q];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) { T.off[n] = carry; *T.nodes = carry; }
+    for (int i = threadIdx.x; i < min(carry, T.cap_nodes); i += kSmallTreeBlock) {
+        T.kmask[i] = 0;
+        T.arrive[i] = 0;
     }
 }
 
@@ -141,17 +196,16 @@ __global__ void __launch_bounds__(256) k_nodes(TreeDev T, const uint64_t* __rest
 }
 
 __global__ void k_zero_cells(TreeDev T) {
-    // child masks of cells must be zero before k_nodes sets their bits; cells
+    // (and the node count.)  Child masks of cells must be zero before k_nodes sets their bits; cells
     // are the non-leaf nodes, whose ids are unknown before the scan, so clear all.
-    int total = *T.nodes;
+    int total = T.off[T.n];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *T.nodes = total;
     if (total > T.cap_nodes) total = T.cap_nodes;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         T.kmask[i] = 0;
         T.arrive[i] = 0;
     }
 }
-
-__global__ void k_copy_total(TreeDev T) { *T.nodes = T.off[T.n]; }
 
 __device__ __forceinline__ float rd(double v) { return __double2float_rd(v); }
 __device__ __forceinline__ float ru(double v) { return __double2float_ru(v); }
@@ -593,13 +647,14 @@ int tree_build(TreeDev& T, const uint64_t* skey, void* scan_scratch, DevStatus* 
     const int n = T.n;
     if (n <= 0) return MHPC_ERR_ARG;
     const int g = grid_for(n, 256, 148 * 16);
-    k_lcp<<<g, 256, 0, s>>>(skey, n, T.dl, T.cnt, st);
-    k_count<<<g, 256, 0, s>>>(T.dl, n, T.cnt);
-    CUDA_TRY(cudaGetLastError());
-    int rc = scan_exclusive_i32(T.cnt, T.off, n, scan_scratch, s);
-    if (rc) return rc;
-    k_copy_total<<<1, 1, 0, s>>>(T);
-    k_zero_cells<<<148 * 8, 256, 0, s>>>(T);
+    if (n <= kSmallTreeN) {
+        k_count_scan_small<<<1, kSmallTreeBlock, 0, s>>>(T, skey, st);
+    } else {
+        k_lcp<<<g, 256, 0, s>>>(skey, n, T.dl, T.cnt, st);
+        int rc = scan_exclusive_i32(T.cnt, T.off, n, scan_scratch, s);
+        if (rc) return rc;
+        k_zero_cells<<<148 * 8, 256, 0, s>>>(T);
+    }
     k_nodes<<<g, 256, 0, s>>>(T, skey, st);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
