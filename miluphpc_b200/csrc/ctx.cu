@@ -192,6 +192,15 @@ int check_particles(const mhpc_ctx* c, const mhpc_particles* p) {
     return MHPC_OK;
 }
 
+// Bytes of the gathered fields from which the gather goes by way of records.
+// Gather and tree build in us by fields / by records, particles in random order:
+// 4 fields, 2^20 / 4,000,000 / 2^23 / 2^24: 116 / 472 / 1111 / 2430 and 112 / 404 /
+// 843 / 1746; 8 fields, 2^20 / 2^21 / 4,000,000: 151 / 351 / 787 and 138 / 263 /
+// 493.  In an order that the curve mostly follows already (a lattice's rows) the
+// records lose: 10 fields, 2^21: 265 and 280, so the line is kept above the sizes
+// whose fields L2 (126 MB) half holds.
+constexpr long kRecordBytes = 192L << 20;
+
 // bounding box, keys, sort, gather into SFC order, tree build
 int stage_tree_build(mhpc_ctx* c, const mhpc_particles* p) {
     const int n = p->n;
@@ -235,7 +244,12 @@ int stage_tree_build(mhpc_ctx* c, const mhpc_particles* p) {
             L.isrc = p->material_id; L.idst = c->smat; L.imax = c->nmat; L.st = c->st;
         }
     }
-    TRY(launch_gather(n, c->perm, L, s));
+    // scratch for records: the potential's four doubles per particle, with SPH
+    // the three records of the pair sums (both written only later)
+    double4* rec = c->cfg.sph ? c->ra : L.count <= 4 ? reinterpret_cast<double4*>(c->pot_scratch) : nullptr;
+    // records pay once the fields are well beyond L2 (kRecordBytes)
+    if (rec && 8L * L.count * n >= kRecordBytes) TRY(launch_gather_records(n, c->perm, L, rec, s));
+    else TRY(launch_gather(n, c->perm, L, s));
     c->T.n = n;
     TRY(tree_build(c->T, c->skey, c->scan_scratch, c->st, s));
     record(c, EV_TREE);
@@ -594,7 +608,9 @@ int mhpc_ctx_create(mhpc_ctx** out, int capacity, const mhpc_config* cfg, const 
     if (cfg->sph) {
         A(c->svx, n); A(c->svy, n); A(c->svz, n); A(c->se, n); A(c->srho, n); A(c->sp, n); A(c->scs, n);
         A(c->sbal, n);
-        A(c->ra, n); A(c->rb, n); A(c->rc, n);
+        A(c->ra, 3 * n);  // (one block: also the gather's scratch)
+        c->rb = c->ra + n;
+        c->rc = c->rb + n;
         A(c->smat, n);
         size_t groups = (n + 31) / 32;
         A(c->nbr, groups * 32 * (size_t)c->maxnb);

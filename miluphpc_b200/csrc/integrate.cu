@@ -5,6 +5,15 @@
 
 namespace {
 
+__device__ __forceinline__ int gathered_id(const GatherList& L, int o) {
+    int v = __ldg(L.isrc + o);
+    if (L.imax > 0 && (v < 0 || v >= L.imax)) {
+        if (L.st) set_status(L.st, MHPC_ERR_ARG, o);
+        v = v < 0 ? 0 : L.imax - 1;
+    }
+    return v;
+}
+
 // Every field's load is issued before the first store: the destination
 // arrays may alias the sources as far as the compiler knows, so a load after
 // a store would wait for the previous load's value (one round trip per field).
@@ -18,14 +27,45 @@ __global__ void __launch_bounds__(256) k_gather(int n, const int* __restrict__ p
 #pragma unroll
         for (int a = 0; a < MHPC_GATHER_MAX; ++a)
             if (a < L.count) L.dst[a][s] = v[a];
-        if (L.isrc) {
-            int v = __ldg(L.isrc + o);
-            if (L.imax > 0 && (v < 0 || v >= L.imax)) {
-                if (L.st) set_status(L.st, MHPC_ERR_ARG, o);
-                v = v < 0 ? 0 : L.imax - 1;
-            }
-            L.idst[s] = v;
-        }
+        if (L.isrc) L.idst[s] = gathered_id(L, o);
+    }
+}
+
+// The gather in two steps for arrays that L2 does not hold: the fields first go
+// into records of 4 R doubles in the caller's order (streaming), and the
+// permuted read is then one or two whole DRAM bursts per particle instead of
+// one 8-byte read per field, of which DRAM moves 64 bytes each.
+// Bound: DRAM; at 2^24 gravity particles the tree stage (gather, node counts,
+// nodes) 2430 us with one read per field, 1746 us with records.
+template <int R>
+__global__ void __launch_bounds__(256) k_pack_records(int n, GatherList L, double4* __restrict__ rec) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+        double v[4 * R];
+#pragma unroll
+        for (int a = 0; a < 4 * R; ++a) v[a] = a < L.count ? __ldg(L.src[a] + i) : 0.0;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(rec + R * i + r), "d"(v[4 * r]),
+                         "d"(v[4 * r + 1]), "d"(v[4 * r + 2]), "d"(v[4 * r + 3])
+                         : "memory");
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) k_gather_records(int n, const int* __restrict__ perm, GatherList L,
+                                                        const double4* __restrict__ rec) {
+    for (long s = blockIdx.x * (long)blockDim.x + threadIdx.x; s < n; s += (long)gridDim.x * blockDim.x) {
+        const int o = __ldg(perm + s);
+        double v[4 * R];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                : "=d"(v[4 * r]), "=d"(v[4 * r + 1]), "=d"(v[4 * r + 2]), "=d"(v[4 * r + 3])
+                : "l"(rec + R * (long)o + r));
+#pragma unroll
+        for (int a = 0; a < 4 * R; ++a)
+            if (a < L.count) L.dst[a][s] = v[a];
+        if (L.isrc) L.idst[s] = gathered_id(L, o);
     }
 }
 
@@ -475,6 +515,24 @@ int launch_gather(int n, const int* perm, const GatherList& L, cudaStream_t s) {
     k_gather<<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(n, perm, L);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
+}
+
+namespace {
+template <int R>
+int gather_records(int n, const int* perm, const GatherList& L, double4* rec, cudaStream_t s) {
+    k_pack_records<R><<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(n, L, rec);
+    k_gather_records<R><<<grid_for(n, 256, 148 * 16), 256, 0, s>>>(n, perm, L, rec);
+    CUDA_TRY(cudaGetLastError());
+    return MHPC_OK;
+}
+}  // namespace
+
+int launch_gather_records(int n, const int* perm, const GatherList& L, double4* rec, cudaStream_t s) {
+    if (n <= 0) return MHPC_OK;
+    if (L.count <= 4) return gather_records<1>(n, perm, L, rec, s);
+    if (L.count <= 8) return gather_records<2>(n, perm, L, rec, s);
+    if (L.count <= 12) return gather_records<3>(n, perm, L, rec, s);
+    return MHPC_ERR_ARG;
 }
 
 int launch_scatter(int n, const int* perm, const GatherList& L, cudaStream_t s) {

@@ -15,6 +15,9 @@ struct GatherList {
 };
 
 int launch_gather(int n, const int* perm, const GatherList& L, cudaStream_t s);
+// The gather by way of records of ceil(count / 4) double4 per particle in `rec`
+// (scratch); count <= 12.
+int launch_gather_records(int n, const int* perm, const GatherList& L, double4* rec, cudaStream_t s);
 int launch_scatter(int n, const int* perm, const GatherList& L, cudaStream_t s);
 int launch_leapfrog_x(const mhpc_particles& p, double dt, cudaStream_t s);
 int launch_leapfrog_v(const mhpc_particles& p, double dt, cudaStream_t s);
