@@ -10,12 +10,11 @@
 // selection among their candidates (all other h frozen), and the pairs whose
 // status changes are removed from or appended to both lists.
 //
-// Kernels of one round: flags + scan + compaction (out-of-band list),
-// k_band_select (selection, one warp per particle: a tree walk below the band,
+// Kernels of one round: k_band_list (out-of-band list), k_band_select (selection, one warp per particle: a tree walk below the band,
 // the particle's own list above it), k_band_events (one event per changed
 // pair, likewise), k_band_mark + k_band_filter (removals: the marked lists
 // re-tested with the new h), k_band_add, k_band_commit.  Every kernel after the
-// compaction reads the list length on the device and returns at once when it
+// first reads the list length on the device and returns at once when it
 // is zero, so the host enqueues all rounds without synchronising.
 #include "sph.cuh"
 #include "walk.cuh"
@@ -60,21 +59,26 @@ struct SelectVisit {
     }
 };
 
-// Out-of-band list of this round; in round 0 its length is recorded as the
-// count before any repair.
-__global__ void k_band_flags(int n, const int* __restrict__ noi, BandRule R, int* flags) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        flags[i] = R.out(noi[i]) ? 1 : 0;
+// hnew = h0 = h, no list marked, all counters zero.
+__global__ void k_band_init(int n, const double* __restrict__ h, double* hnew, double* h0, int* dirty, int* ctr) {
+    if (blockIdx.x == 0 && threadIdx.x < kBandCtr) ctr[threadIdx.x] = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double v = h[i];
+        hnew[i] = v;
+        h0[i] = v;
+        dirty[i] = 0;
+    }
 }
 
-__global__ void k_band_compact_list(int n, const int* __restrict__ flags, const int* __restrict__ off, int* list,
-                                    int* ctr, DevStatus* st, int round) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        if (flags[i]) list[off[i]] = i;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctr[0] = 0;  // events
-        ctr[1] = 0;  // overflow
-        if (round == 0) st->sml_band_before = off[n];
+// Out-of-band list of this round, in any order (every particle's selection,
+// pair changes and commit depend on it alone), and the event counters reset.
+__global__ void __launch_bounds__(256) k_band_list(int n, const int* __restrict__ noi, BandRule R, int* list,
+                                                   int* count, int* ctr) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[0] = ctr[1] = 0;
+    const int step = gridDim.x * blockDim.x;
+    for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += step) {
+        const int i = i0 + threadIdx.x;
+        warp_append(i < n && R.out(noi[i]), i, list, count);
     }
 }
 
@@ -270,65 +274,60 @@ __global__ void __launch_bounds__(kBandBlock) k_band_events(TreeDev T, const dou
     }
 }
 
-// Removals: both ends of every removal event are marked; each marked list is
+// Removals: both ends of every removal event are marked and listed; each marked list is
 // then filtered with the pair test of the new h (d < min(h_i', h_j'), the list
 // walk's test), which drops exactly the pairs the events removed (every pair
 // in a list was present with the old h, and a pair whose status did not change
 // passes).  One warp per marked list, order kept (ballot compaction).
-__global__ void k_band_mark(const int2* __restrict__ ev, const int* __restrict__ ctr, int cap, int* dirty,
+__global__ void k_band_mark(const int2* __restrict__ ev, int* ctr, int cap, int* dirty, int* dlist,
                             const int* skip = nullptr) {
     if (ctr[1] || (skip && *skip)) return;
     const int m = min(ctr[0], cap);
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
-        const int2 v = ev[e];
-        if (v.x >= 0) continue;
-        dirty[~v.x] = 1;
-        dirty[v.y] = 1;
+    const int step = gridDim.x * blockDim.x;
+    for (int e0 = blockIdx.x * blockDim.x; e0 < m; e0 += step) {
+        const int e = e0 + threadIdx.x;
+        const int2 v = e < m ? ev[e] : make_int2(0, 0);
+        const bool removal = e < m && v.x < 0;
+        warp_append(removal && atomicExch(dirty + ~v.x, 1) == 0, ~v.x, dlist, ctr + kBandDirty);
+        warp_append(removal && atomicExch(dirty + v.y, 1) == 0, v.y, dlist, ctr + kBandDirty);
     }
 }
 
-__global__ void k_band_filter(int n, const int* __restrict__ ctr, const double* __restrict__ sx,
-                              const double* __restrict__ sy, const double* __restrict__ sz,
-                              const double* __restrict__ hn, int* nbr, int* noi, int maxnb, int* dirty,
-                              const int* skip = nullptr) {
+__global__ void k_band_filter(const int* __restrict__ dlist, const int* __restrict__ ctr,
+                              const double* __restrict__ sx, const double* __restrict__ sy,
+                              const double* __restrict__ sz, const double* __restrict__ hn, int* nbr, int* noi,
+                              int maxnb, int* dirty, const int* skip = nullptr) {
     if (ctr[1] || (skip && *skip)) return;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-    for (long base = warp * 32; base < n; base += nwarps * 32) {
-        const long me = base + lane;
-        const bool mark = me < n && dirty[me];
-        unsigned todo = __ballot_sync(MHPC_FULL, mark);
-        if (mark) dirty[me] = 0;
-        while (todo) {
-            const int b = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const long a = base + b;
-            const int k = min(noi[a], maxnb);
-            const double px = sx[a], py = sy[a], pz = sz[a], ha = hn[a];
-            const double ha2 = ha * ha;
-            int w = 0;
-            for (int q0 = 0; q0 < k; q0 += 32) {
-                const int q = q0 + lane;
-                int j = -1;
-                bool keep = false;
-                if (q < k) {
-                    j = nbr[nb_index(a, q, maxnb)];
-                    const double d2 = d2_exact(px - __ldg(sx + j), py - __ldg(sy + j), pz - __ldg(sz + j));
-                    const double hj = hn[j];
-                    keep = d2 < ha2 && d2 < hj * hj;
-                }
-                const unsigned bk = __ballot_sync(MHPC_FULL, keep);
-                // entries are only moved towards the front: slot w + rank <= q
-                __syncwarp();
-                if (keep) nbr[nb_index(a, w + __popc(bk & lt), maxnb)] = j;
-                w += __popc(bk);
-                __syncwarp();
+    const int m = ctr[kBandDirty];
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < m; b += nwarps) {
+        const long a = dlist[b];
+        if (lane == 0) dirty[a] = 0;
+        const int k = min(noi[a], maxnb);
+        const double px = sx[a], py = sy[a], pz = sz[a], ha = hn[a];
+        const double ha2 = ha * ha;
+        int w = 0;
+        for (int q0 = 0; q0 < k; q0 += 32) {
+            const int q = q0 + lane;
+            int j = -1;
+            bool keep = false;
+            if (q < k) {
+                j = nbr[nb_index(a, q, maxnb)];
+                const double d2 = d2_exact(px - __ldg(sx + j), py - __ldg(sy + j), pz - __ldg(sz + j));
+                const double hj = hn[j];
+                keep = d2 < ha2 && d2 < hj * hj;
             }
-            if (lane == 0) noi[a] = w;
+            const unsigned bk = __ballot_sync(MHPC_FULL, keep);
+            // entries are only moved towards the front: slot w + rank <= q
+            __syncwarp();
+            if (keep) nbr[nb_index(a, w + __popc(bk & lt), maxnb)] = j;
+            w += __popc(bk);
             __syncwarp();
         }
+        if (lane == 0) noi[a] = w;
+        __syncwarp();
     }
 }
 
@@ -345,8 +344,9 @@ __device__ __forceinline__ void append(int* nbr, int* noi, int maxnb, int a, int
 // Appends land in atomic order: both ends are marked in `appended` and their
 // lists sorted afterwards (k_sort_appended), so that the lists, and the sums
 // over them, do not depend on the order in which the events ran.
-__global__ void k_band_add(const int2* __restrict__ ev, const int* __restrict__ ctr, int cap, int* nbr, int* noi,
-                           int maxnb, DevStatus* st, int* appended, int* trunc = nullptr) {
+__global__ void k_band_add(const int2* __restrict__ ev, int* ctr, int cap, int* nbr, int* noi, int maxnb,
+                           DevStatus* st, int* appended, int* trunc = nullptr) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[kBandDirty] = 0;  // (the filter is done with its list)
     if (ctr[1] || (trunc && *trunc)) return;
     const int m = min(ctr[0], cap);
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
@@ -410,26 +410,22 @@ __global__ void k_sort_appended(int n, int* appended, int* nbr, const int* __res
 }
 
 // The round's new h, or (event buffer overflow: no list was edited) the old
-// ones back into hnew.
-__global__ void k_band_commit(const int* __restrict__ list, const int* __restrict__ list_count,
-                              const int* __restrict__ ctr, double* h, double* hnew, DevStatus* st) {
+// ones back into hnew; the next round's list count is zeroed, and round 0
+// records its own as the count before any repair.
+__global__ void k_band_commit(const int* __restrict__ list, const int* __restrict__ list_count, int* next_count,
+                              const int* __restrict__ ctr, double* h, double* hnew, DevStatus* st, int round) {
     const int m = *list_count;
     const bool ok = ctr[1] == 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *next_count = 0;
+        if (round == 0) st->sml_band_before = m;
+    }
     if (!ok && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->sml_band_skipped, 1);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
         const int i = list[q];
         if (ok) h[i] = hnew[i];
         else hnew[i] = h[i];
     }
-}
-
-__global__ void k_copy_h(int n, const double* __restrict__ a, double* b) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = a[i];
-}
-
-__global__ void k_reset_events(int* ctr) {
-    ctr[0] = 0;
-    ctr[1] = 0;
 }
 
 }  // namespace
@@ -445,12 +441,10 @@ int sph_apply_h_changes(const TreeDev& T, const SphParams& P, const double* x, c
                         const double* h, const double* hnew, int* nbr, int* noi, const int* list,
                         const int* list_count, const BandBuffers& B, int* trunc, DevStatus* st, cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
-    const int g = grid_for(P.n, 256, 148 * 16);
-    k_reset_events<<<1, 1, 0, s>>>(B.ctr);
     k_band_events<<<148 * 8, kBandBlock, 0, s>>>(T, x, y, z, h, hnew, noi, nbr, P.maxnb, list, list_count, T.hmax,
                                                  B.events, B.cap_events, B.ctr, st, trunc);
-    k_band_mark<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, B.dirty, trunc);
-    k_band_filter<<<148 * 8, 128, 0, s>>>(P.n, B.ctr, x, y, z, hnew, nbr, noi, P.maxnb, B.dirty, trunc);
+    k_band_mark<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, B.dirty, B.dlist, trunc);
+    k_band_filter<<<148 * 8, 128, 0, s>>>(B.dlist, B.ctr, x, y, z, hnew, nbr, noi, P.maxnb, B.dirty, trunc);
     k_band_add<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, nbr, noi, P.maxnb, st, B.appended, trunc);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
@@ -461,25 +455,21 @@ int sph_band_fixup(const TreeDev& T, const SphParams& P, const double* x, const 
                    DevStatus* st, cudaStream_t s) {
     if (P.n <= 0 || rounds <= 0) return MHPC_OK;
     const int n = P.n;
-    const int g = grid_for(n, 256, 148 * 16);
-    const int* list_count = B.off + n;
+    const int g = grid_for(n, 256, 148 * 8);
     BandRule R{target, tol};
-    CUDA_TRY(cudaMemsetAsync(B.dirty, 0, sizeof(int) * n, s));
-    k_copy_h<<<g, 256, 0, s>>>(n, h, B.hnew);
-    k_copy_h<<<g, 256, 0, s>>>(n, h, B.h0);
+    k_band_init<<<g, 256, 0, s>>>(n, h, B.hnew, B.h0, B.dirty, B.ctr);
     for (int r = 0; r < rounds; ++r) {
-        k_band_flags<<<g, 256, 0, s>>>(n, noi, R, B.flags);
-        int rc = scan_exclusive_i32(B.flags, B.off, n, B.scan_scratch, s);
-        if (rc) return rc;
-        k_band_compact_list<<<g, 256, 0, s>>>(n, B.flags, B.off, B.list, B.ctr, st, r);
+        int* list_count = B.ctr + kBandCount + (r & 1);
+        k_band_list<<<g, 256, 0, s>>>(n, noi, R, B.list, list_count, B.ctr);
         k_band_select<<<148 * 8, kBandBlock, 0, s>>>(T, x, y, z, h, B.h0, noi, nbr, P.maxnb, B.list, list_count, R,
                                                      P.ord, B.hnew, T.hmax, st);
         k_band_events<<<148 * 8, kBandBlock, 0, s>>>(T, x, y, z, h, B.hnew, noi, nbr, P.maxnb, B.list, list_count,
                                                      T.hmax, B.events, B.cap_events, B.ctr, st);
-        k_band_mark<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, B.dirty);
-        k_band_filter<<<148 * 8, 128, 0, s>>>(n, B.ctr, x, y, z, B.hnew, nbr, noi, P.maxnb, B.dirty);
+        k_band_mark<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, B.dirty, B.dlist);
+        k_band_filter<<<148 * 8, 128, 0, s>>>(B.dlist, B.ctr, x, y, z, B.hnew, nbr, noi, P.maxnb, B.dirty);
         k_band_add<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, nbr, noi, P.maxnb, st, B.appended);
-        k_band_commit<<<148 * 4, 256, 0, s>>>(B.list, list_count, B.ctr, h, B.hnew, st);
+        k_band_commit<<<148 * 4, 256, 0, s>>>(B.list, list_count, B.ctr + kBandCount + ((r + 1) & 1), B.ctr, h, B.hnew,
+                                              st, r);
     }
     k_sort_appended<<<148 * 4, 256, 0, s>>>(n, B.appended, nbr, noi, P.maxnb);
     CUDA_TRY(cudaGetLastError());

@@ -340,9 +340,8 @@ int stage_frnn(mhpc_ctx* c, const mhpc_particles* p, bool variable_h, bool learn
     const int target = sph_target(c);
     c->frnn_learned = learned && variable_h;
     if (variable_h) {
-        CUDA_TRY(cudaMemsetAsync(c->vh_done, 0, sizeof(int) * n, s));
-        CUDA_TRY(cudaMemsetAsync(c->vh_nit, 0xff, sizeof(int) * n, s));  // nit starts at -1
-        CUDA_TRY(cudaMemcpyAsync(c->h_start, c->sh, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+        if (learned)
+            CUDA_TRY(cudaMemcpyAsync(c->h_start, c->sh, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
         // learned path: start the iteration from the predicted h; particles whose
         // prediction lands in the band stop after the first sweep
         if (learned) TRY(mlp_apply_prediction(c->mlp, c->perm, c->sh, n, s));
@@ -355,7 +354,7 @@ int stage_frnn(mhpc_ctx* c, const mhpc_particles* p, bool variable_h, bool learn
             BandBuffers E;
             std::memset(&E, 0, sizeof(E));
             E.dirty = c->vh_count; E.hnew = c->hold; E.events = c->band_ev; E.cap_events = c->band_cap;
-            E.ctr = c->band_ctr; E.scan_scratch = c->scan_scratch; E.appended = c->nb_appended;
+            E.ctr = c->band_ctr; E.dlist = c->vh_flags; E.appended = c->nb_appended;
             TRY(sph_variable_h_lists(c->T, P, c->sx, c->sy, c->sz, c->sh, c->nbr, c->noi, B, E, target,
                                      c->cfg.nb_tolerance, c->cfg.max_sml_iterations,
                                      c->cfg.max_sml_iterations + 2, c->st, s));
@@ -363,12 +362,14 @@ int stage_frnn(mhpc_ctx* c, const mhpc_particles* p, bool variable_h, bool learn
             TRY(sph_variable_h(c->T, P, c->sx, c->sy, c->sz, c->sh, B, target, c->cfg.nb_tolerance,
                                c->cfg.max_sml_iterations, c->cfg.max_sml_iterations + 2, c->st, s));
         }
-        GatherList L;
-        std::memset(&L, 0, sizeof(L));
-        L.count = 1;
-        L.src[0] = c->sh;
-        L.dst[0] = p->sml;
-        TRY(launch_scatter(n, c->perm, L, s));
+        if (c->cfg.sml_band_rounds <= 0) {  // (else after the repair)
+            GatherList L;
+            std::memset(&L, 0, sizeof(L));
+            L.count = 1;
+            L.src[0] = c->sh;
+            L.dst[0] = p->sml;
+            TRY(launch_scatter(n, c->perm, L, s));
+        }
         if (learned)
             TRY(mlp_collect(c->mlp, c->perm, c->h_start, c->sh, MHPC_VH_LISTS ? c->noi : c->vh_count, c->vh_nit,
                             target, c->cfg.nb_tolerance, c->cfg.max_sml_iterations, n, s));
@@ -382,8 +383,8 @@ int stage_frnn(mhpc_ctx* c, const mhpc_particles* p, bool variable_h, bool learn
         // counts that drifted out of the band: repaired on the lists, then the
         // final h goes back to the caller's order
         BandBuffers B;
-        B.flags = c->vh_flags; B.off = c->vh_off; B.list = c->vh_list; B.dirty = c->vh_done; B.hnew = c->hold;
-        B.events = c->band_ev; B.cap_events = c->band_cap; B.ctr = c->band_ctr; B.scan_scratch = c->scan_scratch;
+        B.dlist = c->vh_flags; B.list = c->vh_list; B.dirty = c->vh_done; B.hnew = c->hold;
+        B.events = c->band_ev; B.cap_events = c->band_cap; B.ctr = c->band_ctr;
         B.h0 = c->band_h0;
         B.appended = c->nb_appended;
         TRY(sph_band_fixup(c->T, P, c->sx, c->sy, c->sz, c->sh, c->nbr, c->noi, B, target, c->cfg.nb_tolerance,
@@ -622,7 +623,7 @@ int mhpc_ctx_create(mhpc_ctx** out, int capacity, const mhpc_config* cfg, const 
         // (room for 4 per particle: a round that needs more is skipped and counted)
         c->band_cap = (int)std::min<size_t>(2147483000, std::max<size_t>(4096, 4 * n));
         A(c->band_ev, c->band_cap);
-        A(c->band_ctr, 4);
+        A(c->band_ctr, kBandCtr);
         A(c->band_h0, n);
         A(c->nb_appended, n);
     }

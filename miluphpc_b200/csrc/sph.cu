@@ -10,6 +10,8 @@
 // its own candidates with the reference's pair rule d^2 < h_i^2 && d^2 < h_j^2
 // (j != i), d^2 formed without FMA contraction like the reference build.  All
 // pruning is conservative, so the neighbour set equals the brute-force set.
+#include <algorithm>
+
 #include "sph.cuh"
 #include "walk.cuh"
 
@@ -86,18 +88,15 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
     const int M = *T.nodes;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    const long g = ((long)blockIdx.x * kBlock + threadIdx.x) >> 5;
-    long s = g * 32 + lane;
-    bool valid = s < n;
-    if (MODE == 1) {
-        const long cnt_list = *list_count;
-        if (g * 32 >= cnt_list) return;  // whole warp beyond the list
-        valid = s < cnt_list;
-        s = valid ? list[s] : 0;
-    }
-    const bool active = valid;
-    if (!__any_sync(MHPC_FULL, active)) return;
     FrnnSmem& S = smem[w];
+    const long total = MODE == 1 ? (long)*list_count : (long)n;
+    // one group per warp (a gated re-walk that mostly returns at once has a
+    // smaller grid and takes several)
+    for (long g = ((long)blockIdx.x * kBlock + threadIdx.x) >> 5; g * 32 < total; g += (long)gridDim.x * kWarps) {
+    long s = g * 32 + lane;
+    const bool valid = s < total;
+    if (MODE == 1) s = valid ? list[s] : 0;
+    const bool active = valid;
     double px = 0, py = 0, pz = 0, hi = 0;
     if (valid) { px = sx[s]; py = sy[s]; pz = sz[s]; hi = sh[s]; }
     const double hi2 = hi * hi;
@@ -318,6 +317,7 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
         for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(MHPC_FULL, tot, o);
         if (lane == 0) atomicAdd(&st->noi_sum, tot);
     }
+    }
 }
 
 // Count walk for sparse lists (later variable-h sweeps, where the particles
@@ -373,8 +373,11 @@ __global__ void __launch_bounds__(kBlock) k_count_warp(TreeDev T, const double* 
 // into the snapshot too (hold), and a larger h raises the largest-h bound of
 // the particle's leaf and ancestors (grow-only, stopping at the first ancestor
 // already as large; a bound left larger than the subtree's h only prunes less).
-__global__ void k_vh_update(const int* __restrict__ list, const int* __restrict__ list_count,
-                            const int* __restrict__ count, double* h, double* hold, int* done, int* nit, int target,
+// *next_count (when given) is zeroed; at sweep 1 of the list form the particles
+// still iterating are recorded (the fallback count when the first sweep started
+// from predicted smoothing lengths).
+__global__ void k_vh_update(const int* __restrict__ list, const int* __restrict__ list_count, int* next_count,
+                            DevStatus* record, int n, const int* __restrict__ count, double* h, double* hold, int* done, int* nit, int target,
                             int tol, int max_iter, int maxnb, float* node_hmax, const int* __restrict__ leaf_node,
                             const int* __restrict__ parent, const long long* __restrict__ ord) {
     const int m = *list_count;
@@ -384,6 +387,10 @@ __global__ void k_vh_update(const int* __restrict__ list, const int* __restrict_
     // steps (the reference has no such bound); at the box edge its search
     // already covers every particle.
     const double hcap = ord_to_dbl(ord[1]) - ord_to_dbl(ord[0]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (next_count) *next_count = 0;
+        if (record) { record->predictor_fallback = m; record->predictor_used = n - m; }
+    }
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
         const int i = list[q];
         const int it = ++nit[i];
@@ -415,13 +422,6 @@ __global__ void k_compact(int n, const int* __restrict__ flags, const int* __res
         if (flags[i]) list[off[i]] = i;
 }
 
-// number of particles still iterating after the first sweep (the fallback
-// count when the first sweep started from predicted smoothing lengths)
-__global__ void k_record_active(const int* __restrict__ list_count, int n, DevStatus* st) {
-    st->predictor_fallback = *list_count;
-    st->predictor_used = n - *list_count;
-}
-
 __global__ void k_record_unconverged(const int* __restrict__ list_count, DevStatus* st) {
     st->sml_unconverged = *list_count;
 }
@@ -430,34 +430,49 @@ __global__ void k_copy(int n, const double* __restrict__ a, double* b) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = a[i];
 }
 
-// The particles of `in` that have not stopped, appended to `out` (order
-// irrelevant: every particle's update and pair edits depend on it alone, and
-// the appended lists are sorted at the end); *out_count must be zero.
-__global__ void k_next_list(const int* __restrict__ in, const int* __restrict__ in_count,
-                            const int* __restrict__ done, int* out, int* out_count) {
-    const int m = *in_count;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
-        const int i = in[q];
-        if (!done[i]) out[atomicAdd(out_count, 1)] = i;
+// Start of the iteration: every state array and counter, and the list of all
+// particles.
+__global__ void k_vh_init(int n, const double* __restrict__ h, double* hnew, int* done, int* nit, int* dirty, int* list,
+                          int* list_count, int* ctr) {
+    if (blockIdx.x == 0 && threadIdx.x < kBandCtr) ctr[threadIdx.x] = threadIdx.x == 3 ? 1 : 0;  // the first walk runs
+    if (blockIdx.x == 0 && threadIdx.x == 0) *list_count = n;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        hnew[i] = h[i];
+        done[i] = 0;
+        nit[i] = -1;
+        dirty[i] = 0;
+        list[i] = i;
     }
 }
 
-// End of a sweep on lists: every iterating particle takes its new h; the
-// lists are re-walked when they are truncated (a count above maxnb) or when
-// the sweep's pair changes overflowed the event buffer (nothing was edited).
+// End of a sweep on lists: every iterating particle takes its new h, and the
+// particles that have not stopped form the next list (in any order: every
+// particle's update and pair edits depend on it alone, and the appended lists
+// are sorted at the end); the lists are re-walked when they are truncated (a
+// count above maxnb) or when the sweep's pair changes overflowed the event
+// buffer (nothing was edited).
 __global__ void k_vh_commit(const int* __restrict__ list, const int* __restrict__ list_count,
-                            const double* __restrict__ hnew, double* h, const int* __restrict__ ctr, int* rewalk) {
+                            const double* __restrict__ hnew, double* h, const int* __restrict__ done, int* next,
+                            int* next_count, int* ctr) {
     const int m = *list_count;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *rewalk = (ctr[1] || ctr[2]) ? 1 : 0;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
-        const int i = list[q];
-        h[i] = hnew[i];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctr[3] = (ctr[1] || ctr[2]) ? 1 : 0;
+        ctr[0] = ctr[1] = 0;
+    }
+    const int step = gridDim.x * blockDim.x;
+    for (int q0 = blockIdx.x * blockDim.x; q0 < m; q0 += step) {
+        const int q = q0 + threadIdx.x;
+        const int i = q < m ? list[q] : 0;
+        if (q < m) h[i] = hnew[i];
+        warp_append(q < m && !done[i], i, next, next_count);
     }
 }
 
 // Statistics and the capacity check of the list walk, for lists that the
 // variable-h iteration kept current instead of a final walk.
-__global__ void k_noi_stats(int n, int maxnb, const int* __restrict__ noi, DevStatus* st) {
+__global__ void k_noi_stats(int n, int maxnb, const int* __restrict__ noi, const int* __restrict__ unconverged,
+                            DevStatus* st) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->sml_unconverged = *unconverged;
     int mx = 0;
     unsigned long long tot = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -518,6 +533,8 @@ int sph_variable_h(const TreeDev& T, const SphParams& P, const double* x, const 
     const int* list_count = B.off + P.n;
     // Jacobi snapshot of h and the largest-h bounds; k_vh_update keeps both
     // current from then on
+    CUDA_TRY(cudaMemsetAsync(B.done, 0, sizeof(int) * P.n, s));
+    CUDA_TRY(cudaMemsetAsync(B.nit, 0xff, sizeof(int) * P.n, s));  // nit starts at -1
     k_copy<<<g, 256, 0, s>>>(P.n, h, B.hold);
     int rc0 = tree_node_hmax(T, B.hold, st, s);
     if (rc0) return rc0;
@@ -527,7 +544,6 @@ int sph_variable_h(const TreeDev& T, const SphParams& P, const double* x, const 
         int rc = scan_exclusive_i32(B.flags, B.off, P.n, B.scan_scratch, s);
         if (rc) return rc;
         k_compact<<<g, 256, 0, s>>>(P.n, B.flags, B.off, B.list);
-        if (it == 1) k_record_active<<<1, 1, 0, s>>>(list_count, P.n, st);
         if (it == 0) {
             // first sweep: (nearly) every particle, group walks
             k_frnn<1><<<(int)blocks, kBlock, 0, s>>>(T, P.n, P.maxnb, x, y, z, B.hold, B.list, list_count, T.hmax,
@@ -536,7 +552,7 @@ int sph_variable_h(const TreeDev& T, const SphParams& P, const double* x, const 
             // later sweeps: the few particles still iterating, a warp each
             k_count_warp<<<148 * 8, kBlock, 0, s>>>(T, x, y, z, B.hold, B.list, list_count, T.hmax, B.count, st);
         }
-        k_vh_update<<<g, 256, 0, s>>>(B.list, list_count, B.count, h, B.hold, B.done, B.nit, target, tol, max_iter,
+        k_vh_update<<<g, 256, 0, s>>>(B.list, list_count, nullptr, it == 1 ? st : nullptr, P.n, B.count, h, B.hold, B.done, B.nit, target, tol, max_iter,
                                       P.maxnb, T.hmax, T.leaf_node, T.parent, P.ord);
     }
     k_flags<<<g, 256, 0, s>>>(P.n, B.done, B.flags);
@@ -553,57 +569,37 @@ int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, 
     if (P.n <= 0) return MHPC_OK;
     const long blocks = (((long)P.n + 31) / 32 * 32 + kBlock - 1) / kBlock;
     const int g = grid_for(P.n, 256, 148 * 16);
-    const int* list_count = V.off + P.n;
     int* trunc = B.ctr + 2;   // some list holds fewer entries than its count
     int* rewalk = B.ctr + 3;  // the lists are re-walked after this sweep
     double* hnew = B.hnew;
-    CUDA_TRY(cudaMemsetAsync(B.ctr, 0, sizeof(int) * 4, s));
-    CUDA_TRY(cudaMemsetAsync(rewalk, 1, sizeof(int), s));  // nonzero: the first walk runs
-    CUDA_TRY(cudaMemsetAsync(B.dirty, 0, sizeof(int) * P.n, s));
-    k_copy<<<g, 256, 0, s>>>(P.n, h, hnew);
+    k_vh_init<<<g, 256, 0, s>>>(P.n, h, hnew, V.done, V.nit, B.dirty, V.list, V.cnt, B.ctr);
     int rc = tree_node_hmax(T, h, st, s);
     if (rc) return rc;
     // the lists and counts of the starting h: the counts of the first sweep
     k_frnn<2><<<(int)blocks, kBlock, 0, s>>>(T, P.n, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi, st,
                                               rewalk, trunc);
-    // the first sweep lists every particle (ordered, by a scan); later sweeps
-    // keep the particles of the previous list that have not stopped
-    k_flags<<<g, 256, 0, s>>>(P.n, V.done, V.flags);
-    rc = scan_exclusive_i32(V.flags, V.off, P.n, V.scan_scratch, s);
-    if (rc) return rc;
-    k_compact<<<g, 256, 0, s>>>(P.n, V.flags, V.off, V.list);
-    const int* cur = V.list;
-    const int* cur_count = list_count;
+    // gated re-walks: several groups per warp, so that the launch that finds
+    // nothing to do has few blocks to retire
+    const long gated = std::min(blocks, std::max(148L * MHPC_FRNN_MIN_BLOCKS, blocks / 8));
     for (int it = 0; it < sweeps; ++it) {
-        if (it > 0) {
-            int* out = (it & 1) ? V.list2 : V.list;
-            int* out_count = V.cnt + (it & 1);
-            CUDA_TRY(cudaMemsetAsync(out_count, 0, sizeof(int), s));
-            k_next_list<<<g, 256, 0, s>>>(cur, cur_count, V.done, out, out_count);
-            cur = out;
-            cur_count = out_count;
-        }
-        if (it == 1) k_record_active<<<1, 1, 0, s>>>(cur_count, P.n, st);
+        // the first sweep lists every particle, a later one those that have not stopped
+        const int* cur = (it & 1) ? V.list2 : V.list;
+        int* next = (it & 1) ? V.list : V.list2;
+        const int* cur_count = V.cnt + (it & 1);
+        int* next_count = V.cnt + ((it + 1) & 1);
         // the reference's update from the exact counts of the current h (Jacobi:
         // every new h goes to hnew first)
-        k_vh_update<<<g, 256, 0, s>>>(cur, cur_count, noi, hnew, hnew, V.done, V.nit, target, tol, max_iter,
-                                      P.maxnb, T.hmax, T.leaf_node, T.parent, P.ord);
+        k_vh_update<<<g, 256, 0, s>>>(cur, cur_count, next_count, it == 1 ? st : nullptr, P.n, noi, hnew, hnew, V.done,
+                                      V.nit, target, tol, max_iter, P.maxnb, T.hmax, T.leaf_node, T.parent, P.ord);
         rc = sph_apply_h_changes(T, P, x, y, z, h, hnew, nbr, noi, cur, cur_count, B, trunc, st, s);
         if (rc) return rc;
-        k_vh_commit<<<g, 256, 0, s>>>(cur, cur_count, hnew, h, B.ctr, rewalk);
-        k_frnn<2><<<(int)blocks, kBlock, 0, s>>>(T, P.n, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi,
-                                                  st, rewalk, trunc);
-    }
-    {
-        int* out = (sweeps & 1) ? V.list2 : V.list;
-        int* out_count = V.cnt + (sweeps & 1);
-        CUDA_TRY(cudaMemsetAsync(out_count, 0, sizeof(int), s));
-        k_next_list<<<g, 256, 0, s>>>(cur, cur_count, V.done, out, out_count);
-        k_record_unconverged<<<1, 1, 0, s>>>(out_count, st);
+        k_vh_commit<<<g, 256, 0, s>>>(cur, cur_count, hnew, h, V.done, next, next_count, B.ctr);
+        k_frnn<2><<<(int)gated, kBlock, 0, s>>>(T, P.n, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi, st,
+                                                 rewalk, trunc);
     }
     rc = sph_sort_appended(P, nbr, noi, B.appended, s);
     if (rc) return rc;
-    k_noi_stats<<<g, 256, 0, s>>>(P.n, P.maxnb, noi, st);
+    k_noi_stats<<<grid_for(P.n, 256, 148 * 4), 256, 0, s>>>(P.n, P.maxnb, noi, V.cnt + (sweeps & 1), st);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
 }

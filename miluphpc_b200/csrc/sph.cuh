@@ -56,7 +56,7 @@ int sph_frnn(const TreeDev& T, const SphParams& P, const SphSorted& S, int* nbr,
              cudaStream_t s);
 struct VhBuffers {
     double* hold;        // [n] Jacobi snapshot
-    int* done;           // [n] converged (zeroed by the caller before the first sweep)
+    int* done;           // [n] converged
     int* nit;            // [n] iteration counters (-1 before the first sweep)
     int* count;          // [n] neighbour counts of the last sweep
     int* flags;          // [n] scratch
@@ -107,17 +107,17 @@ int sph_export_nnl(const SphParams& P, const int* nbr, const int* noi, const int
 // it holds too few).  All such particles move
 // at once, and the neighbour lists and counts are edited in place pair by
 // pair, so they equal a fresh list walk on the new h.
+constexpr int kBandDirty = 4, kBandCount = 5, kBandCtr = 8;
 struct BandBuffers {
-    int* flags;          // [n] scratch (particles out of the band)
-    int* off;            // [n+1] scratch (scan); off[n] = particles out of the band
+    int* dlist;          // [n] lists with removed entries
     int* list;           // [n] particles out of the band
-    int* dirty;          // [n] lists with removed entries (zeroed here)
+    int* dirty;          // [n] marks of the lists in dlist
     double* hnew;        // [n] new h (equal to h outside a round)
     double* h0;          // [n] h before the first round
     int2* events;        // [cap_events] pair changes (x >= 0: add (x, y); x < 0: remove (~x, y))
     int cap_events;
-    int* ctr;            // [4] events, overflow flag
-    void* scan_scratch;
+    int* ctr;            // [kBandCtr] events, overflow flag, truncated, re-walk (variable h), length of
+                         // dlist, lengths of alternating rounds' lists
     int* appended;       // [n] lists that received appends (zero outside the calls; cleared by the sort)
 };
 // Sort the lists marked in `appended` by neighbour index and clear the marks.
@@ -129,8 +129,9 @@ int sph_band_fixup(const TreeDev& T, const SphParams& P, const double* x, const 
 // The pair changes of moving every particle of `list` from h to hnew, applied
 // to the lists and counts in place (events, removals, compaction, appends);
 // with `trunc` (variable-h iteration) nothing runs while *trunc is set, and a
-// list that would pass maxnb sets it.  ctr[0..1] are reset here; ctr[1]
-// reports an event-buffer overflow (no list edited).
+// list that would pass maxnb sets it.  The caller zeroes ctr[0..1] and
+// ctr[kBandDirty] before; ctr[1] reports an event-buffer overflow (no list
+// edited).
 int sph_apply_h_changes(const TreeDev& T, const SphParams& P, const double* x, const double* y, const double* z,
                         const double* h, const double* hnew, int* nbr, int* noi, const int* list,
                         const int* list_count, const BandBuffers& B, int* trunc, DevStatus* st, cudaStream_t s);

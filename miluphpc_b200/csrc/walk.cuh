@@ -3,6 +3,18 @@
 #pragma once
 #include "sph.cuh"
 
+// v appended to list by the lanes that want it, one atomic per warp.  All
+// lanes of the warp call it.
+__device__ __forceinline__ void warp_append(bool want, int v, int* list, int* count) {
+    const unsigned b = __ballot_sync(MHPC_FULL, want);
+    if (b == 0) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(b) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(count, __popc(b));
+    base = __shfl_sync(MHPC_FULL, base, leader);
+    if (want) list[base + __popc(b & ((1u << lane) - 1u))] = v;
+}
+
 constexpr int kWalkStack = 512;
 constexpr int kWalkReserve = 7 * 22 + 8;
 constexpr int kWalkSmall = 16;   // cells with at most this many particles are tested whole
