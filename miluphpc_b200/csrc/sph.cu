@@ -26,27 +26,41 @@ constexpr int kSmall = 16;    // cells with at most this many particles are stag
 // four sub-groups of 8 lanes.
 //
 // Traversal: lane-parallel over a per-warp stack in shared memory.  Every
-// step pops up to 32 nodes, one per lane; a node whose particle box misses
-// the group's search box (union of [x - h, x + h]), or whose box grown by
-// its largest h misses the group's points box, is dropped; leaves, cells of
+// step pops up to 32 nodes, one per lane; a node whose particle box is farther
+// from the box of the group's particles than the group's largest h, or than
+// the largest h below the node, is dropped; leaves, cells of
 // at most kSmall particles and shared-key buckets become candidate ranges;
 // other cells push their children.  Stack bound as in the gravity list walk:
 // a pop of k nodes pushes at most 8k, and k is limited so that a depth-first
 // descent (7 per level, 22 levels) always fits on top of the stack.
 //
 // Candidates: the ranges are expanded 32 at a time; each candidate particle
-// is tested against the four sub-groups' boxes (search box, and points box
-// grown by h_j when smoothing lengths differ), both rounded outward to FP32
-// like the node boxes, so no pair that passes the exact test is dropped.
-// Candidates reaching some sub-group go to a shared-memory pool (x, y, z,
-// h_j^2, j) and to that sub-group's list.  A full pool is flushed: for each
-// sub-group, lane (8q + p) tests particle p of the sub-group against list
-// entry 4c + q, so the warp tests 32 pairs per step, and hits are written in
-// list order (ballot prefix over the 4 lanes of a particle).
+// is tested against the four sub-groups: its distance from the sub-group's box
+// must be below h_j and the sub-group's largest h, both with the rounding of
+// the FP32 offsets on top, so no pair that passes the exact test is dropped.
+// (Distances, not boxes grown by h: a box of side s grown by r on all sides
+// holds (s + 2 r)^3, the points within r of it a quarter less at s = 0.75 r,
+// and the pairs to test are proportional to that.)
+// Candidates reaching some sub-group go to a shared-memory pool (x, y, z
+// relative to the group's centre and h_j^2, in FP32, and j) and to that
+// sub-group's list.  A full pool is flushed: for each sub-group, lane (8q + p)
+// tests particle p of the sub-group against list entry 4c + q, so the warp
+// tests 32 pairs per step, and hits are written in list order (ballot prefix
+// over the 4 lanes of a particle).
 //
 // The pair rule is the reference's, d^2 < h_i^2 && d^2 < h_j^2 (j != i), d^2
-// formed without FMA contraction; the walk and the box tests are
-// conservative, so each neighbour set equals the brute-force set.
+// formed without FMA contraction in FP64.  The flush forms d^2 in FP32 and
+// settles the pairs whose d^2 is farther from min(h_i^2, h_j^2) than the FP32
+// error; the few others are tested exactly.  With H the group's largest h and
+// R its half edge plus H (the reach of every candidate), offsets
+// are off by 2^-24 R each, so d^2 for d <= 2 H by less than 8.3e-7 R H +
+// 1.3e-6 H^2, and a pair farther apart cannot come within that of H^2 while
+// R < 1e5 H.  The walk and the box tests are conservative too, so each
+// neighbour set equals the brute-force set.
+// Bound: issue and fixed latency (58 % of the issue slots, 18 resident warps per
+// SM).  List walk in us with FP64 tests and grown boxes / now: Sedov lattice of
+// 262,144 particles 258 / 236, of 2,097,152 1693 / 1510; all walks of a cloud step,
+// 2^20 particles 2229 / 1843, 2^23 16600 / 13850.
 //
 // mode 0: write lists (h_i = h[i], h_j = h[j]) for all particles; mode 1:
 // count only, with h_i = h[i], h_j = h[j] (the variable-h sweep passes the
@@ -61,12 +75,11 @@ constexpr int kPool = 128;
 
 struct FrnnSmem {
     int stk[kStack];
-    double cx[kPool], cy[kPool], cz[kPool], ch2[kPool];  // candidate position, h_j^2
+    float4 cp[kPool];                                     // candidate: offset from the centre, h_j^2
     int cj[kPool];                                        // candidate particle
     unsigned char lst[4][kPool];                          // pool slots per sub-group
     int rf[32], rend[32];                                 // staged ranges: first, end (prefix)
-    float4 slo[4], shi[4];                                // sub-group search boxes
-    float4 plo[4], phi[4];                                // sub-group points boxes
+    float4 slo[4], shi[4];                                // sub-group boxes about the centre; largest h (.w)
 };
 
 #ifndef MHPC_FRNN_MIN_BLOCKS
@@ -100,38 +113,46 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
     double px = 0, py = 0, pz = 0, hi = 0;
     if (valid) { px = sx[s]; py = sy[s]; pz = sz[s]; hi = sh[s]; }
     const double hi2 = hi * hi;
-    // search box (x +- h) and points box, reduced over the sub-group (8
-    // lanes), stored rounded outward, then over the warp
-    double lx = active ? px - hi : 1e300, ly = active ? py - hi : 1e300, lz = active ? pz - hi : 1e300;
-    double ux = active ? px + hi : -1e300, uy = active ? py + hi : -1e300, uz = active ? pz + hi : -1e300;
+    // points box and largest h over the sub-group (8 lanes), then over the warp
+    double hm = active ? hi : 0.0, shm = 0.0;
+    double sl[3] = {}, su[3] = {};  // the sub-group's box
     double plx = active ? px : 1e300, ply = active ? py : 1e300, plz = active ? pz : 1e300;
     double pux = active ? px : -1e300, puy = active ? py : -1e300, puz = active ? pz : -1e300;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        lx = fmin(lx, __shfl_xor_sync(MHPC_FULL, lx, o));
-        ly = fmin(ly, __shfl_xor_sync(MHPC_FULL, ly, o));
-        lz = fmin(lz, __shfl_xor_sync(MHPC_FULL, lz, o));
-        ux = fmax(ux, __shfl_xor_sync(MHPC_FULL, ux, o));
-        uy = fmax(uy, __shfl_xor_sync(MHPC_FULL, uy, o));
-        uz = fmax(uz, __shfl_xor_sync(MHPC_FULL, uz, o));
         plx = fmin(plx, __shfl_xor_sync(MHPC_FULL, plx, o));
         ply = fmin(ply, __shfl_xor_sync(MHPC_FULL, ply, o));
         plz = fmin(plz, __shfl_xor_sync(MHPC_FULL, plz, o));
         pux = fmax(pux, __shfl_xor_sync(MHPC_FULL, pux, o));
         puy = fmax(puy, __shfl_xor_sync(MHPC_FULL, puy, o));
         puz = fmax(puz, __shfl_xor_sync(MHPC_FULL, puz, o));
-        if (o == 4 && (lane & 7) == 0) {
-            const int q = lane >> 3;
-            S.slo[q] = make_float4(__double2float_rd(lx), __double2float_rd(ly), __double2float_rd(lz), 0.f);
-            S.shi[q] = make_float4(__double2float_ru(ux), __double2float_ru(uy), __double2float_ru(uz), 0.f);
-            S.plo[q] = make_float4(__double2float_rd(plx), __double2float_rd(ply), __double2float_rd(plz), 0.f);
-            S.phi[q] = make_float4(__double2float_ru(pux), __double2float_ru(puy), __double2float_ru(puz), 0.f);
+        hm = fmax(hm, __shfl_xor_sync(MHPC_FULL, hm, o));
+        if (o == 4) {
+            sl[0] = plx; sl[1] = ply; sl[2] = plz; su[0] = pux; su[1] = puy; su[2] = puz;
+            shm = hm;
         }
     }
-    const float qlx = __double2float_rd(lx), qly = __double2float_rd(ly), qlz = __double2float_rd(lz);
-    const float qux = __double2float_ru(ux), quy = __double2float_ru(uy), quz = __double2float_ru(uz);
-    const float rlx = __double2float_rd(plx), rly = __double2float_rd(ply), rlz = __double2float_rd(plz);
-    const float rux = __double2float_ru(pux), ruy = __double2float_ru(puy), ruz = __double2float_ru(puz);
+    const float3 g0 = make_float3(__double2float_rd(plx), __double2float_rd(ply), __double2float_rd(plz));
+    const float3 g1 = make_float3(__double2float_ru(pux), __double2float_ru(puy), __double2float_ru(puz));
+    const double cx = 0.5 * (plx + pux), cy = 0.5 * (ply + puy), cz = 0.5 * (plz + puz);
+    const float fx = (float)(px - cx), fy = (float)(py - cy), fz = (float)(pz - cz), fh2 = (float)hi2;
+    const float H = __double2float_ru(hm);
+    const float R = 1.00001f * ((float)fmax(fmax(pux - cx, puy - cy), puz - cz) + H);
+    // |d^2(FP32) - min(h_i^2, h_j^2)| up to which the exact test decides, and what
+    // the rounding of the offsets adds to a distance; at scales where the bounds
+    // do not hold, every candidate goes to every sub-group's exact test
+    const bool scaled = H > 1e-15f && R < 1e15f && R < 1e5f * H;
+    const float band = scaled ? 1e-6f * R * H + 1.6e-6f * H * H : INFINITY;
+    const float slack = scaled ? 3e-7f * R : INFINITY;
+    // a sub-group's box about the centre, and its largest h
+    if ((lane & 7) == 0) {
+        const int q = lane >> 3;
+        const float ax = __double2float_rd(sl[0] - cx), ay = __double2float_rd(sl[1] - cy), az = __double2float_rd(sl[2] - cz);
+        const float bx = __double2float_ru(su[0] - cx), by = __double2float_ru(su[1] - cy), bz = __double2float_ru(su[2] - cz);
+        const bool any = shm > 0.0;
+        S.slo[q] = make_float4(ax, ay, az, any ? 1.000001f * __double2float_ru(shm) + slack : -1.f);
+        S.shi[q] = make_float4(bx, by, bz, 0.f);
+    }
     int k = 0;     // neighbours found for this lane's particle
     int pool = 0;  // pool entries (warp-uniform)
     int cnt0 = 0, cnt1 = 0, cnt2 = 0, cnt3 = 0;  // list entries per sub-group (warp-uniform)
@@ -142,8 +163,8 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
         for (int sg = 0; sg < 4; ++sg) {
             const int cntg = sg == 0 ? cnt0 : sg == 1 ? cnt1 : sg == 2 ? cnt2 : cnt3;
             const int src = 8 * sg + p;
-            const double ix = __shfl_sync(MHPC_FULL, px, src), iy = __shfl_sync(MHPC_FULL, py, src);
-            const double iz = __shfl_sync(MHPC_FULL, pz, src), ih2 = __shfl_sync(MHPC_FULL, hi2, src);
+            const float ix = __shfl_sync(MHPC_FULL, fx, src), iy = __shfl_sync(MHPC_FULL, fy, src);
+            const float iz = __shfl_sync(MHPC_FULL, fz, src), ih2 = __shfl_sync(MHPC_FULL, fh2, src);
             const int is = __shfl_sync(MHPC_FULL, (int)s, src);
             const bool iact = __shfl_sync(MHPC_FULL, (int)active, src) != 0;
             int kb = __shfl_sync(MHPC_FULL, k, src);
@@ -155,9 +176,16 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
                 if (iact && c < cntg) {
                     const int slot = S.lst[sg][c];
                     j = S.cj[slot];
-                    const double dx = ix - S.cx[slot], dy = iy - S.cy[slot], dz = iz - S.cz[slot];
-                    const double d = d2_exact(dx, dy, dz);
-                    hit = j != is && d < ih2 && d < S.ch2[slot];
+                    const float4 q4 = S.cp[slot];
+                    const float dx = ix - q4.x, dy = iy - q4.y, dz = iz - q4.z;
+                    const float over = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - fminf(ih2, q4.w);
+                    hit = over < -band;
+                    if (!hit && !(over > band)) {
+                        const double hs = sh[is], hj = sh[j];
+                        const double d = d2_exact(sx[is] - sx[j], sy[is] - sy[j], sz[is] - sz[j]);
+                        hit = d < hs * hs && d < hj * hj;
+                    }
+                    hit = hit && j != is;
                 }
                 const unsigned b = __ballot_sync(MHPC_FULL, hit) & pmask;
                 if (MODE != 1 && hit) {
@@ -195,13 +223,9 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
         if (act) {
             const int2 lk = __ldg(T.link + nd);
             const float4 bl = __ldg(T.bmin + nd), bh = __ldg(T.bmax + nd);
-            bool overlap = !(bh.x < qlx || bl.x > qux || bh.y < qly || bl.y > quy || bh.z < qlz || bl.z > quz);
-            if (overlap && node_hmax) {
-                const float hn = __ldg(node_hmax + nd);
-                overlap = !(__fadd_ru(bh.x, hn) < rlx || __fadd_rd(bl.x, -hn) > rux || __fadd_ru(bh.y, hn) < rly ||
-                            __fadd_rd(bl.y, -hn) > ruy || __fadd_ru(bh.z, hn) < rlz || __fadd_rd(bl.z, -hn) > ruz);
-            }
-            if (overlap) {
+            // a pair needs d < h_i and d < h_j: the boxes must come within both
+            const float lim = node_hmax ? fminf(H, __ldg(node_hmax + nd)) : H;
+            if (box_gap2(g0, g1, bl, bh) <= __fmul_ru(lim, lim)) {
                 rf = __ldg(T.first + nd);
                 if (lk.y & ND_LEAF) {
                     rlen = 1;
@@ -259,7 +283,8 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
             if (pool + 32 > kPool) flush();
             const int c = c0 + lane;
             int mask = 0, j = 0;
-            double qx = 0, qy = 0, qz = 0, hj = 0;
+            float rx = 0.f, ry = 0.f, rz = 0.f;
+            double hj = 0;
             if (c < ncand) {
                 int lo = 0, hi_r = nr - 1;
                 while (lo < hi_r) {
@@ -268,28 +293,24 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
                     else lo = mid + 1;
                 }
                 j = S.rf[lo] + c - (lo ? S.rend[lo - 1] : 0);
-                qx = __ldg(sx + j); qy = __ldg(sy + j); qz = __ldg(sz + j); hj = __ldg(sh + j);
-                const float xd = __double2float_rd(qx), xu = __double2float_ru(qx);
-                const float yd = __double2float_rd(qy), yu = __double2float_ru(qy);
-                const float zd = __double2float_rd(qz), zu = __double2float_ru(qz);
-                const float hf = __double2float_ru(hj);
+                const double qx = __ldg(sx + j), qy = __ldg(sy + j), qz = __ldg(sz + j);
+                hj = __ldg(sh + j);
+                rx = (float)(qx - cx); ry = (float)(qy - cy); rz = (float)(qz - cz);
+                const float hf = 1.000001f * (float)hj + slack;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float4 a = S.slo[q], b = S.shi[q];
-                    bool in = !(xu < a.x || xd > b.x || yu < a.y || yd > b.y || zu < a.z || zd > b.z);
-                    if (node_hmax) {
-                        const float4 e = S.plo[q], f = S.phi[q];
-                        in = in && !(__fadd_ru(xu, hf) < e.x || __fadd_rd(xd, -hf) > f.x ||
-                                     __fadd_ru(yu, hf) < e.y || __fadd_rd(yd, -hf) > f.y ||
-                                     __fadd_ru(zu, hf) < e.z || __fadd_rd(zd, -hf) > f.z);
-                    }
-                    mask |= (int)in << q;
+                    const float gx = fmaxf(fmaxf(a.x - rx, rx - b.x), 0.f), gy = fmaxf(fmaxf(a.y - ry, ry - b.y), 0.f),
+                                gz = fmaxf(fmaxf(a.z - rz, rz - b.z), 0.f);
+                    const float lim = fminf(a.w, hf);
+                    mask |= (int)(lim > 0.f && fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= lim * lim) << q;
                 }
             }
             const unsigned bp = __ballot_sync(MHPC_FULL, mask != 0);
             if (mask) {
                 const int slot = pool + __popc(bp & lt);
-                S.cx[slot] = qx; S.cy[slot] = qy; S.cz[slot] = qz; S.ch2[slot] = hj * hj; S.cj[slot] = j;
+                S.cp[slot] = make_float4(rx, ry, rz, (float)(hj * hj));
+                S.cj[slot] = j;
                 const unsigned b0 = __ballot_sync(bp, mask & 1), b1 = __ballot_sync(bp, mask & 2);
                 const unsigned b2 = __ballot_sync(bp, mask & 4), b3 = __ballot_sync(bp, mask & 8);
                 if (mask & 1) S.lst[0][cnt0 + __popc(b0 & lt)] = (unsigned char)slot;

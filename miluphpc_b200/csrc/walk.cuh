@@ -3,6 +3,15 @@
 #pragma once
 #include "sph.cuh"
 
+// Lower bound (every step rounded down) of the squared distance between the
+// boxes [al, ah] and [bl, bh].
+__device__ __forceinline__ float box_gap2(const float3& al, const float3& ah, const float4& bl, const float4& bh) {
+    const float gx = fmaxf(fmaxf(__fsub_rd(bl.x, ah.x), __fsub_rd(al.x, bh.x)), 0.f);
+    const float gy = fmaxf(fmaxf(__fsub_rd(bl.y, ah.y), __fsub_rd(al.y, bh.y)), 0.f);
+    const float gz = fmaxf(fmaxf(__fsub_rd(bl.z, ah.z), __fsub_rd(al.z, bh.z)), 0.f);
+    return __fmaf_rd(gx, gx, __fmaf_rd(gy, gy, __fmul_rd(gz, gz)));
+}
+
 // v appended to list by the lanes that want it, one atomic per warp.  All
 // lanes of the warp call it.
 __device__ __forceinline__ void warp_append(bool want, int v, int* list, int* count) {
@@ -36,10 +45,9 @@ __device__ __forceinline__ void warp_walk(const TreeDev& T, int M, bool valid, d
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     if (!__any_sync(MHPC_FULL, valid)) return;
-    const float lx = __double2float_rd(px - rad), ly = __double2float_rd(py - rad), lz = __double2float_rd(pz - rad);
-    const float ux = __double2float_ru(px + rad), uy = __double2float_ru(py + rad), uz = __double2float_ru(pz + rad);
-    const float fx0 = __double2float_rd(px), fy0 = __double2float_rd(py), fz0 = __double2float_rd(pz);
-    const float fx1 = __double2float_ru(px), fy1 = __double2float_ru(py), fz1 = __double2float_ru(pz);
+    const float3 p0 = make_float3(__double2float_rd(px), __double2float_rd(py), __double2float_rd(pz));
+    const float3 p1 = make_float3(__double2float_ru(px), __double2float_ru(py), __double2float_ru(pz));
+    const float fr = __double2float_ru(rad);
     int top = 0;
     if (lane == 0) {
         int c = 0;
@@ -61,11 +69,9 @@ __device__ __forceinline__ void warp_walk(const TreeDev& T, int M, bool valid, d
             const int2 lk = __ldg(T.link + nd);
             const float4 bl = __ldg(T.bmin + nd), bh = __ldg(T.bmax + nd);
             const float hn = __ldg(node_hmax + nd);
-            const bool overlap =
-                !(bh.x < lx || bl.x > ux || bh.y < ly || bl.y > uy || bh.z < lz || bl.z > uz) &&
-                !(__fadd_ru(bh.x, hn) < fx0 || __fadd_rd(bl.x, -hn) > fx1 || __fadd_ru(bh.y, hn) < fy0 ||
-                  __fadd_rd(bl.y, -hn) > fy1 || __fadd_ru(bh.z, hn) < fz0 || __fadd_rd(bl.z, -hn) > fz1);
-            if (overlap) {
+            // a pair needs d < rad and d < h_j: the box must come within both
+            const float lim = fminf(fr, hn);
+            if (box_gap2(p0, p1, bl, bh) <= __fmul_ru(lim, lim)) {
                 rf = __ldg(T.first + nd);
                 if (lk.y & ND_LEAF) {
                     rlen = 1;

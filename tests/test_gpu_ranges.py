@@ -208,3 +208,38 @@ def test_pair_sums_fp32_large(cuda):
     assert np.abs(out[1][0] / out[0][0] - 1.0).max() < 2e-6
     for a, b in zip(out[0][1:], out[1][1:]):
         assert np.abs(a - b).max() <= 2e-5 * np.abs(a).max()
+
+
+# ------------------------------------------------------------ neighbour lists
+@pytest.mark.parametrize("avg_h", [0, 1])
+@pytest.mark.parametrize("scale,offset", [(1.0, 0.0), (1e-20, 0.0), (1e-14, 3e-15), (1e20, 0.0), (1.0, 1e6), (1.0, -3e3)])
+def test_neighbour_lists_scales(scale, offset, avg_h, cuda):
+    """Every list equals the brute-force set at scales where the FP32 form of the
+    pair test holds and where it does not, far from the origin, with particles
+    far outside (groups much wider than h) and distances that equal h."""
+    rng = np.random.default_rng(17)
+    C = ics.rotating_cloud(4000, seed=6)
+    n = 4096
+    pos = {k: np.concatenate([C[k], np.zeros(96)]) for k in ("x", "y", "z")}
+    g = np.arange(64)
+    pos["x"][4000:4064], pos["y"][4000:4064], pos["z"][4000:4064] = 3.0 + 0.25 * (g & 3), 0.25 * ((g >> 2) & 3), 0.25 * (g >> 4)
+    for k in ("x", "y", "z"):
+        pos[k][4064:] = rng.uniform(-1e3, 1e3, 32)
+        pos[k] = pos[k] * scale + offset
+    h = np.full(n, C["sml"][0])
+    if avg_h:
+        h = h * rng.uniform(0.6, 1.4, n)
+    h[4000:4064] = 0.25  # lattice neighbours at exactly h: no pair
+    h[4064:] = 40.0 if avg_h else h[0]
+    S = dict(pos, sml=h * scale, mass=np.full(n, 1.0 / n), e=np.ones(n), rho=np.ones(n), p=np.ones(n), cs=np.ones(n),
+             **{f: np.zeros(n) for f in ("vx", "vy", "vz")})
+    sim = Miluphpc(sph_cfg(integrate_sml=avg_h, integrate_energy=0, max_num_interactions=400), S,
+                   materials=[material(interactions=60, eos_type=0, K=1.0, gamma=1.0)], want_nnl=True)
+    sim.rhs(0)
+    off, nbr = O.frnn(S["x"], S["y"], S["z"], S["sml"])
+    noi = sim.numpy("noi")
+    assert np.array_equal(noi, np.diff(off))
+    nnl = sim.t["nnl"].cpu().numpy().reshape(n, 400)
+    for i in range(n):
+        assert np.array_equal(np.sort(nnl[i, :noi[i]]), nbr[off[i]:off[i + 1]]), i
+    sim.close()
