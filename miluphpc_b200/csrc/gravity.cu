@@ -541,12 +541,14 @@ constexpr int kListGroup = 32 * kPPL;
 constexpr int kEvalUnroll = kPPL == 2 ? 8 : 4;
 constexpr int kListSub = 8;
 constexpr int kListStack = 1024;
+constexpr int kLeafQueue = 32 * 8 + 32;  // a step's leaf children on top of fewer than 32
 constexpr int kListReserve = 7 * 22 + 8;
 
 // of one group, served by a team of W warps
 template <int W>
 struct ListSmem {
-    int stk[kListStack];
+    int stk[kListStack + 256 * (W - 1)];
+    int lq[W > 1 ? kLeafQueue * W : 1];  // leaves to fetch (teams)
     float4 cpos[64 * W];  // cell: x, y, z (group frame), m
     float4 cq0[64 * W];   // cell: Qxx Qxy Qxz Qyy
     float2 cq1[64 * W];   // cell: Qyz Qzz
@@ -751,12 +753,15 @@ constexpr int kListBlock = 128;
 // fraction of its largest (the oracle's statement uses the same floor)
 constexpr float kRelFloor = 0.1f;
 // Groups up to which a group gets a team of kListBlock / 32 warps: they test
-// kListBlock nodes a step and share the evaluation of the lists.  Walk in
-// us, Plummer (relative rule), one warp a group / teams of four:
-//   n        1,000   4,000   20,011   50,000   100,003   200,000   400,000   1,000,000
-//   1 warp      80     201      287      428       508       697      1047        1786
-//   4 warps     43      90      127      209       301       516       883        1923
-constexpr long kTeamGroups = 148 * 64;
+// kListBlock nodes a step, fetch the leaves among an opened cell's children
+// straight into the leaf list, and share the evaluation.  Walk in us, Plummer
+// (relative rule):
+//   n              1,000   20,011   50,000   100,003   400,000   2^20   2^21    2^24
+//   1 warp            80      287      428       508      1047   1786   3621   23740
+//   4 warps           43      127      209       301       883   1923   3984
+//   4, leaf queue     33      102                256       796   1768   3650   28029
+// (For one warp a queue of leaves saved a fifth of the steps and no time: 23813.)
+constexpr long kTeamGroups = 148 * 112;
 // Resident blocks per SM the list walk is compiled for: 5 (96 registers, no
 // spills in the force walk) measured 3 % faster at 16.7 M than the
 // unconstrained 116 registers (4 blocks); 6 blocks (80 registers) spill and
@@ -876,10 +881,11 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
     team_sync<W>();  // (also the sub-boxes, which every warp writes alike)
     int top = S.top;
     double ax[kPPL] = {}, ay[kPPL] = {}, az[kPPL] = {}, ph[kPPL] = {};
-    int ncell = 0, nleaf = 0;
+    int ncell = 0, nleaf = 0, nlq = 0;
+    constexpr int kStack = kListStack + 256 * (W - 1);
     unsigned long long tested = 0, ncell_tot = 0, nleaf_tot = 0;
     while (top > 0) {
-        int room = (kListStack - kListReserve - top) / 7;
+        int room = (kStack - kListReserve - top) / 7;
         int k = top < 32 * W ? top : 32 * W;
         if (k > room) k = room > 1 ? room : 1;
         const bool act = tt < k;
@@ -949,7 +955,11 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
         const int mask = open ? (__float_as_int(w3.z) >> 9) : 0;
         const bool bucket = open && (mask & 0x100);
         const unsigned bb = __ballot_sync(MHPC_FULL, bucket);
-        const int nkid = (open && !bucket) ? __popc(mask & 0xff) : 0;
+        // an opened cell's children go to the stack; for a team its leaves, which
+        // need no test, to the queue.  One scan for both counts (leaves in the
+        // high half).
+        const int leaves = (W > 1 && open && !bucket) ? (mask >> 9) & 0xff : 0;
+        const int nkid = (open && !bucket) ? __popc(mask & 0xff & ~leaves) + (__popc(leaves) << 16) : 0;
         int incl = nkid;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -958,7 +968,7 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
         }
         // places in the lists and on the stack: this warp's, after the warps before it
         int nl = __popc(bl), nc = __popc(bc), ndefer = __popc(bb), total = 0;
-        int lbase = nleaf, cbase = ncell, kbase = top, dbase = 0;
+        int lbase = nleaf, cbase = ncell, kbase = top, qbase = nlq, dbase = 0;
         if (W == 1) {
             total = __shfl_sync(MHPC_FULL, incl, 31);
         } else {
@@ -967,7 +977,7 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
             nl = nc = ndefer = 0;
 #pragma unroll
             for (int q = 0; q < W; ++q) {
-                if (q == w) { lbase += nl; cbase += nc; kbase += total; dbase = ndefer; }
+                if (q == w) { lbase += nl; cbase += nc; kbase += total & 0xffff; qbase += total >> 16; dbase = ndefer; }
                 nl += S.cnt[q][0]; nc += S.cnt[q][1]; total += S.cnt[q][2]; ndefer += S.cnt[q][3];
             }
         }
@@ -981,7 +991,8 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
         }
         ncell += nc;
         if (bucket) S.defer[dbase + __popc(bb & lt)] = nd;
-        if (top + total > kListStack) {
+        const int pushed = W > 1 ? total & 0xffff : total;
+        if (top + pushed > kStack) {
             // unreachable by the bound on k; stop instead of overrunning
             if (tt == 0) set_status(st, MHPC_ERR_DEPTH, 2);
             return;
@@ -990,12 +1001,25 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
             const int4 k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
             const int4 k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
             const int all[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-            int pos = kbase + incl - nkid;
+            int pos = kbase + (W == 1 ? incl - nkid : (incl - nkid) & 0xffff);
+            if (W == 1) {
 #pragma unroll
-            for (int d = 0; d < 8; ++d)
-                if ((mask >> d) & 1) S.stk[pos++] = all[d];
+                for (int d = 0; d < 8; ++d)
+                    if ((mask >> d) & 1) S.stk[pos++] = all[d];
+            } else {
+                qbase += (incl - nkid) >> 16;
+#pragma unroll
+                for (int d = 0; d < 8; ++d) {
+                    if ((leaves >> d) & 1) S.lq[qbase++] = all[d];
+                    else if ((mask >> d) & 1) S.stk[pos++] = all[d];
+                }
+            }
         }
-        top += total;
+        top += pushed;
+        if (W > 1) {
+            nlq += total >> 16;
+            tested += total >> 16;
+        }
         team_sync<W>();
         if (ncell >= 32 * W) {
             eval_cells_sel<W, kGuard, kPot>(S, w, ncell, rx, ry, rz, e2, ax, ay, az, ph);
@@ -1008,6 +1032,26 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
             nleaf_tot += nleaf;
             nleaf = 0;
             team_sync<W>();
+        }
+        // queued leaves, 32 W at a time (all that are left once the stack is
+        // empty): their positions go to the leaf list
+        while (W > 1 && (nlq >= 32 * W || (top == 0 && nlq > 0))) {
+            const int got = min(nlq, 32 * W);
+            nlq -= got;
+            if (tt < got) {
+                const float4* wl = T.wrec + 4 * (size_t)S.lq[nlq + tt];
+                const float4 hp = __ldg(wl), lp = __ldg(wl + 1);
+                S.lpos[nleaf + tt] = make_float4((hp.x - chx) + (lp.x - clx), (hp.y - chy) + (lp.y - cly),
+                                                 (hp.z - chz) + (lp.z - clz), hp.w);
+            }
+            nleaf += got;
+            team_sync<W>();
+            if (nleaf >= 32 * W) {
+                eval_leaves_sel<W, kGuard, kPot>(S, w, nleaf, rx, ry, rz, e2, ax, ay, az, ph);
+                nleaf_tot += nleaf;
+                nleaf = 0;
+                team_sync<W>();
+            }
         }
         // shared-key buckets: their children are consecutive leaves (the leaf
         // list holds fewer than 32 W entries here, at most 64 W - 1 after a round)

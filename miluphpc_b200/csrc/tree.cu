@@ -233,7 +233,8 @@ __device__ __forceinline__ Kids cell_kids(const TreeDev& T, int p) {
 // of the centre of mass, the geometric opening criterion edge^2/theta (-1 for
 // leaves), the quadrupole, the link info with the child mask, and M l^3.
 __device__ __forceinline__ void put_wrec(const TreeDev& T, int i, double x, double y, double z, double m, int info,
-                                         int mask, float4 q0, float2 q1, double edge0, double inv_theta) {
+                                         int mask, int leaves, float4 q0, float2 q1, double edge0,
+                                         double inv_theta) {
     const float hx = (float)x, hy = (float)y, hz = (float)z;
     float crit = -1.f, ml3 = 0.f;
     if (!(info & ND_LEAF)) {
@@ -245,7 +246,7 @@ __device__ __forceinline__ void put_wrec(const TreeDev& T, int i, double x, doub
     w[0] = make_float4(hx, hy, hz, (float)m);
     w[1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz), crit);
     w[2] = q0;
-    w[3] = make_float4(q1.x, q1.y, __int_as_float((info & 0x1ff) | (mask << 9)), ml3);
+    w[3] = make_float4(q1.x, q1.y, __int_as_float((info & 0x1ff) | (mask << 9) | (leaves << 18)), ml3);
 }
 
 // Loads of values that the running upward pass itself writes, never through
@@ -276,7 +277,7 @@ __device__ __forceinline__ void leaf_moments(const TreeDev& T, int a, int leaf, 
         T.bmax[leaf] = make_float4(ru(px), ru(py), ru(pz), 0.f);
     }
     if (want_quad)
-        put_wrec(T, leaf, px, py, pz, pm, __ldg(&T.link[leaf].y), 0, make_float4(0.f, 0.f, 0.f, 0.f),
+        put_wrec(T, leaf, px, py, pz, pm, __ldg(&T.link[leaf].y), 0, 0, make_float4(0.f, 0.f, 0.f, 0.f),
                  make_float2(0.f, 0.f), edge0, inv_theta);
 }
 
@@ -287,7 +288,9 @@ __device__ __forceinline__ void leaf_moments(const TreeDev& T, int a, int leaf, 
 // a load behind each slot's test waits for the one before it.  With `local`
 // the first pass over the children also brings their quadrupoles into L1 for
 // the second.
-template <int kB>
+// kLeafMask: the record also tells which slots hold leaves, for the list walk's
+// teams; a walk that finds no such slot takes leaves as nodes.
+template <int kB, bool kLeafMask>
 __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids& K, int want_quad, int want_box,
                                              double edge0, double inv_theta, bool local) {
     double m = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
@@ -352,6 +355,7 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
     }
     if (want_quad) {
         double q[6] = {0, 0, 0, 0, 0, 0};
+        int leaves = 0;  // slots that hold leaves
         // a0, a1: the child's quadrupole from its walk record (one 32-byte sector)
         auto add_quad = [&](const double4& cc, const float4& a0, const float4& a1) {
             const double s0 = cc.x - mx, s1 = cc.y - my, s2 = cc.z - mz;
@@ -388,12 +392,15 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
                 }
 #pragma unroll
                 for (int d = 0; d < kQ; ++d)
-                    if ((part >> d) & 1) add_quad(cc[d], a0[d], a1[d]);
+                    if ((part >> d) & 1) {
+                        add_quad(cc[d], a0[d], a1[d]);
+                        if (kLeafMask && (__float_as_int(a1[d].z) & ND_LEAF)) leaves |= 1 << (d0 + d);
+                    }
             }
         }
         const float4 q0 = make_float4((float)q[0], (float)q[1], (float)q[2], (float)q[3]);
         const float2 q1 = make_float2((float)q[4], (float)q[5]);
-        put_wrec(T, p, mx, my, mz, m, lkp.y, K.mask, q0, q1, edge0, inv_theta);
+        put_wrec(T, p, mx, my, mz, m, lkp.y, K.mask, leaves, q0, q1, edge0, inv_theta);
     }
 }
 
@@ -433,6 +440,8 @@ constexpr int kUpHand = 1024;
 //   2            68       79        90       141         313
 //   4            55       93        97       120         262
 //   8                                        136         283         682   2504
+// (8 positions, above 2,000,000 particles, leave out the mask of leaf slots: no
+// walk of that size asks for it, and it cost 100 us at 2^24.)
 inline int up_per(int n) {
     if (n <= 8192) return 4;
     if (n <= 65536) return 1;
@@ -610,7 +619,7 @@ __global__ void __launch_bounds__(kUpBlock, 3) k_upward(TreeDev T, const double*
     upward_chunk<kUpPer>(
         T, [&](int a, int leaf) { leaf_moments(T, a, leaf, sx, sy, sz, sm, want_quad, want_box, edge0, inv_theta); },
         [&](int p, bool local) {
-            cell_moments<4>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta, local);
+            cell_moments<4, (kUpPer < 8)>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta, local);
         });
 }
 

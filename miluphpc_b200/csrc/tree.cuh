@@ -36,7 +36,8 @@ struct TreeDev {
     //   [0] float(x), float(y), float(z), m   (FP32 hi part of the centre of mass)
     //   [1] x - float(x), ..., opening criterion edge^2/theta (-1 for leaves)
     //   [2] Qxx Qxy Qxz Qyy  (traceless quadrupole about the centre of mass; 0 for leaves)
-    //   [3] Qyz Qzz, bits (link info & 0x1ff) | kmask << 9, M l^3 (cells; l = edge)
+    //   [3] Qyz Qzz, bits (link info & 0x1ff) | kmask << 9 | slots holding leaves << 18,
+    //       M l^3 (cells; l = edge)
     float4* wrec;
     float* hmax;        // [cap] largest smoothing length below the node (rounded up)
     int* arrive;        // [cap] completed children counted for cells that cross a block's
