@@ -19,7 +19,13 @@ namespace {
 
 constexpr int kBlock = 128;
 constexpr int kWarps = kBlock / 32;
-constexpr int kSmall = 16;    // cells with at most this many particles are staged whole
+// cells with at most this many particles are staged whole (8: 4 % slower, 4: 20 %)
+constexpr int kSmall = 16;
+// Gap between consecutive particles, in h, at which a group is cut.  Variable h
+// of a 2^20 cloud in us, uncut / 2 / 1.5 / 1 / 0.7: 3870 / 3600 / 3440 / 3390 /
+// 3400; list walk of a 35,937 lattice 95 / 95 / 107 / 115 / 212, of larger lattices
+// the same from 1 on.
+constexpr double kCut = 1.5;
 
 // ------------------------------------------------------------ FRNN walk
 // One warp per 32 consecutive (sorted or listed) particles, lane = particle,
@@ -59,7 +65,7 @@ constexpr int kSmall = 16;    // cells with at most this many particles are stag
 // neighbour set equals the brute-force set.
 // Bound: issue and fixed latency (58 % of the issue slots, 18 resident warps per
 // SM).  List walk in us with FP64 tests and grown boxes / now: Sedov lattice of
-// 262,144 particles 258 / 236, of 2,097,152 1693 / 1510; all walks of a cloud step,
+// 262,144 particles 258 / 224, of 2,097,152 1693 / 1432; all walks of a cloud step,
 // 2^20 particles 2229 / 1843, 2^23 16600 / 13850.
 //
 // mode 0: write lists (h_i = h[i], h_j = h[j]) for all particles; mode 1:
@@ -83,12 +89,12 @@ struct FrnnSmem {
 };
 
 #ifndef MHPC_FRNN_MIN_BLOCKS
-#define MHPC_FRNN_MIN_BLOCKS 6
+#define MHPC_FRNN_MIN_BLOCKS 7
 #endif
 template <int MODE>
-// 6 blocks per SM (the register cap costs a few spilled values, the extra
-// warps hide more of the walk's latency)
-__global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T, int n, int maxnb, const double* __restrict__ sx,
+// 7 blocks per SM: the list walk of 2,097,152 particles in us with 5 / 6 / 7: 1632 /
+// 1496 / 1432 (the extra warps hide more of the walk's latency)
+__global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T, int n, int ppw, int maxnb, const double* __restrict__ sx,
                                                  const double* __restrict__ sy, const double* __restrict__ sz,
                                                  const double* __restrict__ sh, const int* __restrict__ list,
                                                  const int* __restrict__ list_count,
@@ -105,14 +111,35 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
     const long total = MODE == 1 ? (long)*list_count : (long)n;
     // one group per warp (a gated re-walk that mostly returns at once has a
     // smaller grid and takes several)
-    for (long g = ((long)blockIdx.x * kBlock + threadIdx.x) >> 5; g * 32 < total; g += (long)gridDim.x * kWarps) {
-    long s = g * 32 + lane;
-    const bool valid = s < total;
+    for (long g = ((long)blockIdx.x * kBlock + threadIdx.x) >> 5; g * ppw < total; g += (long)gridDim.x * kWarps) {
+    long s = g * ppw + lane;
+    const bool valid = lane < ppw && s < total;
     if (MODE == 1) s = valid ? list[s] : 0;
-    const bool active = valid;
+    int k = 0;     // neighbours found for this lane's particle
+    // The curve jumps between cells of the tree: a group across such a place would
+    // walk the whole box between its two ends.  It is cut where two consecutive
+    // particles are far apart, and its parts walk one after the other.
+    unsigned rest = __ballot_sync(MHPC_FULL, valid);
+    unsigned cuts;
+    {
+        double px = 0, py = 0, pz = 0, hm = 0;
+        if (valid) { px = sx[s]; py = sy[s]; pz = sz[s]; hm = sh[s]; }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) hm = fmax(hm, __shfl_xor_sync(MHPC_FULL, hm, o));
+        const double nx = __shfl_down_sync(MHPC_FULL, px, 1), ny = __shfl_down_sync(MHPC_FULL, py, 1);
+        const double nz = __shfl_down_sync(MHPC_FULL, pz, 1);
+        const bool next = lane < 31 && ((rest >> (lane + 1)) & 1u);
+        const double gap = fmax(fmax(fabs(nx - px), fabs(ny - py)), fabs(nz - pz));
+        cuts = __ballot_sync(MHPC_FULL, next && gap > kCut * hm);
+    }
+    while (rest) {
+    const unsigned after = cuts & ~((1u << (__ffs(rest) - 1)) - 1u);
+    const unsigned part = after ? rest & (2u * (after & (0u - after)) - 1u) : rest;
+    rest &= ~part;
+    cuts &= ~part;
+    const bool active = (part >> lane) & 1u;
     double px = 0, py = 0, pz = 0, hi = 0;
-    if (valid) { px = sx[s]; py = sy[s]; pz = sz[s]; hi = sh[s]; }
-    const double hi2 = hi * hi;
+    if (active) { px = sx[s]; py = sy[s]; pz = sz[s]; hi = sh[s]; }
     // points box and largest h over the sub-group (8 lanes), then over the warp
     double hm = active ? hi : 0.0, shm = 0.0;
     double sl[3] = {}, su[3] = {};  // the sub-group's box
@@ -135,7 +162,7 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
     const float3 g0 = make_float3(__double2float_rd(plx), __double2float_rd(ply), __double2float_rd(plz));
     const float3 g1 = make_float3(__double2float_ru(pux), __double2float_ru(puy), __double2float_ru(puz));
     const double cx = 0.5 * (plx + pux), cy = 0.5 * (ply + puy), cz = 0.5 * (plz + puz);
-    const float fx = (float)(px - cx), fy = (float)(py - cy), fz = (float)(pz - cz), fh2 = (float)hi2;
+    const float fx = (float)(px - cx), fy = (float)(py - cy), fz = (float)(pz - cz), fh2 = (float)(hi * hi);
     const float H = __double2float_ru(hm);
     const float R = 1.00001f * ((float)fmax(fmax(pux - cx, puy - cy), puz - cz) + H);
     // |d^2(FP32) - min(h_i^2, h_j^2)| up to which the exact test decides, and what
@@ -153,7 +180,6 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
         S.slo[q] = make_float4(ax, ay, az, any ? 1.000001f * __double2float_ru(shm) + slack : -1.f);
         S.shi[q] = make_float4(bx, by, bz, 0.f);
     }
-    int k = 0;     // neighbours found for this lane's particle
     int pool = 0;  // pool entries (warp-uniform)
     int cnt0 = 0, cnt1 = 0, cnt2 = 0, cnt3 = 0;  // list entries per sub-group (warp-uniform)
     auto flush = [&]() {
@@ -169,30 +195,39 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
             const bool iact = __shfl_sync(MHPC_FULL, (int)active, src) != 0;
             int kb = __shfl_sync(MHPC_FULL, k, src);
             const unsigned pmask = 0x01010101u << p;
-            for (int c0 = 0; c0 < cntg; c0 += 4) {
-                const int c = c0 + q;
-                bool hit = false;
-                int j = 0;
-                if (iact && c < cntg) {
-                    const int slot = S.lst[sg][c];
-                    j = S.cj[slot];
-                    const float4 q4 = S.cp[slot];
-                    const float dx = ix - q4.x, dy = iy - q4.y, dz = iz - q4.z;
-                    const float over = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - fminf(ih2, q4.w);
-                    hit = over < -band;
-                    if (!hit && !(over > band)) {
-                        const double hs = sh[is], hj = sh[j];
-                        const double d = d2_exact(sx[is] - sx[j], sy[is] - sy[j], sz[is] - sz[j]);
-                        hit = d < hs * hs && d < hj * hj;
+            // two entries per lane and step: their loads and sums overlap
+            for (int c0 = 0; c0 < cntg; c0 += 8) {
+                bool hit[2];
+                int j[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int c = c0 + 4 * u + q;
+                    hit[u] = false;
+                    j[u] = 0;
+                    if (iact && c < cntg) {
+                        const int slot = S.lst[sg][c];
+                        j[u] = S.cj[slot];
+                        const float4 q4 = S.cp[slot];
+                        const float dx = ix - q4.x, dy = iy - q4.y, dz = iz - q4.z;
+                        const float over = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - fminf(ih2, q4.w);
+                        hit[u] = over < -band;
+                        if (!hit[u] && !(over > band)) {
+                            const double hs = sh[is], hj = sh[j[u]];
+                            const double d = d2_exact(sx[is] - sx[j[u]], sy[is] - sy[j[u]], sz[is] - sz[j[u]]);
+                            hit[u] = d < hs * hs && d < hj * hj;
+                        }
+                        hit[u] = hit[u] && j[u] != is;
                     }
-                    hit = hit && j != is;
                 }
-                const unsigned b = __ballot_sync(MHPC_FULL, hit) & pmask;
-                if (MODE != 1 && hit) {
-                    const int pos = kb + __popc(b & lt);
-                    if (pos < maxnb) nbr[nb_index(is, pos, maxnb)] = j;
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const unsigned b = __ballot_sync(MHPC_FULL, hit[u]) & pmask;
+                    if (MODE != 1 && hit[u]) {
+                        const int pos = kb + __popc(b & lt);
+                        if (pos < maxnb) nbr[nb_index(is, pos, maxnb)] = j[u];
+                    }
+                    kb += __popc(b);
                 }
-                kb += __popc(b);
             }
             // lane p (q = 0) holds particle 8 sg + p's count: its owner takes it
             const int knew = __shfl_sync(MHPC_FULL, kb, p);
@@ -326,14 +361,15 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
         __syncwarp();
     }
     flush();
-    if (active) {
+    }
+    if (valid) {
         noi[s] = k;
         if (MODE == 0 && k > maxnb) set_status(st, MHPC_ERR_NEIGHBOURS, (int)s);
         if (MODE == 2 && k > maxnb) *trunc = 1;
         if (MODE == 0) atomicMax(&st->max_noi, k);
     }
     if (MODE == 0) {
-        unsigned long long tot = active ? (unsigned long long)k : 0ULL;
+        unsigned long long tot = valid ? (unsigned long long)k : 0ULL;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(MHPC_FULL, tot, o);
         if (lane == 0) atomicAdd(&st->noi_sum, tot);
@@ -529,17 +565,29 @@ __global__ void k_export_nnl(int n, int maxnb, const int* __restrict__ nbr, cons
 
 }  // namespace
 
+namespace {
+// Particles per warp of the neighbour walk.  With 32 a small n has one warp per
+// scheduler or fewer, and a walk is a chain of round trips and list tests; with
+// one sub-group of 8 there are four times the warps, with less to test each.
+// List walk in us with 8 / 16 / 32: Sedov lattice of 8,000 particles 56 / 74 / 109,
+// 35,937 127 / 115 / 156, 110,592 213 / 168 / 138; variable h of a cloud of 20,011
+// 493 / 527 / 556, 50,000 628 / 626 / 695, 100,000 841 / 798 / 773.
+int frnn_group(int n) { return n <= 25000 ? 8 : n <= 65000 ? 16 : 32; }
+long frnn_blocks(int n, int ppw) { return (((long)n + ppw - 1) / ppw + kWarps - 1) / kWarps; }
+}  // namespace
+
 int sph_frnn(const TreeDev& T, const SphParams& P, const SphSorted& S, int* nbr, int* noi, DevStatus* st,
              cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
-    long blocks = (((long)P.n + 31) / 32 * 32 + kBlock - 1) / kBlock;
+    const int ppw = frnn_group(P.n);
+    const long blocks = frnn_blocks(P.n, ppw);
     const float* hmax = nullptr;
     if (P.avg_h) {  // smoothing lengths differ: prune nodes by their largest h
         int rc = tree_node_hmax(T, S.h, st, s);
         if (rc) return rc;
         hmax = T.hmax;
     }
-    k_frnn<0><<<(int)blocks, kBlock, 0, s>>>(T, P.n, P.maxnb, S.x, S.y, S.z, S.h, nullptr, nullptr, hmax, nbr, noi,
+    k_frnn<0><<<(int)blocks, kBlock, 0, s>>>(T, P.n, ppw, P.maxnb, S.x, S.y, S.z, S.h, nullptr, nullptr, hmax, nbr, noi,
                                               st);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;
@@ -549,7 +597,8 @@ int sph_variable_h(const TreeDev& T, const SphParams& P, const double* x, const 
                    double* h, const VhBuffers& B, int target, int tol, int max_iter, int sweeps, DevStatus* st,
                    cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
-    const long blocks = (((long)P.n + 31) / 32 * 32 + kBlock - 1) / kBlock;
+    const int ppw = frnn_group(P.n);
+    const long blocks = frnn_blocks(P.n, ppw);
     const int g = grid_for(P.n, 256, 148 * 16);
     const int* list_count = B.off + P.n;
     // Jacobi snapshot of h and the largest-h bounds; k_vh_update keeps both
@@ -567,7 +616,7 @@ int sph_variable_h(const TreeDev& T, const SphParams& P, const double* x, const 
         k_compact<<<g, 256, 0, s>>>(P.n, B.flags, B.off, B.list);
         if (it == 0) {
             // first sweep: (nearly) every particle, group walks
-            k_frnn<1><<<(int)blocks, kBlock, 0, s>>>(T, P.n, P.maxnb, x, y, z, B.hold, B.list, list_count, T.hmax,
+            k_frnn<1><<<(int)blocks, kBlock, 0, s>>>(T, P.n, ppw, P.maxnb, x, y, z, B.hold, B.list, list_count, T.hmax,
                                                       nullptr, B.count, st);
         } else {
             // later sweeps: the few particles still iterating, a warp each
@@ -588,7 +637,8 @@ int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, 
                          double* h, int* nbr, int* noi, const VhBuffers& V, const BandBuffers& B, int target,
                          int tol, int max_iter, int sweeps, DevStatus* st, cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
-    const long blocks = (((long)P.n + 31) / 32 * 32 + kBlock - 1) / kBlock;
+    const int ppw = frnn_group(P.n);
+    const long blocks = frnn_blocks(P.n, ppw);
     const int g = grid_for(P.n, 256, 148 * 16);
     int* trunc = B.ctr + 2;   // some list holds fewer entries than its count
     int* rewalk = B.ctr + 3;  // the lists are re-walked after this sweep
@@ -597,7 +647,7 @@ int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, 
     int rc = tree_node_hmax(T, h, st, s);
     if (rc) return rc;
     // the lists and counts of the starting h: the counts of the first sweep
-    k_frnn<2><<<(int)blocks, kBlock, 0, s>>>(T, P.n, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi, st,
+    k_frnn<2><<<(int)blocks, kBlock, 0, s>>>(T, P.n, ppw, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi, st,
                                               rewalk, trunc);
     // gated re-walks: several groups per warp, so that the launch that finds
     // nothing to do has few blocks to retire
@@ -615,7 +665,7 @@ int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, 
         rc = sph_apply_h_changes(T, P, x, y, z, h, hnew, nbr, noi, cur, cur_count, B, trunc, st, s);
         if (rc) return rc;
         k_vh_commit<<<g, 256, 0, s>>>(cur, cur_count, hnew, h, V.done, next, next_count, B.ctr);
-        k_frnn<2><<<(int)gated, kBlock, 0, s>>>(T, P.n, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi, st,
+        k_frnn<2><<<(int)gated, kBlock, 0, s>>>(T, P.n, ppw, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi, st,
                                                  rewalk, trunc);
     }
     rc = sph_sort_appended(P, nbr, noi, B.appended, s);
