@@ -24,6 +24,9 @@ namespace {
 constexpr int kBandBlock = 128;  // 4 warps, one particle per warp
 constexpr int kBandWarps = kBandBlock / 32;
 constexpr int kBandCap = 256;    // candidates held per particle during the selection
+// resident blocks per SM (and the grids): a warp waits on one tree walk at a time,
+// so as many walks as registers and shared memory allow
+constexpr int kEventBlocks = 10, kSelectBlocks = 8;
 // The band's two repair targets and the search radius of a particle with
 // count n and smoothing length h (the same arithmetic as the oracle's).
 struct BandRule {
@@ -94,7 +97,7 @@ __global__ void __launch_bounds__(256) k_band_list(int n, const int* __restrict_
 // h of the first round) cannot gain a pair: it keeps h without a walk.  A
 // new h above the old one raises the largest-h bounds of the particle's leaf
 // and ancestors (grow-only).
-__global__ void __launch_bounds__(kBandBlock) k_band_select(TreeDev T, const double* __restrict__ sx,
+__global__ void __launch_bounds__(kBandBlock, kSelectBlocks) k_band_select(TreeDev T, const double* __restrict__ sx,
                                                             const double* __restrict__ sy,
                                                             const double* __restrict__ sz,
                                                             const double* __restrict__ h,
@@ -228,7 +231,7 @@ struct EventVisit {
     }
 };
 
-__global__ void __launch_bounds__(kBandBlock) k_band_events(TreeDev T, const double* __restrict__ sx,
+__global__ void __launch_bounds__(kBandBlock, kEventBlocks) k_band_events(TreeDev T, const double* __restrict__ sx,
                                                             const double* __restrict__ sy,
                                                             const double* __restrict__ sz,
                                                             const double* __restrict__ h,
@@ -359,9 +362,34 @@ __global__ void k_band_add(const int2* __restrict__ ev, int* ctr, int cap, int* 
     }
 }
 
-// Every list marked in `appended` sorted by neighbour index (one warp per
-// list: ranks by counting, the entries are distinct), and the mark cleared.
-constexpr int kSortPerLane = 8;  // lists up to 256 entries in registers; longer ones by lane 0
+// The list of a (k entries, distinct, at most 32 R) sorted by neighbour index:
+// R entries per lane, ranks by counting over the warp.
+template <int R>
+__device__ __forceinline__ void sort_list(int* nbr, int maxnb, long a, int k, int lane) {
+    int val[R], rank[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int q = lane + 32 * r;
+        val[r] = q < k ? nbr[nb_index(a, q, maxnb)] : 0;
+        rank[r] = 0;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int m = min(32, k - 32 * r);
+        for (int l = 0; l < m; ++l) {
+            const int v = __shfl_sync(MHPC_FULL, val[r], l);
+#pragma unroll
+            for (int t = 0; t < R; ++t) rank[t] += v < val[t];
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (lane + 32 * r < k) nbr[nb_index(a, rank[r], maxnb)] = val[r];
+}
+
+// Every list marked in `appended` sorted (one warp per list), and the mark
+// cleared.
 __global__ void k_sort_appended(int n, int* appended, int* nbr, const int* __restrict__ noi, int maxnb) {
     const int lane = threadIdx.x & 31;
     const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -376,23 +404,10 @@ __global__ void k_sort_appended(int n, int* appended, int* nbr, const int* __res
             todo &= todo - 1;
             const long a = base + b;
             const int k = min(noi[a], maxnb);
-            if (k <= 32 * kSortPerLane) {
-                int val[kSortPerLane], rank[kSortPerLane];
-#pragma unroll
-                for (int r = 0; r < kSortPerLane; ++r) {
-                    const int q = lane + 32 * r;
-                    val[r] = q < k ? nbr[nb_index(a, q, maxnb)] : 0;
-                    rank[r] = 0;
-                }
-                for (int q = 0; q < k; ++q) {
-                    const int v = nbr[nb_index(a, q, maxnb)];
-#pragma unroll
-                    for (int r = 0; r < kSortPerLane; ++r) rank[r] += v < val[r];
-                }
-                __syncwarp();
-#pragma unroll
-                for (int r = 0; r < kSortPerLane; ++r)
-                    if (lane + 32 * r < k) nbr[nb_index(a, rank[r], maxnb)] = val[r];
+            if (k <= 64) {
+                sort_list<2>(nbr, maxnb, a, k, lane);
+            } else if (k <= 256) {
+                sort_list<8>(nbr, maxnb, a, k, lane);
             } else if (lane == 0) {
                 for (int q = 1; q < k; ++q) {  // insertion sort in place
                     const int v = nbr[nb_index(a, q, maxnb)];
@@ -441,7 +456,7 @@ int sph_apply_h_changes(const TreeDev& T, const SphParams& P, const double* x, c
                         const double* h, const double* hnew, int* nbr, int* noi, const int* list,
                         const int* list_count, const BandBuffers& B, int* trunc, DevStatus* st, cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
-    k_band_events<<<148 * 8, kBandBlock, 0, s>>>(T, x, y, z, h, hnew, noi, nbr, P.maxnb, list, list_count, T.hmax,
+    k_band_events<<<148 * kEventBlocks, kBandBlock, 0, s>>>(T, x, y, z, h, hnew, noi, nbr, P.maxnb, list, list_count, T.hmax,
                                                  B.events, B.cap_events, B.ctr, st, trunc);
     k_band_mark<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, B.dirty, B.dlist, trunc);
     k_band_filter<<<148 * 8, 128, 0, s>>>(B.dlist, B.ctr, x, y, z, hnew, nbr, noi, P.maxnb, B.dirty, trunc);
@@ -461,9 +476,9 @@ int sph_band_fixup(const TreeDev& T, const SphParams& P, const double* x, const 
     for (int r = 0; r < rounds; ++r) {
         int* list_count = B.ctr + kBandCount + (r & 1);
         k_band_list<<<g, 256, 0, s>>>(n, noi, R, B.list, list_count, B.ctr);
-        k_band_select<<<148 * 8, kBandBlock, 0, s>>>(T, x, y, z, h, B.h0, noi, nbr, P.maxnb, B.list, list_count, R,
+        k_band_select<<<148 * kSelectBlocks, kBandBlock, 0, s>>>(T, x, y, z, h, B.h0, noi, nbr, P.maxnb, B.list, list_count, R,
                                                      P.ord, B.hnew, T.hmax, st);
-        k_band_events<<<148 * 8, kBandBlock, 0, s>>>(T, x, y, z, h, B.hnew, noi, nbr, P.maxnb, B.list, list_count,
+        k_band_events<<<148 * kEventBlocks, kBandBlock, 0, s>>>(T, x, y, z, h, B.hnew, noi, nbr, P.maxnb, B.list, list_count,
                                                      T.hmax, B.events, B.cap_events, B.ctr, st);
         k_band_mark<<<148 * 4, 256, 0, s>>>(B.events, B.ctr, B.cap_events, B.dirty, B.dlist);
         k_band_filter<<<148 * 8, 128, 0, s>>>(B.dlist, B.ctr, x, y, z, B.hnew, nbr, noi, P.maxnb, B.dirty);

@@ -357,7 +357,7 @@ int stage_frnn(mhpc_ctx* c, const mhpc_particles* p, bool variable_h, bool learn
             E.ctr = c->band_ctr; E.dlist = c->vh_flags; E.appended = c->nb_appended;
             TRY(sph_variable_h_lists(c->T, P, c->sx, c->sy, c->sz, c->sh, c->nbr, c->noi, B, E, target,
                                      c->cfg.nb_tolerance, c->cfg.max_sml_iterations,
-                                     c->cfg.max_sml_iterations + 2, c->st, s));
+                                     c->cfg.max_sml_iterations + 2, c->cfg.sml_band_rounds <= 0, c->st, s));
         } else {
             TRY(sph_variable_h(c->T, P, c->sx, c->sy, c->sz, c->sh, B, target, c->cfg.nb_tolerance,
                                c->cfg.max_sml_iterations, c->cfg.max_sml_iterations + 2, c->st, s));

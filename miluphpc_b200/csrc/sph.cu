@@ -635,7 +635,7 @@ int sph_variable_h(const TreeDev& T, const SphParams& P, const double* x, const 
 
 int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, const double* y, const double* z,
                          double* h, int* nbr, int* noi, const VhBuffers& V, const BandBuffers& B, int target,
-                         int tol, int max_iter, int sweeps, DevStatus* st, cudaStream_t s) {
+                         int tol, int max_iter, int sweeps, bool sort_lists, DevStatus* st, cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
     const int ppw = frnn_group(P.n);
     const long blocks = frnn_blocks(P.n, ppw);
@@ -668,8 +668,10 @@ int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, 
         k_frnn<2><<<(int)gated, kBlock, 0, s>>>(T, P.n, ppw, P.maxnb, x, y, z, h, nullptr, nullptr, T.hmax, nbr, noi, st,
                                                  rewalk, trunc);
     }
-    rc = sph_sort_appended(P, nbr, noi, B.appended, s);
-    if (rc) return rc;
+    if (sort_lists) {
+        rc = sph_sort_appended(P, nbr, noi, B.appended, s);
+        if (rc) return rc;
+    }
     k_noi_stats<<<grid_for(P.n, 256, 148 * 4), 256, 0, s>>>(P.n, P.maxnb, noi, V.cnt + (sweeps & 1), st);
     CUDA_TRY(cudaGetLastError());
     return MHPC_OK;

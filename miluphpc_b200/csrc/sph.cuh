@@ -145,7 +145,8 @@ int sph_apply_h_changes(const TreeDev& T, const SphParams& P, const double* x, c
 // right-hand side is not needed).  Lists that pass maxnb during the
 // iteration, or an event-buffer overflow, fall back to a full list walk after
 // that sweep.  Uses B.hnew and B.ctr[0..3]; T.hmax stays an upper bound
-// (grow-only) of the current h.
+// (grow-only) of the current h.  Without sort_lists the lists with appends stay
+// marked and unsorted (sph_band_fixup, run next, sorts them with its own).
 int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, const double* y, const double* z,
                          double* h, int* nbr, int* noi, const VhBuffers& V, const BandBuffers& B, int target,
-                         int tol, int max_iter, int sweeps, DevStatus* st, cudaStream_t s);
+                         int tol, int max_iter, int sweeps, bool sort_lists, DevStatus* st, cudaStream_t s);

@@ -65,19 +65,23 @@ __device__ __forceinline__ void warp_walk(const TreeDev& T, int M, bool valid, d
         __syncwarp();
         top -= kk;
         int rf = 0, rlen = 0, kmask = 0;
+        int4 k0 = make_int4(0, 0, 0, 0), k1 = k0;
         if (act) {
+            // the child slots come with the box: a walk of one particle waits for
+            // each round trip
+            k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
+            k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
             const int2 lk = __ldg(T.link + nd);
             const float4 bl = __ldg(T.bmin + nd), bh = __ldg(T.bmax + nd);
             const float hn = __ldg(node_hmax + nd);
+            const int fs = __ldg(T.first + nd), l = __ldg(T.last + nd), km = __ldg(T.kmask + nd);
             // a pair needs d < rad and d < h_j: the box must come within both
             const float lim = fminf(fr, hn);
             if (box_gap2(p0, p1, bl, bh) <= __fmul_ru(lim, lim)) {
-                rf = __ldg(T.first + nd);
+                rf = fs;
                 if (lk.y & ND_LEAF) {
                     rlen = 1;
                 } else {
-                    const int l = __ldg(T.last + nd);
-                    const int km = __ldg(T.kmask + nd);
                     if (l - rf + 1 <= kWalkSmall || (km & 0x100)) rlen = l - rf + 1;
                     else kmask = km & 0xff;
                 }
@@ -96,8 +100,6 @@ __device__ __forceinline__ void warp_walk(const TreeDev& T, int M, bool valid, d
             return;
         }
         if (nkid) {
-            const int4 k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
-            const int4 k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
             const int all[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
             int wpos = top + incl - nkid;
 #pragma unroll

@@ -243,3 +243,48 @@ def test_neighbour_lists_scales(scale, offset, avg_h, cuda):
     for i in range(n):
         assert np.array_equal(np.sort(nnl[i, :noi[i]]), nbr[off[i]:off[i + 1]]), i
     sim.close()
+
+
+# 8 particles per warp up to 25,000, 16 up to 65,000, then 32
+@pytest.mark.parametrize("n", [25_000, 25_001, 65_000, 65_001])
+def test_neighbour_counts_group_sizes(n, cuda):
+    """Counts of the neighbour walk and of the variable-h walk (same start h, one
+    sweep decides nothing: tolerance above every count) are the brute-force
+    counts at the edges of the group sizes."""
+    C = ics.rotating_cloud(n, seed=8)
+    rng = np.random.default_rng(n)
+    S = dict({k: C[k] for k in ("x", "y", "z")}, sml=C["sml"] * rng.uniform(0.7, 1.2, n), mass=np.full(n, 1.0 / n),
+             e=np.ones(n), rho=np.ones(n), p=np.ones(n), cs=np.ones(n), **{f: np.zeros(n) for f in ("vx", "vy", "vz")})
+    off, _ = O.frnn(S["x"], S["y"], S["z"], S["sml"])
+    for kw in (dict(integrate_sml=1), dict(variable_sml=1, nb_tolerance=1000)):
+        sim = Miluphpc(sph_cfg(integrate_energy=0, max_num_interactions=400, **kw), S,
+                       materials=[material(interactions=60, eos_type=0, K=1.0, gamma=1.0)])
+        sim.rhs(0)
+        assert np.array_equal(sim.numpy("sml"), S["sml"])
+        assert np.array_equal(sim.numpy("noi"), np.diff(off))
+        sim.close()
+
+
+# lists with appended entries are sorted with 2 entries per lane up to 64, 8 up
+# to 256, by one lane above
+@pytest.mark.parametrize("target", [55, 200, 270])
+@pytest.mark.parametrize("rounds", [0, 4])
+def test_appended_lists(target, rounds, cuda):
+    """Lists of a variable-h cloud equal the brute-force sets of its final h,
+    whatever length the appended lists are sorted at."""
+    n = 3000
+    C = ics.rotating_cloud(n, seed=9)
+    rng = np.random.default_rng(target)
+    h = C["sml"] * (target / 60.0) ** (1.0 / 3.0) * rng.uniform(0.8, 1.2, n)
+    S = dict({k: C[k] for k in ("x", "y", "z")}, sml=h, mass=np.full(n, 1.0 / n),
+             e=np.ones(n), rho=np.ones(n), p=np.ones(n), cs=np.ones(n), **{f: np.zeros(n) for f in ("vx", "vy", "vz")})
+    sim = Miluphpc(sph_cfg(variable_sml=1, integrate_energy=0, max_num_interactions=700, sml_band_rounds=rounds), S,
+                   materials=[material(interactions=target, eos_type=0, K=1.0, gamma=1.0)], want_nnl=True)
+    sim.rhs(0)
+    off, nbr = O.frnn(S["x"], S["y"], S["z"], sim.numpy("sml"))
+    noi = sim.numpy("noi")
+    assert np.array_equal(noi, np.diff(off))
+    nnl = sim.t["nnl"].cpu().numpy().reshape(n, 700)
+    for i in range(n):
+        assert np.array_equal(np.sort(nnl[i, :noi[i]]), nbr[off[i]:off[i + 1]]), i
+    sim.close()
