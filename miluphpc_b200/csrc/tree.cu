@@ -404,6 +404,103 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
     }
 }
 
+// The cell of each eight lanes of a warp (of an `act` group), one child slot per
+// lane: all children arrive in two round trips, where one lane takes one per
+// batch of slots.  The centre of mass is summed in slot order like above, from
+// the lanes' products; the quadrupole is reduced over the lanes.  Every lane of
+// the warp calls it; a shared-key bucket is left to the group's first lane.
+template <bool kLeafMask>
+__device__ __forceinline__ void cell_moments_wide(const TreeDev& T, bool act, int p, int want_quad, int want_box,
+                                                  double edge0, double inv_theta, bool local) {
+    const int lane = threadIdx.x & 31, sub = lane & 7, base = lane & 24;
+    int mask = 0, kid = 0;
+    int2 lk = make_int2(0, 0);
+    if (act) {
+        mask = __ldg(T.kmask + p);
+        kid = __ldg(T.kids + 8 * (size_t)p + sub);
+        lk = __ldg(T.link + p);
+    }
+    if (mask & 0x100) {
+        if (sub == 0) cell_moments<1, kLeafMask>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta, local);
+        act = false;
+        mask = 0;
+    }
+    const bool has = (mask >> sub) & 1;
+    double4 cc = make_double4(0., 0., 0., 0.);
+    float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+    float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+    float4 hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+    if (has) {
+        cc = ld_up_d4(&T.com[kid], local);
+        if (want_quad) {
+            a0 = ld_up(T.wrec + 4 * (size_t)kid + 2, local);
+            a1 = ld_up(T.wrec + 4 * (size_t)kid + 3, local);
+        }
+        if (want_box) {
+            lo = ld_up(&T.bmin[kid], local);
+            hi = ld_up(&T.bmax[kid], local);
+        }
+    }
+    const double tx = __dmul_rn(cc.x, cc.w), ty = __dmul_rn(cc.y, cc.w), tz = __dmul_rn(cc.z, cc.w);
+    double m = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+        const double vx = __shfl_sync(MHPC_FULL, tx, base + d), vy = __shfl_sync(MHPC_FULL, ty, base + d);
+        const double vz = __shfl_sync(MHPC_FULL, tz, base + d), vm = __shfl_sync(MHPC_FULL, cc.w, base + d);
+        if ((mask >> d) & 1) {
+            mx = __dadd_rn(mx, vx); my = __dadd_rn(my, vy); mz = __dadd_rn(mz, vz);
+            m = __dadd_rn(m, vm);
+        }
+    }
+    if (m > 0.0) {
+        mx = __ddiv_rn(mx, m);
+        my = __ddiv_rn(my, m);
+        mz = __ddiv_rn(mz, m);
+    }
+    if (want_box) {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            lo.x = fminf(lo.x, __shfl_xor_sync(MHPC_FULL, lo.x, o));
+            lo.y = fminf(lo.y, __shfl_xor_sync(MHPC_FULL, lo.y, o));
+            lo.z = fminf(lo.z, __shfl_xor_sync(MHPC_FULL, lo.z, o));
+            hi.x = fmaxf(hi.x, __shfl_xor_sync(MHPC_FULL, hi.x, o));
+            hi.y = fmaxf(hi.y, __shfl_xor_sync(MHPC_FULL, hi.y, o));
+            hi.z = fmaxf(hi.z, __shfl_xor_sync(MHPC_FULL, hi.z, o));
+        }
+    }
+    double q[6] = {0, 0, 0, 0, 0, 0};
+    int leaves = 0;
+    if (want_quad) {
+        const bool leaf = __float_as_int(a1.z) & ND_LEAF;
+        if (kLeafMask) leaves = (__ballot_sync(MHPC_FULL, has && leaf) >> base) & 0xff;
+        if (has) {
+            const double s0 = cc.x - mx, s1 = cc.y - my, s2 = cc.z - mz;
+            const double ss = s0 * s0 + s1 * s1 + s2 * s2;
+            const double w = cc.w;
+            q[0] = w * (3.0 * s0 * s0 - ss); q[1] = w * 3.0 * s0 * s1; q[2] = w * 3.0 * s0 * s2;
+            q[3] = w * (3.0 * s1 * s1 - ss); q[4] = w * 3.0 * s1 * s2; q[5] = w * (3.0 * s2 * s2 - ss);
+            if (!leaf) {
+                q[0] += a0.x; q[1] += a0.y; q[2] += a0.z; q[3] += a0.w; q[4] += a1.x; q[5] += a1.y;
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int i = 0; i < 6; ++i) q[i] += __shfl_xor_sync(MHPC_FULL, q[i], o);
+    }
+    if (act && sub == 0) {
+        T.com[p] = make_double4(mx, my, mz, m);
+        if (want_box) {
+            T.bmin[p] = lo;
+            T.bmax[p] = hi;
+        }
+        if (want_quad)
+            put_wrec(T, p, mx, my, mz, m, lk.y, mask, leaves,
+                     make_float4((float)q[0], (float)q[1], (float)q[2], (float)q[3]),
+                     make_float2((float)q[4], (float)q[5]), edge0, inv_theta);
+    }
+}
+
 // The upward pass in one launch.  Block b owns the sorted particles
 // [a0, a1) = [b C, (b + 1) C): it completes their leaves, then, deepest level
 // first with a block barrier between levels, every cell that starts and ends
@@ -440,8 +537,13 @@ constexpr int kUpHand = 1024;
 //   2            68       79        90       141         313
 //   4            55       93        97       120         262
 //   8                                        136         283         682   2504
+// With walk records up to kWideN particles one position per thread and a cell on
+// eight lanes, where a cell's time is its round trips: 54 us at 1,000, 57 at 20,011,
+// 68 at 100,003, 148 at 300,000.  (Without them a cell has too little to share:
+// 78 us against 55 at 131,072.)
 // (8 positions, above 2,000,000 particles, leave out the mask of leaf slots: no
 // walk of that size asks for it, and it cost 100 us at 2^24.)
+constexpr int kWideN = 200000;
 inline int up_per(int n) {
     if (n <= 8192) return 4;
     if (n <= 65536) return 1;
@@ -471,6 +573,28 @@ __device__ __forceinline__ void hand_off(const TreeDev& T, int p, Combine&& comb
     }
 }
 
+// The same for the parents of each eight lanes (-1: none), combined by eight
+// lanes; every lane of the warp calls it.
+template <typename CombineWide>
+__device__ __forceinline__ void hand_off_wide(const TreeDev& T, int p, CombineWide&& combine) {
+    const int lane = threadIdx.x & 31, base = lane & 24;
+    while (__any_sync(MHPC_FULL, p >= 0)) {
+        int go = 0;
+        if (lane == base && p >= 0) {
+            go = atomicAdd(T.arrive + p, 1) == cell_nkids(T, p) - 1;
+            if (go) T.arrive[p] = 0;
+        }
+        fence_acq_rel();
+        __syncwarp();
+        if (!__shfl_sync(MHPC_FULL, go, base)) p = -1;
+        fence_acq_rel();
+        combine(p >= 0, p, false);
+        fence_acq_rel();
+        __syncwarp();
+        if (p >= 0) p = __ldg(T.parent + p);
+    }
+}
+
 // Minimum over the block of per-thread aggregates, exclusive, from the left
 // (prefix) or from the right (suffix); identity 255.
 __device__ __forceinline__ void block_min_scans(int agg, int* wtot, int& pre, int& suf) {
@@ -496,8 +620,9 @@ __device__ __forceinline__ void block_min_scans(int agg, int* wtot, int& pre, in
     suf = min(right, lane < 31 ? qe : 255);
 }
 
-template <int kUpPer, typename Leaf, typename Combine>
-__device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, Combine&& combine) {
+template <int kUpPer, bool kWide, typename Leaf, typename Combine, typename CombineWide>
+__device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, Combine&& combine,
+                                             CombineWide&& combine_wide) {
     constexpr int kUpChunk = kUpPer * kUpBlock;
     __shared__ int queue[kUpBlock / 32][32 * kUpPer];             // cell
     __shared__ unsigned short qpos[kUpBlock / 32][32 * kUpPer];   // its first position - a0
@@ -592,12 +717,17 @@ __device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, C
             qi[w++] = (unsigned short)i;
         }
         __syncwarp();
-        for (int k = lane; k < total; k += 32) {
-            const int p = q[k];
-            combine(p, true);
+        for (int k0 = 0; k0 < total; k0 += kWide ? 4 : 32) {
+            const int k = k0 + (kWide ? lane >> 3 : lane);
+            const bool act = k < total;
+            const int p = act ? q[k] : -1;
+            if (kWide) combine_wide(act, p, true);
+            else if (act) combine(p, true);
             // parent of level L - 1 crossing a range boundary: queued for the hand-off
-            const int i = qi[k];
-            if (L > 1 && (pre[i] >= L - 1 || suf[i] >= L - 1)) queue_parent(p);
+            if (act && (!kWide || (lane & 7) == 0)) {
+                const int i = qi[k];
+                if (L > 1 && (pre[i] >= L - 1 || suf[i] >= L - 1)) queue_parent(p);
+            }
         }
         __syncwarp();
     }
@@ -605,10 +735,17 @@ __device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, C
     fence_acq_rel();
     __syncthreads();
     const int nh = min(nhand, kUpHand);
-    for (int k = threadIdx.x; k < nh; k += kUpBlock) hand_off(T, hand[k], combine);
+    if (kWide) {
+        for (int k0 = warp * 4; k0 < nh; k0 += kUpBlock / 8) {
+            const int k = k0 + (lane >> 3);
+            hand_off_wide(T, k < nh ? hand[k] : -1, combine_wide);
+        }
+    } else {
+        for (int k = threadIdx.x; k < nh; k += kUpBlock) hand_off(T, hand[k], combine);
+    }
 }
 
-template <int kUpPer>
+template <int kUpPer, bool kWide>
 __global__ void __launch_bounds__(kUpBlock, 3) k_upward(TreeDev T, const double* __restrict__ sx,
                                                      const double* __restrict__ sy, const double* __restrict__ sz,
                                                      const double* __restrict__ sm, int want_quad, int want_box,
@@ -616,10 +753,14 @@ __global__ void __launch_bounds__(kUpBlock, 3) k_upward(TreeDev T, const double*
                                                      const DevStatus* st) {
     if (st->code) return;
     const double edge0 = want_quad ? ord_to_dbl(ord[1]) - ord_to_dbl(ord[0]) : 0.0;
-    upward_chunk<kUpPer>(
+    upward_chunk<kUpPer, kWide>(
         T, [&](int a, int leaf) { leaf_moments(T, a, leaf, sx, sy, sz, sm, want_quad, want_box, edge0, inv_theta); },
         [&](int p, bool local) {
-            cell_moments<4, (kUpPer < 8)>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta, local);
+            cell_moments<kWide ? 1 : 4, (kUpPer < 8)>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta,
+                                                      local);
+        },
+        [&](bool act, int p, bool local) {
+            cell_moments_wide<(kUpPer < 8)>(T, act, p, want_quad, want_box, edge0, inv_theta, local);
         });
 }
 
@@ -628,7 +769,7 @@ __global__ void __launch_bounds__(kUpBlock, 3) k_upward(TreeDev T, const double*
 template <int kUpPer>
 __global__ void __launch_bounds__(kUpBlock, 4) k_hmax(TreeDev T, const double* __restrict__ h, const DevStatus* st) {
     if (st->code) return;
-    upward_chunk<kUpPer>(
+    upward_chunk<kUpPer, false>(
         T, [&](int a, int leaf) { T.hmax[leaf] = __double2float_ru(h[a]); },
         [&](int p, bool local) {
             const int km = __ldg(T.kmask + p);
@@ -646,7 +787,8 @@ __global__ void __launch_bounds__(kUpBlock, 4) k_hmax(TreeDev T, const double* _
                     if ((K.mask >> d) & 1) m = fmaxf(m, v[d]);
             }
             T.hmax[p] = m;
-        });
+        },
+        [](bool, int, bool) {});
 }
 
 
@@ -672,14 +814,18 @@ int tree_build(TreeDev& T, const uint64_t* skey, void* scan_scratch, DevStatus* 
 int tree_upward(TreeDev& T, const double* sx, const double* sy, const double* sz, const double* sm,
                 int want_quad, int want_box, const long long* ord, double theta, DevStatus* st, cudaStream_t s) {
     const double inv_theta = want_quad ? 1.0 / theta : 0.0;
-#define MHPC_UP(P_)                                                                                              \
-    k_upward<P_><<<(T.n + P_ * kUpBlock - 1) / (P_ * kUpBlock), kUpBlock, 0, s>>>(T, sx, sy, sz, sm, want_quad, \
-                                                                                 want_box, ord, inv_theta, st)
-    switch (up_per(T.n)) {
-        case 1: MHPC_UP(1); break;
-        case 2: MHPC_UP(2); break;
-        case 4: MHPC_UP(4); break;
-        default: MHPC_UP(8); break;
+#define MHPC_UP(P_, W_)                                                                                                \
+    k_upward<P_, W_><<<(T.n + P_ * kUpBlock - 1) / (P_ * kUpBlock), kUpBlock, 0, s>>>(T, sx, sy, sz, sm, want_quad, \
+                                                                                     want_box, ord, inv_theta, st)
+    if (want_quad && T.n <= kWideN) {
+        MHPC_UP(1, true);
+    } else {
+        switch (up_per(T.n)) {
+            case 1: MHPC_UP(1, false); break;
+            case 2: MHPC_UP(2, false); break;
+            case 4: MHPC_UP(4, false); break;
+            default: MHPC_UP(8, false); break;
+        }
     }
 #undef MHPC_UP
     CUDA_TRY(cudaGetLastError());

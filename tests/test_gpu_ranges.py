@@ -151,14 +151,15 @@ def test_sort_scratch_serves_smaller_n(cuda):
 
 # ------------------------------------------------------------- upward pass
 # 4 positions per thread up to 8,192, 1 up to 65,536, 2 up to 200,000, 4 up to 2,000,000,
-# then 8; nodes are counted in one block up to 16,384
-@pytest.mark.parametrize("n", [1, 2, 5, 8192, 8193, 16_384, 16_385, 65_536, 65_537, 200_001, 2_000_001])
+# then 8; with walk records (precision 1) eight lanes per cell up to 200,000; nodes are
+# counted in one block up to 16,384
+@pytest.mark.parametrize("n", [1, 2, 5, 8192, 8193, 16_384, 16_385, 65_536, 65_537, 200_000, 200_001, 2_000_001])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_upward_pass_sizes(n, precision, cuda):
     """The cells' masses and centres of mass are bit-equal to the oracle's
     (Lebesgue order: the same sums; compared as sorted lists, the numbering
     differs), whatever the block sizes."""
-    if precision and n > 100_000:
+    if precision and n > 300_000:
         pytest.skip("the block sizes are the same")
     P = ics.plummer(n, seed=12) if n > 1 else {k: np.array([0.5]) for k in ("x", "y", "z", "mass", "vx", "vy", "vz")}
     sim = Miluphpc(gravity_cfg(sfc=0, precision=precision, theta_mixed=0.3), P)
