@@ -44,7 +44,7 @@ constexpr int kWalkBlock = 128;
 //   W = 1                 93    170     223     267      418      793       2326
 //   W = 2                 58     98     134     177      369      748       2347
 //   W = 4                 38     57      84     161      352      772       2547
-//   W = 8                 31     40      89     176      436      989       3400
+//   W = 8                 29     37      89     176      436      989       3400
 __host__ __device__ constexpr int v2_stack(int W) { return 512 + 256 * (W - 1); }
 constexpr int kV2Reserve = 7 * 22 + 8;
 
@@ -139,10 +139,15 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
         double4 c = make_double4(0, 0, 0, 0);
         double dp = 0;
         int mask = 0;
+        int4 k0 = make_int4(0, 0, 0, 0), k1 = k0;
         if (act) {
             const int2 lk = __ldg(T.link + nd);
             c = ldg_d4(T.com + nd);
             mask = __ldg(T.kmask + nd);
+            if (W == 8) {  // a step's time is its round trips: child slots with the record
+                k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
+                k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
+            }
             const int L = lk.y & 0xff;
             if (lk.y & ND_LEAF) {
                 acc = L > 1;
@@ -226,8 +231,10 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
             return;
         }
         if (nkid) {
-            const int4 k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
-            const int4 k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
+            if (W < 8) {
+                k0 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd));
+                k1 = __ldg(reinterpret_cast<const int4*>(T.kids + 8 * (size_t)nd) + 1);
+            }
             const int all[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
             int pos = top + kbase + incl - nkid;
 #pragma unroll
@@ -951,7 +958,16 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
                 open = !ok;
             }
         }
-        const unsigned bl = __ballot_sync(MHPC_FULL, acc_leaf), bc = __ballot_sync(MHPC_FULL, acc_cell);
+        auto put_leaf = [&](int i) { S.lpos[i] = make_float4(nx, ny, nz, m); };
+        auto put_cell = [&](int i) {
+            S.cpos[i] = make_float4(nx, ny, nz, m);
+            S.cq0[i] = w2;
+            S.cq1[i] = make_float2(w3.x, w3.y);
+        };
+        const unsigned bl = __ballot_sync(MHPC_FULL, acc_leaf);
+        if (W == 1 && acc_leaf) put_leaf(nleaf + __popc(bl & lt));
+        const unsigned bc = __ballot_sync(MHPC_FULL, acc_cell);
+        if (W == 1 && acc_cell) put_cell(ncell + __popc(bc & lt));
         const int mask = open ? (__float_as_int(w3.z) >> 9) : 0;
         const bool bucket = open && (mask & 0x100);
         const unsigned bb = __ballot_sync(MHPC_FULL, bucket);
@@ -981,14 +997,9 @@ __global__ void __launch_bounds__(kListBlock, MHPC_LISTS_MIN_BLOCKS) k_grav_list
                 nl += S.cnt[q][0]; nc += S.cnt[q][1]; total += S.cnt[q][2]; ndefer += S.cnt[q][3];
             }
         }
-        if (acc_leaf) S.lpos[lbase + __popc(bl & lt)] = make_float4(nx, ny, nz, m);
+        if (W > 1 && acc_leaf) put_leaf(lbase + __popc(bl & lt));
         nleaf += nl;
-        if (acc_cell) {
-            const int i = cbase + __popc(bc & lt);
-            S.cpos[i] = make_float4(nx, ny, nz, m);
-            S.cq0[i] = w2;
-            S.cq1[i] = make_float2(w3.x, w3.y);
-        }
+        if (W > 1 && acc_cell) put_cell(cbase + __popc(bc & lt));
         ncell += nc;
         if (bucket) S.defer[dbase + __popc(bb & lt)] = nd;
         const int pushed = W > 1 ? total & 0xffff : total;
