@@ -558,7 +558,8 @@ int sort_pairs_u64(const uint64_t* keys_in, const int* vals_in, uint64_t* keys_o
         const size_t zero_bytes = (size_t)((char*)S.look - (char*)S.hist) +
                                   sizeof(unsigned long long) * kPasses * kRadix * (size_t)ntiles;
         CUDA_TRY(cudaMemsetAsync(S.hist, 0, zero_bytes, s));
-        k_hist<<<grid_for(n, kBlock, 148 * 4), kBlock, 0, s>>>(keys_in, n, S.hist);
+        // (1024 keys a block or more: a block ends with up to 2048 global atomics)
+        k_hist<<<grid_for(n, 4 * kBlock, 148 * 4), kBlock, 0, s>>>(keys_in, n, S.hist);
     }
     // per device (a process may drive several GPUs); cheap host calls
     CUDA_TRY(cudaFuncSetAttribute(k_pass<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
