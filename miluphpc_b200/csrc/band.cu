@@ -41,7 +41,7 @@ struct BandRule {
 
 struct SelectSmem {
     int stk[kWalkStack];
-    int rf[32], re[32];
+    int rf[32];
     double d2[kBandCap];
     int cnt;
 };
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kBandBlock, kSelectBlocks) k_band_select(TreeD
                 }
             } else {
                 SelectVisit v{sx, sy, sz, h, px, py, pz, rad * rad, (long)s, m};
-                warp_walk(T, M, true, px, py, pz, rad, node_hmax, m->stk, m->rf, m->re, st, v);
+                warp_walk(T, M, true, px, py, pz, rad, node_hmax, m->stk, m->rf, st, v);
             }
             __syncwarp();
             const int found = m->cnt;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kBandBlock, kSelectBlocks) k_band_select(TreeD
 
 struct EventSmem {
     int stk[kWalkStack];
-    int rf[32], re[32];
+    int rf[32];
 };
 
 // Who reports a pair whose status changes.  Only particles whose h changed
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kBandBlock, kEventBlocks) k_band_events(TreeDe
             }
         } else {
             EventVisit v{sx, sy, sz, h, hnew, px, py, pz, hio * hio, hin * hin, (long)s, ev, cap, ctr};
-            warp_walk(T, M, true, px, py, pz, hin, node_hmax, m->stk, m->rf, m->re, st, v);
+            warp_walk(T, M, true, px, py, pz, hin, node_hmax, m->stk, m->rf, st, v);
         }
         __syncwarp();
     }

@@ -63,9 +63,9 @@ constexpr double kCut = 1.5;
 // 1.3e-6 H^2, and a pair farther apart cannot come within that of H^2 while
 // R < 1e5 H.  The walk and the box tests are conservative too, so each
 // neighbour set equals the brute-force set.
-// Bound: issue and fixed latency (58 % of the issue slots, 18 resident warps per
+// Bound: issue and fixed latency (58 % of the issue slots, 18 active warps per
 // SM).  List walk in us with FP64 tests and grown boxes / now: Sedov lattice of
-// 262,144 particles 258 / 224, of 2,097,152 1693 / 1432; all walks of a cloud step,
+// 262,144 particles 258 / 203, of 2,097,152 1693 / 1303; all walks of a cloud step,
 // 2^20 particles 2229 / 1843, 2^23 16600 / 13850.
 //
 // mode 0: write lists (h_i = h[i], h_j = h[j]) for all particles; mode 1:
@@ -84,7 +84,7 @@ struct FrnnSmem {
     float4 cp[kPool];                                     // candidate: offset from the centre, h_j^2
     int cj[kPool];                                        // candidate particle
     unsigned char lst[4][kPool];                          // pool slots per sub-group
-    int rf[32], rend[32];                                 // staged ranges: first, end (prefix)
+    int rf[32];                                           // staged ranges: first particle less begin
     float4 slo[4], shi[4];                                // sub-group boxes about the centre; largest h (.w)
 };
 
@@ -192,39 +192,46 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
             const float ix = __shfl_sync(MHPC_FULL, fx, src), iy = __shfl_sync(MHPC_FULL, fy, src);
             const float iz = __shfl_sync(MHPC_FULL, fz, src), ih2 = __shfl_sync(MHPC_FULL, fh2, src);
             const int is = __shfl_sync(MHPC_FULL, (int)s, src);
-            const bool iact = __shfl_sync(MHPC_FULL, (int)active, src) != 0;
+            const int mine = __shfl_sync(MHPC_FULL, (int)active, src) ? cntg : 0;  // entries to test
             int kb = __shfl_sync(MHPC_FULL, k, src);
             const unsigned pmask = 0x01010101u << p;
+            int* const row = nbr + nb_index(is, 0, maxnb);
             // two entries per lane and step: their loads and sums overlap
             for (int c0 = 0; c0 < cntg; c0 += 8) {
-                bool hit[2];
+                bool hit[2], near[2];
                 int j[2];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int c = c0 + 4 * u + q;
-                    hit[u] = false;
-                    j[u] = 0;
-                    if (iact && c < cntg) {
+                    hit[u] = near[u] = false;
+                    j[u] = is;
+                    if (c < mine) {
                         const int slot = S.lst[sg][c];
                         j[u] = S.cj[slot];
                         const float4 q4 = S.cp[slot];
                         const float dx = ix - q4.x, dy = iy - q4.y, dz = iz - q4.z;
                         const float over = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - fminf(ih2, q4.w);
                         hit[u] = over < -band;
-                        if (!hit[u] && !(over > band)) {
-                            const double hs = sh[is], hj = sh[j[u]];
-                            const double d = d2_exact(sx[is] - sx[j[u]], sy[is] - sy[j[u]], sz[is] - sz[j[u]]);
+                        near[u] = !(fabsf(over) > band);
+                    }
+                }
+                if (near[0] || near[1]) {
+                    const double hs = sh[is], xs = sx[is], ys = sy[is], zs = sz[is];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                        if (near[u]) {
+                            const double hj = sh[j[u]];
+                            const double d = d2_exact(xs - sx[j[u]], ys - sy[j[u]], zs - sz[j[u]]);
                             hit[u] = d < hs * hs && d < hj * hj;
                         }
-                        hit[u] = hit[u] && j[u] != is;
-                    }
                 }
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
+                    hit[u] = hit[u] && j[u] != is;
                     const unsigned b = __ballot_sync(MHPC_FULL, hit[u]) & pmask;
                     if (MODE != 1 && hit[u]) {
                         const int pos = kb + __popc(b & lt);
-                        if (pos < maxnb) nbr[nb_index(is, pos, maxnb)] = j[u];
+                        if (pos < maxnb) row[32 * pos] = j[u];
                     }
                     kb += __popc(b);
                 }
@@ -275,13 +282,13 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
             }
         }
         // push the children of opened cells
+        // (one scan for the children, at most 256, and for the staged ranges;
+        // ranges above 65,536 particles, a shared-key bucket's, by a second one)
         const int nkid = __popc(kmask);
-        int incl = nkid;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(MHPC_FULL, incl, o);
-            if (lane >= o) incl += v;
-        }
+        const bool wide = __any_sync(MHPC_FULL, rlen > 65536);
+        const int both = warp_scan(nkid | (wide ? 0 : rlen << 9), lane);
+        const int incl = both & 511;
+        const int rincl = wide ? warp_scan(rlen, lane) : both >> 9;
         const int total = __shfl_sync(MHPC_FULL, incl, 31);
         if (top + total > kStack) {
             // unreachable by the bound on kk; stop instead of overrunning
@@ -298,36 +305,24 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
                 if ((kmask >> d) & 1) S.stk[wpos++] = all[d];
         }
         top += total;
-        // staged ranges: compact, with the running end of each
-        int rincl = rlen;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(MHPC_FULL, rincl, o);
-            if (lane >= o) rincl += v;
-        }
+        // staged ranges: compact, each with its first particle less its begin
+        const int begin = rincl - rlen;
         const int ncand = __shfl_sync(MHPC_FULL, rincl, 31);
         const unsigned br = __ballot_sync(MHPC_FULL, rlen > 0);
-        const int nr = __popc(br);
-        if (rlen > 0) {
-            const int r = __popc(br & lt);
-            S.rf[r] = rf;
-            S.rend[r] = rincl;
-        }
+        if (rlen > 0) S.rf[__popc(br & lt)] = rf - begin;
         __syncwarp();
+        int begun = 0;  // ranges that begin before this batch
         for (int c0 = 0; c0 < ncand; c0 += 32) {
             if (pool + 32 > kPool) flush();
             const int c = c0 + lane;
             int mask = 0, j = 0;
             float rx = 0.f, ry = 0.f, rz = 0.f;
             double hj = 0;
+            // a lane's range is the last that begins at or before it
+            const unsigned at = (unsigned)(begin - c0);
+            const unsigned bits = __reduce_or_sync(MHPC_FULL, rlen > 0 && at < 32u ? 1u << at : 0u);
             if (c < ncand) {
-                int lo = 0, hi_r = nr - 1;
-                while (lo < hi_r) {
-                    const int mid = (lo + hi_r) >> 1;
-                    if (S.rend[mid] > c) hi_r = mid;
-                    else lo = mid + 1;
-                }
-                j = S.rf[lo] + c - (lo ? S.rend[lo - 1] : 0);
+                j = S.rf[begun + __popc(bits & (2u * lt + 1u)) - 1] + c;
                 const double qx = __ldg(sx + j), qy = __ldg(sy + j), qz = __ldg(sz + j);
                 hj = __ldg(sh + j);
                 rx = (float)(qx - cx); ry = (float)(qy - cy); rz = (float)(qz - cz);
@@ -341,21 +336,20 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
                     mask |= (int)(lim > 0.f && fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= lim * lim) << q;
                 }
             }
-            const unsigned bp = __ballot_sync(MHPC_FULL, mask != 0);
+            const unsigned b0 = __ballot_sync(MHPC_FULL, mask & 1), b1 = __ballot_sync(MHPC_FULL, mask & 2);
+            const unsigned b2 = __ballot_sync(MHPC_FULL, mask & 4), b3 = __ballot_sync(MHPC_FULL, mask & 8);
+            const unsigned bp = b0 | b1 | b2 | b3;
             if (mask) {
                 const int slot = pool + __popc(bp & lt);
                 S.cp[slot] = make_float4(rx, ry, rz, (float)(hj * hj));
                 S.cj[slot] = j;
-                const unsigned b0 = __ballot_sync(bp, mask & 1), b1 = __ballot_sync(bp, mask & 2);
-                const unsigned b2 = __ballot_sync(bp, mask & 4), b3 = __ballot_sync(bp, mask & 8);
                 if (mask & 1) S.lst[0][cnt0 + __popc(b0 & lt)] = (unsigned char)slot;
                 if (mask & 2) S.lst[1][cnt1 + __popc(b1 & lt)] = (unsigned char)slot;
                 if (mask & 4) S.lst[2][cnt2 + __popc(b2 & lt)] = (unsigned char)slot;
                 if (mask & 8) S.lst[3][cnt3 + __popc(b3 & lt)] = (unsigned char)slot;
             }
-            const unsigned a0 = __ballot_sync(MHPC_FULL, mask & 1), a1 = __ballot_sync(MHPC_FULL, mask & 2);
-            const unsigned a2 = __ballot_sync(MHPC_FULL, mask & 4), a3 = __ballot_sync(MHPC_FULL, mask & 8);
-            cnt0 += __popc(a0); cnt1 += __popc(a1); cnt2 += __popc(a2); cnt3 += __popc(a3);
+            begun += __popc(bits);
+            cnt0 += __popc(b0); cnt1 += __popc(b1); cnt2 += __popc(b2); cnt3 += __popc(b3);
             pool += __popc(bp);
         }
         __syncwarp();
@@ -402,7 +396,7 @@ __global__ void __launch_bounds__(kBlock) k_count_warp(TreeDev T, const double* 
                                                        const float* __restrict__ node_hmax, int* __restrict__ count,
                                                        DevStatus* st) {
     __shared__ int stk[kWarps][kWalkStack];
-    __shared__ int rfs[kWarps][32], rends[kWarps][32];
+    __shared__ int rfs[kWarps][32];
     if (st->code) return;
     const int M = *T.nodes;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -413,7 +407,7 @@ __global__ void __launch_bounds__(kBlock) k_count_warp(TreeDev T, const double* 
         const double px = sx[s], py = sy[s], pz = sz[s], hi = sh[s];
         int k = 0;
         CountVisit v{sx, sy, sz, sh, px, py, pz, hi * hi, (long)s, &k};
-        warp_walk(T, M, true, px, py, pz, hi, node_hmax, stk[w], rfs[w], rends[w], st, v);
+        warp_walk(T, M, true, px, py, pz, hi, node_hmax, stk[w], rfs[w], st, v);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(MHPC_FULL, k, o);
         if (lane == 0) count[s] = k;

@@ -24,6 +24,16 @@ __device__ __forceinline__ void warp_append(bool want, int v, int* list, int* co
     if (want) list[base + __popc(b & ((1u << lane) - 1u))] = v;
 }
 
+// inclusive sum over the lanes
+__device__ __forceinline__ int warp_scan(int v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(MHPC_FULL, v, o);
+        if (lane >= o) v += u;
+    }
+    return v;
+}
+
 constexpr int kWalkStack = 512;
 constexpr int kWalkReserve = 7 * 22 + 8;
 constexpr int kWalkSmall = 16;   // cells with at most this many particles are tested whole
@@ -40,7 +50,7 @@ constexpr int kWalkSmall = 16;   // cells with at most this many particles are t
 // that a depth-first descent (7 per level, 22 levels) always fits on top.
 template <class Visit>
 __device__ __forceinline__ void warp_walk(const TreeDev& T, int M, bool valid, double px, double py, double pz,
-                                          double rad, const float* __restrict__ node_hmax, int* S, int* RF, int* RE,
+                                          double rad, const float* __restrict__ node_hmax, int* S, int* RF,
                                           DevStatus* st, Visit& visit) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
@@ -87,13 +97,13 @@ __device__ __forceinline__ void warp_walk(const TreeDev& T, int M, bool valid, d
                 }
             }
         }
+        // (one scan for the children, at most 256, and for the candidate ranges;
+        // ranges above 65,536 particles, a shared-key bucket's, by a second one)
         const int nkid = __popc(kmask);
-        int incl = nkid;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(MHPC_FULL, incl, o);
-            if (lane >= o) incl += v;
-        }
+        const bool wide = __any_sync(MHPC_FULL, rlen > 65536);
+        const int both = warp_scan(nkid | (wide ? 0 : rlen << 9), lane);
+        const int incl = both & 511;
+        const int rincl = wide ? warp_scan(rlen, lane) : both >> 9;
         const int total = __shfl_sync(MHPC_FULL, incl, 31);
         if (top + total > kWalkStack) {  // unreachable by the bound on kk
             if (lane == 0) set_status(st, MHPC_ERR_DEPTH, 8);
@@ -107,30 +117,19 @@ __device__ __forceinline__ void warp_walk(const TreeDev& T, int M, bool valid, d
                 if ((kmask >> d) & 1) S[wpos++] = all[d];
         }
         top += total;
-        // candidate ranges of this step with running ends
-        int rincl = rlen;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(MHPC_FULL, rincl, o);
-            if (lane >= o) rincl += v;
-        }
+        // candidate ranges of this step: compact, each with its first particle less
+        // its begin; a lane's range is the last that begins at or before it
+        const int begin = rincl - rlen;
         const int ncand = __shfl_sync(MHPC_FULL, rincl, 31);
         const unsigned br = __ballot_sync(MHPC_FULL, rlen > 0);
-        const int nr = __popc(br);
-        if (rlen > 0) {
-            const int slot = __popc(br & lt);
-            RF[slot] = rf;
-            RE[slot] = rincl;
-        }
+        if (rlen > 0) RF[__popc(br & lt)] = rf - begin;
         __syncwarp();
-        for (int c = lane; c < ncand; c += 32) {
-            int lo = 0, hr = nr - 1;
-            while (lo < hr) {
-                const int mid = (lo + hr) >> 1;
-                if (RE[mid] > c) hr = mid;
-                else lo = mid + 1;
-            }
-            visit(RF[lo] + c - (lo ? RE[lo - 1] : 0));
+        int begun = 0;  // ranges that begin before this batch
+        for (int c0 = 0; c0 < ncand; c0 += 32) {
+            const unsigned at = (unsigned)(begin - c0);
+            const unsigned bits = __reduce_or_sync(MHPC_FULL, rlen > 0 && at < 32u ? 1u << at : 0u);
+            if (c0 + lane < ncand) visit(RF[begun + __popc(bits & (2u * lt + 1u)) - 1] + c0 + lane);
+            begun += __popc(bits);
         }
         __syncwarp();
     }

@@ -289,3 +289,23 @@ def test_appended_lists(target, rounds, cuda):
     for i in range(n):
         assert np.array_equal(np.sort(nnl[i, :noi[i]]), nbr[off[i]:off[i + 1]]), i
     sim.close()
+
+
+def test_neighbour_walk_wide_bucket(cuda):
+    """A shared-key bucket of more than 65,536 particles, which the walks stage as
+    one range: 80,000 particles on a line shorter than a grid cell, 2.5 spacings
+    of h, so each has its two neighbours on either side."""
+    n, d = 80_000, 5e-13
+    x = np.concatenate([0.3 + d * np.arange(n), [0.0, 1.0]])
+    y, z = np.full(n + 2, 0.3), np.full(n + 2, 0.3)
+    y[n:] = z[n:] = [0.0, 1.0]
+    h = np.full(n + 2, 2.5 * d)
+    S = dict(x=x, y=y, z=z, sml=h, mass=np.full(n + 2, 1.0 / n), e=np.ones(n + 2), rho=np.ones(n + 2),
+             p=np.ones(n + 2), cs=np.ones(n + 2), **{f: np.zeros(n + 2) for f in ("vx", "vy", "vz")})
+    want = np.array([np.sum(np.abs(x[max(0, i - 4):min(n, i + 5)] - x[i]) < h[i]) - 1 for i in range(n)])
+    sim = Miluphpc(sph_cfg(integrate_energy=0, max_num_interactions=64), S,
+                   materials=[material(interactions=60, eos_type=0, K=1.0, gamma=1.0)])
+    sim.rhs(0)
+    noi = sim.numpy("noi")
+    assert np.array_equal(noi[:n], want) and (noi[n:] == 0).all()
+    sim.close()
