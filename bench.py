@@ -437,17 +437,17 @@ def run_ours(args, wl):
     if rank == 0:
         traffic = load_traffic(args.workload, args.variant)
         if sph:
-            # internal forces: the particle's own state read once (FP64: x,y,z,v,m,h,rho,p,c_s = 88 B;
-            # mixed: the packed FP32 views, 56 B), the rates written (40 B) and its neighbour
+            # internal forces: the particle's own records read once (FP64: three of 32 B, mixed:
+            # two), the rates written (40 B) and its neighbour
             # list read (4 B per entry); neighbour gathers stay on chip (SFC order) and are
             # reported separately
             mixed = args.variant == "mixed"
-            own = 56.0 if mixed else 88.0
+            own = 64.0 if mixed else 96.0
             nb = float(last.get("mean_noi") or 0.0)
             nbytes = (own + 40.0 + 4.0 * nb) * n
             achieved = nbytes / (kern_ms / 1e3) / 1e9
             peak = hbm_peak_gbs()
-            roof = {"kernel": "k_forces_f32" if mixed else "k_forces", "bound": "hbm", "achieved": round(achieved, 1),
+            roof = {"kernel": "k_forces", "bound": "hbm", "achieved": round(achieved, 1),
                     "peak": peak["value"], "unit": "GB/s", "frac": round(achieved / peak["value"], 4),
                     "traffic": traffic, "peak_source": peak["source"],
                     "work_unit": "%d B state read + 40 B written + 4 B per neighbour-list entry, per particle"
@@ -502,7 +502,7 @@ def run_ours(args, wl):
             "roofline": roof,
             "cpu_baseline": cpu,
             "e2e": e2e,
-            "gpu_launches": args.steps * launches_per_step(args.variant, wl["kind"], args.band_rounds)
+            "gpu_launches": args.steps * launches_per_step(args.variant, wl["kind"], n, args.band_rounds)
             + (refresh_launches(sim_cfg_refresh, step_t0, args.steps) if learned_on else 0),
             "clocks": clk,
         }
@@ -648,36 +648,36 @@ def hbm_peak_gbs():
         return {"value": 6650.0, "source": "fallback 6.65 TB/s"}
 
 
-def launches_per_step(variant, kind="gravity", band_rounds=8):
-    """This library's kernel launches in one timed step (counted from the
-    launch sequence; the ncu launch lists in profiles/ show the same)."""
-    # every RHS: bbox, bbox_finish, keys, hist, hist_scan, 8 onesweep (13), gather (1),
-    # tree: lcp, count, 4 scan, copy_total, zero_cells, nodes (9), upward pass (1)
-    tree = 13 + 1 + 9 + 1
+def launches_per_step(variant, kind, n, band_rounds=8):
+    """This library's kernel launches in one timed step of n particles (counted
+    from the launch sequence; the ncu launch lists in profiles/ show the same)."""
     mixed = variant == "mixed"
+    fields = {"sph": 10, "cloud": 8}.get(kind, 4)
+    # every RHS: bbox, keys; sort in one block, by look-back (histograms, 8 passes) or
+    # by counted tiles (8 x 3); gather (by records: 2); tree: counts and scan in one
+    # block or counts, 3 scan, clearing; nodes; upward pass
+    sort = 1 if n <= 4096 else 9 if n <= 600_000 else 24
+    gather = 2 if 8 * fields * n >= 192 << 20 else 1
+    tree = 2 + sort + gather + (1 if n <= 16_384 else 5) + 1 + 1
     if kind == "sph":
-        # frnn, (mixed: position pack), density+EOS, forces; noi export on the
-        # first RHS only; predictor-corrector: 3 step-size kernels, predictor, corrector
+        # frnn, record pack, density+EOS, forces; noi export on the first RHS only;
+        # predictor-corrector: 3 step-size kernels, predictor, corrector
         # (+1: the status fold at the start of every SPH right-hand side)
-        rhs = 1 + tree + 1 + (1 if mixed else 0) + 2
+        rhs = 1 + tree + 4
         return (rhs + 1) + rhs + 3 + 2
     grav = tree + 1  # + the walk
     if kind == "cloud":
-        # variable h on lists: copy of h, largest-h bounds (one upward pass), the
-        # list walk of the starting h, the first sweep's list (flags, 4 scan,
-        # compact), 7 sweeps x (update, event reset, events, marks, filter, appends,
-        # commit, gated re-walk), the next list of each later sweep (6), record after
-        # the first sweep, final list + record, sort of the appended lists, list
-        # statistics, scatter of h; band repair: 2 copies,
-        # rounds x (flags, 4 scan, compact, select, events, remove, compact, add,
-        # commit), sort of the appended lists, scatter of h; (mixed: position pack)
-        # density, forces, noi export, band statistics; learned h: apply, collect,
-        # features; explicit Euler update
-        vh = 1 + 1 + 1 + 6 + 7 * 8 + 6 + 1 + 2 + 1 + 1 + 1
-        band = (2 + 12 * band_rounds + 1 + 1) if band_rounds > 0 else 0
-        sphk = band + (1 if mixed else 0) + 4
+        # variable h on lists: start, largest-h bounds (one upward pass), the list
+        # walk of the starting h, 7 sweeps x (update, events, marks, filter, appends,
+        # commit, gated re-walk), list statistics; without a band repair the sort of
+        # the appended lists and the scatter of h; band repair: start, rounds x (list,
+        # select, events, marks, filter, appends, commit), sort of the appended lists,
+        # scatter of h; record pack, density, forces, noi export, band statistics;
+        # learned h: apply, collect, features; explicit Euler update
+        vh = 3 + 7 * 7 + 1
+        band = 1 + 7 * band_rounds + 2 if band_rounds > 0 else 2
         learned = 3 if mixed else 0
-        return 1 + grav + vh + sphk + learned + 1  # status fold, ..., explicit Euler
+        return 1 + grav + vh + band + 5 + learned + 1  # status fold, ..., explicit Euler
     return grav + 2  # leapfrog updateX, updateV
 
 
