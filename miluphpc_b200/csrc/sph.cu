@@ -66,7 +66,8 @@ constexpr double kCut = 1.5;
 // Bound: issue and fixed latency (58 % of the issue slots, 18 active warps per
 // SM).  List walk in us with FP64 tests and grown boxes / now: Sedov lattice of
 // 262,144 particles 258 / 203, of 2,097,152 1693 / 1303; all walks of a cloud step,
-// 2^20 particles 2229 / 1843, 2^23 16600 / 13850.
+// 2^20 particles 2229 / 1500, 2^23 16600 / 10500.  Of the 1303: the tree walk 334,
+// staging the candidates 180, pair tests and list writes 790.
 //
 // mode 0: write lists (h_i = h[i], h_j = h[j]) for all particles; mode 1:
 // count only, with h_i = h[i], h_j = h[j] (the variable-h sweep passes the
