@@ -71,6 +71,9 @@ struct mhpc_ctx {
     int* nb_appended = nullptr;  // [n] lists with appended entries (zero between calls)
     bool band_ran = false;
     bool dens_ready = false;  // the sorted rho, p, c_s are the density pass's of this tree
+    // the form of the pair sums (SphParams::mixed) that the records ra, rb, rc hold
+    // for this tree, the current h and the density pass's rho, p, c_s; -1: none
+    int rec_form = -1;
     // run totals of the per-RHS counters (SPH configurations); st_pending: *st
     // holds a finished RHS whose counters are not yet in *run
     RunTotals* run = nullptr;
@@ -205,6 +208,7 @@ constexpr long kRecordBytes = 192L << 20;
 int stage_tree_build(mhpc_ctx* c, const mhpc_particles* p) {
     const int n = p->n;
     cudaStream_t s = c->stream;
+    c->rec_form = -1;
     TRY(launch_bbox(p->x, p->y, p->z, n, c->ord, c->st, s));
     TRY(launch_keys(p->x, p->y, p->z, n, c->ord, c->cfg.sfc, c->keys, nullptr, s));
     record(c, EV_KEYS);
@@ -340,6 +344,7 @@ int stage_frnn(mhpc_ctx* c, const mhpc_particles* p, bool variable_h, bool learn
     const int target = sph_target(c);
     c->frnn_learned = learned && variable_h;
     if (variable_h) {
+        c->rec_form = -1;  // h changes below
         if (learned)
             CUDA_TRY(cudaMemcpyAsync(c->h_start, c->sh, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
         // learned path: start the iteration from the predicted h; particles whose
@@ -412,6 +417,7 @@ int stage_density_eos(mhpc_ctx* c, const mhpc_particles* p) {
     if (c->cfg.balsara) TRY(sph_balsara(P, S, c->nbr, c->noi, c->st, c->stream));
     record(c, EV_DENS);
     c->dens_ready = true;
+    c->rec_form = P.mixed;
     return MHPC_OK;
 }
 
@@ -426,7 +432,8 @@ int stage_forces(mhpc_ctx* c, const mhpc_particles* p) {
     SphSorted S = sph_sorted(c, p);
     const int target = sph_target(c);
     const bool learned = c->frnn_learned;
-    TRY(sph_forces(P, S, c->dens_ready, c->nbr, c->noi, c->perm, p->ax, p->ay, p->az, p->drhodt, p->dedt, p->dsmldt, c->st, s));
+    TRY(sph_forces(P, S, c->dens_ready && c->rec_form == P.mixed, c->nbr, c->noi, c->perm, p->ax, p->ay, p->az,
+                   p->drhodt, p->dedt, p->dsmldt, c->st, s));
     if (p->nnl || p->noi) TRY(sph_export_nnl(P, c->nbr, c->noi, c->perm, p->nnl, p->noi, s));
     if (c->cfg.variable_sml) TRY(sph_band_stats(P, c->noi, target, c->cfg.nb_tolerance, c->st, s));
     record(c, EV_FORCES);

@@ -84,7 +84,9 @@ int sph_density_eos(const SphParams& P, const SphSorted& S, const int* nbr, cons
 int sph_balsara(const SphParams& P, const SphSorted& S, const int* nbr, const int* noi, DevStatus* st,
                 cudaStream_t s);
 // Internal forces; P.mixed: pair terms in FP32, FP64 accumulation.  packed: the
-// records of S are those of the density pass of this tree and lists.
+// records of S are those of a density pass of this tree in the same form
+// (P.mixed), and h has not changed since; otherwise they are packed anew from
+// the sorted state.
 int sph_forces(const SphParams& P, const SphSorted& S, bool packed, const int* nbr, const int* noi, const int* perm,
                double* ax, double* ay, double* az, double* drhodt, double* dedt, double* dsmldt, DevStatus* st,
                cudaStream_t s);

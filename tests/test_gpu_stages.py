@@ -364,6 +364,51 @@ def test_stage_exports_equal_rhs(cuda):
     b.close()
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("between", ["no density", "precision", "second search"])
+def test_forces_on_current_state(between, precision, cuda):
+    """mhpc_forces sums over the state as it is when it is called: the caller's
+    rho, p and c_s where no density pass ran on this tree; the density pass's
+    after a change of precision; the current h after a variable-h search that
+    follows the density pass.  FP64 sums within 1e-10 of the largest rate, FP32
+    within 2e-5 (the bars of this file)."""
+    second = between == "second search"
+    S, C = _cloud_state(5_000, spread=(0.7, 1.4)) if second else (_sedov_state(18), None)
+    n = len(S["x"])
+    rng = np.random.default_rng(3)
+    if between == "no density":
+        for k in ("rho", "p", "cs"):
+            S[k] = rng.uniform(0.5, 1.5, n)
+    mat = material(interactions=60, eos_type=0, K=0.3, gamma=1.4)
+    first = 1 - precision if between == "precision" else precision
+    cfg = sph_cfg(precision=first, variable_sml=int(second), max_num_interactions=400)
+    sim = Miluphpc(cfg, S, materials=[mat])
+    lib, sp = L(), ctypes.byref(sim.soa)
+    _lib.check(lib.mhpc_tree_build(sim.ctx, sp), "tree_build")
+    _lib.check(lib.mhpc_com(sim.ctx, sp), "com")
+    _lib.check(lib.mhpc_frnn(sim.ctx, sp, 0, 0), "frnn")
+    if between != "no density":
+        _lib.check(lib.mhpc_density_eos(sim.ctx, sp), "density_eos")
+    if second:
+        _lib.check(lib.mhpc_frnn(sim.ctx, sp, 1, 0), "frnn with variable h")
+    cfg.precision = precision
+    sim.set_config(cfg)
+    _lib.check(lib.mhpc_forces(sim.ctx, sp), "forces")
+    _lib.check(lib.mhpc_ctx_status(sim.ctx), "status")
+    h = sim.numpy("sml")
+    assert np.any(h != S["sml"]) == second
+    off, nbr = O.frnn(S["x"], S["y"], S["z"], h)
+    assert np.array_equal(sim.numpy("noi"), np.diff(off))
+    f = O.forces(S["x"], S["y"], S["z"], S["vx"], S["vy"], S["vz"], S["mass"], h, sim.numpy("rho"), sim.numpy("p"),
+                 sim.numpy("cs"), off, nbr, 1.0, 2.0, avg_h=second)
+    frac = 2e-5 if precision else 1e-10
+    scale = np.abs(np.stack(f[:3])).max()
+    for k, want, top in [(k, w, scale) for k, w in zip(("ax", "ay", "az"), f[:3])] + \
+            [("drhodt", f[3], np.abs(f[3]).max()), ("dedt", f[4], np.abs(f[4]).max())]:
+        np.testing.assert_allclose(sim.numpy(k), want, rtol=0, atol=frac * top, err_msg=k)
+    sim.close()
+
+
 # ------------------------------------------------- neighbour-band repair
 def test_band_repair_matches_oracle(cuda):
     """The band repair (sml_band_rounds) from the h the variable-h iteration
