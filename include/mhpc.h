@@ -167,7 +167,8 @@ int mhpc_keys(const double* x, const double* y, const double* z, int n, const do
 /* HelperNS::sortArray (src/helper.cu:150-166) with TreeNS::prepareSorting
  * (tree.cu:1404-1413): stable ascending sort of 64-bit keys with int values
  * (vals_in NULL = 0..n-1).  Scratch is caller-provided device memory of
- * mhpc_sort_scratch_bytes(n) bytes; the inputs are not modified. */
+ * mhpc_sort_scratch_bytes(n) bytes; the inputs are not modified, unless
+ * keys_out is keys_in or vals_out is vals_in (sorted in place). */
 size_t mhpc_sort_scratch_bytes(int n);
 int mhpc_sort_pairs(const uint64_t* keys_in, const int* vals_in, uint64_t* keys_out,
                     int* vals_out, int n, void* scratch, size_t scratch_bytes, void* stream);

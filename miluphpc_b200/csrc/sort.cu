@@ -321,7 +321,8 @@ k_pass(const uint64_t* __restrict__ kin, const int* __restrict__ vin, uint64_t* 
 // All passes in one block, for at most THREADS x ITEMS keys.  Keys
 // and their input positions stay in shared memory; a pass ranks like k_pass.
 // Slots from n on hold the largest key and come last: they follow every input
-// position, and the sort is stable.
+// position, and the sort is stable.  The outputs may be the inputs' arrays (the
+// other forms go through scratch), so none of the four is __restrict__.
 template <int THREADS, int ITEMS>
 struct BlockSortSmem {
     uint64_t key[THREADS * ITEMS];
@@ -332,10 +333,8 @@ struct BlockSortSmem {
 };
 
 template <int THREADS, int ITEMS>
-__global__ void __launch_bounds__(THREADS) k_block_sort(const uint64_t* __restrict__ kin,
-                                                                  const int* __restrict__ vin,
-                                                                  uint64_t* __restrict__ kout,
-                                                                  int* __restrict__ vout, int n) {
+__global__ void __launch_bounds__(THREADS) k_block_sort(const uint64_t* kin, const int* vin, uint64_t* kout,
+                                                        int* vout, int n) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BlockSortSmem<THREADS, ITEMS>& S = *reinterpret_cast<BlockSortSmem<THREADS, ITEMS>*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -345,7 +344,7 @@ __global__ void __launch_bounds__(THREADS) k_block_sort(const uint64_t* __restri
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const int idx = base + i * 32;
-        key[i] = idx < n ? __ldg(kin + idx) : ~0ULL;
+        key[i] = idx < n ? kin[idx] : ~0ULL;
         pos[i] = (unsigned short)idx;
     }
     const unsigned lt = lanemask_lt();
@@ -400,12 +399,20 @@ __global__ void __launch_bounds__(THREADS) k_block_sort(const uint64_t* __restri
             pos[i] = S.pos[base + i * 32];
         }
     }
+    // every value is read before the first is written
+    int val[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        val[i] = pos[i];
+        if (vin && base + i * 32 < n) val[i] = vin[pos[i]];
+    }
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const int idx = base + i * 32;
         if (idx < n) {
             kout[idx] = key[i];
-            vout[idx] = vin ? __ldg(vin + pos[i]) : (int)pos[i];
+            vout[idx] = val[i];
         }
     }
 }

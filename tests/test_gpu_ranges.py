@@ -105,13 +105,13 @@ def test_keys_near_grid_points(lo, hi, curve, cuda):
 
 
 # -------------------------------------------------------------------- sort
-def gpu_sort(keys, vals=None):
+def gpu_sort(keys, vals=None, in_place=False):
     dev = torch.device("cuda:0")
     n, L = len(keys), _lib.load()
     kin = torch.as_tensor(keys.view(np.int64), device=dev)
     vin = torch.as_tensor(vals, device=dev) if vals is not None else None
-    kout = torch.zeros(n, dtype=torch.int64, device=dev)
-    vout = torch.zeros(n, dtype=torch.int32, device=dev)
+    kout = kin if in_place else torch.zeros(n, dtype=torch.int64, device=dev)
+    vout = vin if in_place else torch.zeros(n, dtype=torch.int32, device=dev)
     nb = L.mhpc_sort_scratch_bytes(n)
     scratch = torch.zeros(nb, dtype=torch.uint8, device=dev)
     _lib.check(L.mhpc_sort_pairs(dptr(kin), dptr(vin) if vin is not None else None, dptr(kout), dptr(vout), n,
@@ -138,6 +138,20 @@ def test_sort_sizes(n, cuda):
         ks, vs = gpu_sort(keys, vals)
         assert np.array_equal(ks, keys[order])
         assert np.array_equal(vs, order.astype(np.int32) if vals is None else vals[order])
+
+
+@pytest.mark.parametrize("n", [1, 33, 1000, 1024, 1025, 3000, 4096, 4097, 200_001, 600_001])
+def test_sort_in_place(n, cuda):
+    """Keys and values sorted in the arrays they came in, by every form of the
+    sort (a value must be read before its place is written)."""
+    for seed in range(5):
+        rng = np.random.default_rng(seed)
+        keys = rng.integers(0, 2 ** 64 - 1, n, dtype=np.uint64, endpoint=True)
+        vals = rng.permutation(n).astype(np.int32)
+        order = np.argsort(keys, kind="stable")
+        ks, vs = gpu_sort(keys, vals, in_place=True)
+        assert np.array_equal(ks, keys[order])
+        assert np.array_equal(vs, vals[order])
 
 
 def test_sort_scratch_serves_smaller_n(cuda):
