@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
     const double cx = 0.5 * (lox + hix), cy = 0.5 * (loy + hiy), cz = 0.5 * (loz + hiz);
     // the margin of 1e-6 is several times the FP32 roundings of the offsets and
     // squares below (a few 2^-24 each)
-    constexpr float kUp = 1.f + 1e-6f, kDown = 1.f - 1e-6f;
+    constexpr float kUp = 1.f + 1e-6f, kDown = 1.f - 1e-6f, kDpMin = 1e-30f;
     const float bx = kUp * (float)fmax(hix - cx, cx - lox), by = kUp * (float)fmax(hiy - cy, cy - loy),
                 bz = kUp * (float)fmax(hiz - cz, cz - loz), ef = kUp * (float)emax;
     // dp(L) = (radius^2 / theta) * 0.25^(L-1); powers of two scale exactly,
@@ -161,8 +161,12 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
                 const float z0 = fmaxf(fmaf(kDown, nz, -bz), 0.f), z1 = fmaf(kUp, nz, bz);
                 const float near2 = fmaf(x0, x0, fmaf(y0, y0, z0 * z0));
                 const float far2 = fmaf(x1, x1, fmaf(y1, y1, fmaf(z1, z1, ef)));
-                acc = near2 * kDown > __double2float_ru(dp);
-                open = far2 * kUp < __double2float_rd(dp);
+                // (below 1e-30 the squares near FP32's subnormals carry more than the
+                // margin: the vote decides; above its range they are infinite, and
+                // neither comparison holds unless it is true)
+                const float dlow = __double2float_rd(dp);
+                acc = dlow >= kDpMin && near2 * kDown > __double2float_ru(dp);
+                open = dlow >= kDpMin && far2 * kUp < dlow;
                 vote = !acc && !open;
             }
         }

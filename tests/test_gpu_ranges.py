@@ -69,6 +69,24 @@ def test_v2_walk_shared_keys(n, cuda):
     sim.close()
 
 
+@pytest.mark.parametrize("k", [-90, -76, -73, -70, -66, -56, -40, 40, 66, 90])
+def test_v2_walk_scales(k, cuda):
+    """A system scaled by 2^k (every product of the walk scales exactly in FP64)
+    has the same interactions, and its accelerations scale by 2^-2k: the cells
+    that FP32 decides, and those it must leave to the vote because squares of
+    their distances are below or above FP32's normal range."""
+    n, s = 20_000, 2.0 ** k
+    P = ics.plummer(n, seed=5)
+    out = []
+    for f in (1.0, s):
+        sim = Miluphpc(gravity_cfg(sfc=1, theta=0.5, smoothing=1e-4 * f * f), {**P, **{c: P[c] * f for c in "xyz"}})
+        sim.rhs(0)
+        out.append((sim.stats()["gravity_interactions"], [sim.numpy(c) * f * f for c in ("g_ax", "g_ay", "g_az")]))
+        sim.close()
+    assert out[0][0] == out[1][0]
+    assert rel_err(*out[1][1], *out[0][1]).max() < 1e-12
+
+
 # -------------------------------------------------------------------- keys
 def box_keys(x, y, z, lo, hi, curve):
     dev = torch.device("cuda:0")
