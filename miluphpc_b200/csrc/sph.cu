@@ -24,8 +24,16 @@ constexpr int kSmall = 16;
 // Gap between consecutive particles, in h, at which a group is cut.  Variable h
 // of a 2^20 cloud in us, uncut / 2 / 1.5 / 1 / 0.7: 3870 / 3600 / 3440 / 3390 /
 // 3400; list walk of a 35,937 lattice 95 / 95 / 107 / 115 / 212, of larger lattices
-// the same from 1 on.
-constexpr double kCut = 1.5;
+// the same from 1 on.  Where h is no longer than the spacing every gap is longer
+// than that: a cut must also be kCutMean times the mean of the group's other gaps,
+// and while there are more than kMaxCuts the gap asked for is doubled.  List walk
+// in us, uncut / 1.5 h alone / now: lattice of 262,144 at h = 0.4 and 1 spacings 48 /
+// 633 / 59 and 71 / 96 / 89, of 1,000,000 at 0.4 1814 / 2543 / 243, uniform ball of
+// 1,000,000 at 0.4 and 2 neighbours 10600 / 1846 / 440 and 10300 / 815 / 634.  (Means
+// times 2.5: 66 us at 262,144, 0.4; times 4: a Plummer sphere of 20,000 in groups of
+// 8 stays uncut, 316 against 48.  2 cuts: 100,000 at 60 neighbours 176 against 167.)
+constexpr double kCut = 1.5, kCutMean = 3.0;
+constexpr int kMaxCuts = 3;
 
 // ------------------------------------------------------------ FRNN walk
 // One warp per 32 consecutive (sorted or listed) particles, lane = particle,
@@ -131,7 +139,22 @@ __global__ void __launch_bounds__(kBlock, MHPC_FRNN_MIN_BLOCKS) k_frnn(TreeDev T
         const double nz = __shfl_down_sync(MHPC_FULL, pz, 1);
         const bool next = lane < 31 && ((rest >> (lane + 1)) & 1u);
         const double gap = fmax(fmax(fabs(nx - px), fabs(ny - py)), fabs(nz - pz));
-        cuts = __ballot_sync(MHPC_FULL, next && gap > kCut * hm);
+        double far = kCut * hm;
+        cuts = __ballot_sync(MHPC_FULL, next && gap > far);
+        if (cuts) {
+            float sum = next ? (float)gap : 0.f, top = sum;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sum += __shfl_xor_sync(MHPC_FULL, sum, o);
+                top = fmaxf(top, __shfl_xor_sync(MHPC_FULL, top, o));
+            }
+            far = fmax(far, kCutMean * (double)((sum - top) / (float)max(__popc(rest) - 2, 1)));
+            cuts = __ballot_sync(MHPC_FULL, next && gap > far);
+            for (int k = 0; __popc(cuts) > kMaxCuts; ++k) {
+                far *= 2.0;
+                cuts = k < 10 ? __ballot_sync(MHPC_FULL, next && gap > far) : 0u;
+            }
+        }
     }
     while (rest) {
     const unsigned after = cuts & ~((1u << (__ffs(rest) - 1)) - 1u);

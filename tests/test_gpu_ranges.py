@@ -278,6 +278,63 @@ def test_neighbour_lists_scales(scale, offset, avg_h, cuda):
     sim.close()
 
 
+def sparse_state(nside, spacings, jitter=0.3, seed=3):
+    """Jittered lattice with h of `spacings` lattice spacings, for EOS 0."""
+    S = ics.sedov(nside=nside, seed=seed, jitter=jitter)
+    n = nside ** 3
+    return dict({k: S[k] for k in ("x", "y", "z")}, sml=np.full(n, spacings / nside), mass=np.full(n, 1.0 / n),
+                e=np.ones(n), rho=np.ones(n), p=np.ones(n), cs=np.ones(n), **{f: np.zeros(n) for f in ("vx", "vy", "vz")})
+
+
+@pytest.mark.parametrize("nside,spacings", [(16, 0.0)] + [(k, f) for k in (16, 33, 41) for f in (0.3, 0.8, 1.2)])
+def test_neighbour_lists_sparse(nside, spacings, cuda):
+    """Lists where h is about the spacing or less (every gap between consecutive
+    particles is longer than the cut in h; groups of 8, 16 and 32) equal the
+    brute-force sets."""
+    S, n = sparse_state(nside, spacings), nside ** 3
+    if spacings == 0.0:
+        S["sml"][:] = 1e-300
+    sim = Miluphpc(sph_cfg(integrate_energy=0, max_num_interactions=64), S,
+                   materials=[material(interactions=60, eos_type=0, K=1.0, gamma=1.0)], want_nnl=True)
+    sp = ctypes.byref(sim.soa)
+    for f in ("tree_build", "com"):
+        _lib.check(getattr(sim.L, "mhpc_" + f)(sim.ctx, sp), f)
+    _lib.check(sim.L.mhpc_frnn(sim.ctx, sp, 0, 0), "frnn")
+    _lib.check(sim.L.mhpc_forces(sim.ctx, sp), "forces")
+    off, nbr = O.frnn(S["x"], S["y"], S["z"], S["sml"])
+    noi = sim.numpy("noi")
+    assert np.array_equal(noi, np.diff(off))
+    nnl = np.sort(np.where(np.arange(64) < noi[:, None], sim.t["nnl"].cpu().numpy().reshape(n, 64), n), axis=1)
+    want = np.full((n, 64), n)
+    want[np.arange(64) < noi[:, None]] = nbr
+    assert np.array_equal(nnl, want)
+    sim.close()
+
+
+def test_neighbour_walk_sparse_time(cuda):
+    """The walk of a lattice whose h is below its spacing costs no more than
+    twice the one whose h reaches the next neighbours (a group cut at every
+    particle walks 32 times: 6.6 times the cost)."""
+    us = []
+    for spacings in (0.4, 1.0):
+        sim = Miluphpc(sph_cfg(integrate_energy=0, max_num_interactions=64), sparse_state(64, spacings, jitter=1e-3),
+                       materials=[material(interactions=60, eos_type=0, K=1.0, gamma=1.0)])
+        sp = ctypes.byref(sim.soa)
+        for f in ("tree_build", "com"):
+            _lib.check(getattr(sim.L, "mhpc_" + f)(sim.ctx, sp), f)
+        t = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            _lib.check(sim.L.mhpc_frnn(sim.ctx, sp, 0, 0), "frnn")
+            b.record()
+            torch.cuda.synchronize()
+            t.append(a.elapsed_time(b) * 1e3)
+        us.append(min(t[2:]))
+        sim.close()
+    assert us[0] < 2.0 * us[1], us
+
+
 # 8 particles per warp up to 25,000, 16 up to 65,000, then 32
 @pytest.mark.parametrize("n", [25_000, 25_001, 65_000, 65_001])
 def test_neighbour_counts_group_sizes(n, cuda):
