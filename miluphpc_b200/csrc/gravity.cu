@@ -1,11 +1,13 @@
 // Barnes-Hut gravity walks.
 //
-// Both walks give one warp to 32 consecutive particles of the sorted order,
-// exactly the grouping of the reference's computeForces_v2
-// (src/gravity/gravity.cu:726-903, launched 256x256 with warps taking
-// consecutive `sorted` entries).  The tree is in depth-first pre-order with a
-// skip pointer per node, so the walk needs no stack: accepting a node jumps
-// to its skip pointer, opening it steps to node+1.
+// The plain v2 walk and the mixed list walk take a group of consecutive sorted
+// particles (32 for v2, exactly the grouping of the reference's
+// computeForces_v2, src/gravity/gravity.cu:726-903, launched 256x256 with warps
+// taking consecutive `sorted` entries; 64 for the lists) through the tree
+// together, lane-parallel over a stack of nodes in shared memory.  The v1 walk
+// (one thread per particle) and the per-lane vote walk use the depth-first
+// pre-order and the skip pointers of the tree instead and need no stack:
+// accepting a node jumps to its skip pointer, opening it steps to node + 1.
 #include "gravity.cuh"
 
 namespace {
@@ -772,11 +774,18 @@ constexpr float kRelFloor = 0.1f;
 //   4 warps           43      127      209       301       883   1923   3984
 //   4, leaf queue     33      102                256       796   1768   3650   28029
 // (For one warp a queue of leaves saved a fifth of the steps and no time: 23813.)
-constexpr long kTeamGroups = 148 * 112;
-// Resident blocks per SM the list walk is compiled for: 5 (96 registers, no
-// spills in the force walk) measured 3 % faster at 16.7 M than the
-// unconstrained 116 registers (4 blocks); 6 blocks (80 registers) spill and
-// run 1-2 % slower than 4.
+// With the geometric rule (also every potential) the lists are longer and the
+// team's barriers cost more than they share from about 650,000 on.  Geometric
+// walk / potential in us, Plummer, 1 warp: 400,000 1603 / 2318, 600,000 2277 / 3287,
+// 800,000 2955 / 4163, 1,060,864 3927 / 5455; 4 warps 1495 / 2225, 2250 / 3250,
+// 3025 / 4259, 4057 / 5621.  (A uniform cloud's geometric walk gains up to 1,060,864:
+// 2220 -> 2083 at 800,000; the line keeps both at one warp's time or less.)
+constexpr long kTeamGroups = 148 * 112, kTeamGroupsGeometric = 148 * 64;
+// Resident blocks per SM the list walk is compiled for: 5 (96 registers) measured
+// 3 % faster at 16.7 M than the unconstrained 116 registers (4 blocks); 6 blocks
+// (80 registers) spill and run 1-2 % slower than 4.  At 96 registers the relative
+// rule without guard has no spills in either form; the team spills 72 bytes with
+// the geometric rule and 92 to 96 with the guard, one warp 12 to 16 with the guard.
 #ifndef MHPC_LISTS_MIN_BLOCKS
 #define MHPC_LISTS_MIN_BLOCKS 5
 #endif
@@ -1178,11 +1187,11 @@ int gravity_lists(const TreeDev& T, const GravParams& P, const double* sx, const
                   cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
     const long groups = ((long)P.n + kListGroup - 1) / kListGroup;
-    const bool team = groups <= kTeamGroups;
-    const long blocks = team ? groups : (groups * 32 + kListBlock - 1) / kListBlock;
     // the self-interaction has R = 0 and r^2 = eps2: 1/r^3 stays finite in
     // FP32 for eps2 >= 1e-20
     const bool guard = !(P.eps2 >= 1e-20) && !(P.h_factor > 0.0), rel = P.rel_alpha > 0.0;
+    const bool team = groups <= (rel && !P.pot ? kTeamGroups : kTeamGroupsGeometric);
+    const long blocks = team ? groups : (groups * 32 + kListBlock - 1) / kListBlock;
 #define MHPC_LISTS(G_, R_, P_)                                                                                     \
     do {                                                                                                           \
         if (team)                                                                                                  \

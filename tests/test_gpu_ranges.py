@@ -206,6 +206,58 @@ def test_upward_pass_sizes(n, precision, cuda):
     sim.close()
 
 
+# ------------------------------------------------------------------ list walk
+# teams of four warps up to 606,208 particles (relative rule: 1,060,864), then one
+# warp a group; above 2,000,000 the records have no mask of leaf slots
+@pytest.mark.parametrize("n,mac,eps2", [(606_208, 0, 1e-4), (606_209, 0, 1e-4), (606_209, 0, 0.0),
+                                        (1_060_864, 1, 1e-4), (1_060_865, 1, 1e-4), (1_060_865, 1, 0.0),
+                                        (2_000_001, 0, 1e-4), (2_000_001, 1, 1e-4)])
+def test_list_walk_sizes(n, mac, eps2, cuda):
+    """The list walk on either side of its lines, relative and geometric rule,
+    guarded (eps2 = 0) or not: p99 <= 1e-3 of the direct sum, and (eps2 > 0)
+    close to the FP64 statement of the same rule with the same interactions;
+    bars as for 131,072 particles in the parity tests."""
+    P = ics.plummer(n, seed=1)
+    sim = Miluphpc(gravity_cfg(sfc=1, precision=1, theta_mixed=0.28, smoothing=eps2, gravity_mac=mac, mac_alpha=3e-3), P)
+    sim.rhs(0)
+    prev = np.sqrt(sum(sim.numpy(f) ** 2 for f in ("g_ax", "g_ay", "g_az")))
+    if mac:
+        sim.rhs(1)
+    g = [sim.numpy(f) for f in ("g_ax", "g_ay", "g_az")]
+    tg = np.random.default_rng(7).choice(n, 512, replace=False).astype(np.int32)
+    d = O.direct(P["x"], P["y"], P["z"], P["mass"], tg, eps2)[:3]
+    assert np.percentile(rel_err(*(c[tg] for c in g), *d), 99) <= 1e-3
+    if eps2 > 0:
+        bb = O.bbox(P["x"], P["y"], P["z"])
+        T = O.Tree(P["x"], P["y"], P["z"], P["mass"], bb)
+        q = O.quad(T)
+        _, perm = O.sort(O.keys(P["x"], P["y"], P["z"], bb, 1))
+        radius = 0.5 * (bb[1] - bb[0])
+        if mac:
+            *o, cnt, nq = O.gravity_boxes_rel(T, perm, radius, 1.0, eps2, q, prev, 3e-3, 3)
+        else:
+            *o, cnt, nq = O.gravity_boxes(T, perm, radius, 0.28, eps2, q, gsize=64, nsub=8)
+        assert np.percentile(rel_err(*g, *o), 99) < 2e-4
+        st = sim.stats()
+        assert abs(st["gravity_interactions"] / cnt.sum() - 1.0) < (3e-3 if mac else 1e-3)
+        assert abs(st["gravity_quad_interactions"] / nq.sum() - 1.0) < (1e-2 if mac else 1e-3)
+    sim.close()
+
+
+@pytest.mark.parametrize("n", [606_208, 606_209])
+def test_potential_walk_sizes(n, cuda):
+    """Potentials of both forms of the list walk against the direct sum."""
+    P = ics.plummer(n, seed=11)
+    sim = Miluphpc(gravity_cfg(sfc=1, precision=1, theta_mixed=0.3, smoothing=1e-4), P)
+    w, pot = sim.potential(per_particle=True)
+    pot = pot.cpu().numpy()
+    tg = np.arange(0, n, n // 512).astype(np.int32)
+    ref = O.direct(P["x"], P["y"], P["z"], P["mass"], tg, 1e-4)[3]
+    assert np.percentile(np.abs(pot[tg] / ref - 1.0), 99) < 1e-3
+    assert abs(w - 0.5 * np.sum(P["mass"] * pot)) <= 1e-12 * abs(w)
+    sim.close()
+
+
 # --------------------------------------------------------------- pair sums
 # 4 lanes per particle up to 65,536, then 2 (FP32 density: 1 above 500,000)
 @pytest.mark.parametrize("nside", [9, 40, 41])
