@@ -673,7 +673,7 @@ __device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, C
         const int i = atomicAdd(&nhand, 1);
         if (i < kUpHand) {
             hand[i] = p;
-        } else {  // queue full (not reached for kUpChunk particles): hand off at once
+        } else {  // queue full (a shared-key run longer than the range): hand off at once
             fence_acq_rel();
             hand_off(T, p, combine);
         }

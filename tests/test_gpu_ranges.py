@@ -191,8 +191,6 @@ def test_upward_pass_sizes(n, precision, cuda):
     """The cells' masses and centres of mass are bit-equal to the oracle's
     (Lebesgue order: the same sums; compared as sorted lists, the numbering
     differs), whatever the block sizes."""
-    if precision and n > 300_000:
-        pytest.skip("the block sizes are the same")
     P = ics.plummer(n, seed=12) if n > 1 else {k: np.array([0.5]) for k in ("x", "y", "z", "mass", "vx", "vy", "vz")}
     sim = Miluphpc(gravity_cfg(sfc=0, precision=precision, theta_mixed=0.3), P)
     sim.rhs(0)
@@ -203,6 +201,51 @@ def test_upward_pass_sizes(n, precision, cuda):
     assert c == T.nodes - n
     for k in ("m", "x", "y", "z"):
         assert np.array_equal(np.sort(tr[k][n:n + c]), np.sort(getattr(T, k)[n:n + c])), k
+    sim.close()
+
+
+# a block's range is 1024 sorted particles up to 8,192 and from 200,001 on, 2048 above
+# 2,000,000; its queue of hand-offs holds 1024
+@pytest.mark.parametrize("n", [8_000, 300_001, 2_000_001])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_upward_pass_runs_longer_than_a_block(n, precision, cuda):
+    """Runs of identical positions longer than a block's range: a block inside one
+    hands off every particle of its range, more than its queue holds.  Masses are
+    equal powers of two and coordinates multiples of 2^-26, so the sums over a
+    cell's particles (those with its prefix) are exact: masses equal, centres of
+    mass within the roundings of a bucket's 2600 sums, 2600 * 2^-53 * 16 = 5e-12."""
+    P = ics.plummer(n, seed=31)
+    P["mass"] = np.full(n, 2.0 ** -22)
+    for k in "xyz":
+        P[k] = np.round(P[k] * 2.0 ** 26) * 2.0 ** -26
+        for a, src in ((200, 100), (3000, 7000)):
+            P[k][a:a + 2600] = P[k][src]
+    sim = Miluphpc(gravity_cfg(sfc=0, precision=precision, theta_mixed=0.3), P)
+    sp = ctypes.byref(sim.soa)
+    _lib.check(sim.L.mhpc_stage_tree(sim.ctx, sp), "stage_tree")
+    _lib.check(sim.L.mhpc_ctx_status(sim.ctx), "status")
+    keys, perm = sim.export_sorted()
+    tr = sim.export_tree()
+    child = tr["child"].reshape(-1, 8)
+    sums = {k: np.concatenate([[0.0], np.cumsum(P[k][perm])]) for k in "xyz"}
+    node, pre = np.zeros(1, dtype=np.int64), np.zeros(1, dtype=np.uint64)
+    cells = longest = 0
+    for level in range(1, 22):
+        ch = child[node].astype(np.int64)
+        r, c = np.nonzero(ch >= n)
+        node, pre = ch[r, c], (pre[r] << np.uint64(3)) | c.astype(np.uint64)
+        if not len(node):
+            break
+        sh = np.uint64(3 * (21 - level))
+        lo = np.searchsorted(keys, pre << sh, side="left")
+        hi = np.searchsorted(keys, (pre << sh) | np.uint64((1 << (3 * (21 - level))) - 1), side="right")
+        assert np.array_equal(tr["m"][node], (hi - lo) * 2.0 ** -22)
+        for k in "xyz":
+            assert np.abs(tr[k][node] - (sums[k][hi] - sums[k][lo]) / (hi - lo)).max() < 5e-12
+        cells += len(node)
+        if level == 21:
+            longest = (hi - lo).max()
+    assert cells == tr["cells"] and longest >= 2600
     sim.close()
 
 
@@ -255,6 +298,70 @@ def test_potential_walk_sizes(n, cuda):
     ref = O.direct(P["x"], P["y"], P["z"], P["mass"], tg, 1e-4)[3]
     assert np.percentile(np.abs(pot[tg] / ref - 1.0), 99) < 1e-3
     assert abs(w - 0.5 * np.sum(P["mass"] * pot)) <= 1e-12 * abs(w)
+    sim.close()
+
+
+# ---------------------------------------------------------- gather by records
+# fields of 192 MiB and more go through records of 4, 8 or 12 doubles: 6,291,456
+# particles of 4 fields, 3,145,728 of 8, 2,097,152 of 12
+@pytest.mark.parametrize("n", [6_291_455, 6_291_456])
+def test_gather_gravity_fields(n, cuda):
+    """x, y, z and mass (4 fields): masses and centres of mass of all cells
+    bit-equal to the oracle's tree, masses all different."""
+    P = ics.plummer(n, seed=12)
+    P["mass"] = np.random.default_rng(1).uniform(0.5, 1.5, n) / n
+    sim = Miluphpc(gravity_cfg(sfc=0), P)
+    _lib.check(sim.L.mhpc_stage_tree(sim.ctx, ctypes.byref(sim.soa)), "stage_tree")
+    _lib.check(sim.L.mhpc_ctx_status(sim.ctx), "status")
+    bb = O.bbox(P["x"], P["y"], P["z"])
+    T = O.Tree(P["x"], P["y"], P["z"], P["mass"], bb)
+    tr = sim.export_tree(T.num_nodes)
+    c = tr["cells"]
+    assert c == T.nodes - n
+    for k in ("m", "x", "y", "z"):
+        assert np.array_equal(np.sort(tr[k][n:n + c]), np.sort(getattr(T, k)[n:n + c])), k
+    sim.close()
+
+
+@pytest.mark.parametrize("fields,nside", [(8, 146), (8, 147), (12, 127), (12, 128)])
+def test_gather_sph_fields(fields, nside, cuda):
+    """x, y, z, mass, h and v (8 fields), and with them e, rho, p and c_s (12
+    fields, two materials by id): every field in its particle's place.  Material
+    1 of the 12 has an equation of state without rules, so its p and c_s come
+    back as they went in; material 0's follow from its e, rho and previous p.
+    Forces of the shuffled lattice within 1e-10 of the oracle's."""
+    n = nside ** 3
+    rng = np.random.default_rng(nside)
+    S = ics.sedov(nside=nside, seed=4, jitter=0.2)
+    order = rng.permutation(n)
+    S = {k: v[order] for k, v in S.items() if isinstance(v, np.ndarray)}
+    S["sml"] = rng.uniform(1.1, 1.3, n) / nside
+    S["mass"] = rng.uniform(0.5, 1.5, n) / n
+    for k in ("vx", "vy", "vz"):
+        S[k] = 0.1 * rng.standard_normal(n)
+    for k in ("e", "rho", "p", "cs"):
+        S[k] = rng.uniform(0.5, 1.5, n)
+    mats = [material(interactions=60, eos_type=3)]
+    if fields == 12:
+        mats = [material(interactions=60, eos_type=9, gamma=1.5), material(interactions=60, eos_type=7)]
+        S["material_id"] = rng.integers(0, 2, n).astype(np.int32)
+    sim = Miluphpc(sph_cfg(integrate_density=int(fields == 12), max_num_interactions=40), S, materials=mats)
+    sim.rhs(0)
+    rho, p, cs = (sim.numpy(k) for k in ("rho", "p", "cs"))
+    off, nbr = O.frnn(S["x"], S["y"], S["z"], S["sml"])
+    assert np.array_equal(sim.numpy("noi"), np.diff(off))
+    if fields == 12:
+        m0 = S["material_id"] == 0
+        assert np.array_equal(rho, S["rho"])
+        assert np.array_equal(p[~m0], S["p"][~m0]) and np.array_equal(cs[~m0], S["cs"][~m0])
+        np.testing.assert_allclose(p[m0], 0.5 * S["rho"][m0] * S["e"][m0], rtol=1e-15)
+        np.testing.assert_allclose(cs[m0], np.sqrt(1.5 * S["p"][m0] / S["rho"][m0]), rtol=1e-15)
+    else:
+        want = O.density(S["x"], S["y"], S["z"], S["mass"], S["sml"], off, nbr)
+        np.testing.assert_allclose(rho, want, rtol=1e-12)
+    f = O.forces(S["x"], S["y"], S["z"], S["vx"], S["vy"], S["vz"], S["mass"], S["sml"], rho, p, cs, off, nbr, 1.0, 2.0)
+    for got, want in zip(("ax", "ay", "az", "drhodt", "dedt"), f):
+        assert np.abs(sim.numpy(got) - want).max() <= 1e-10 * np.abs(want).max(), got
     sim.close()
 
 
