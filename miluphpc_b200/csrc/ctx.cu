@@ -616,7 +616,11 @@ int mhpc_ctx_create(mhpc_ctx** out, int capacity, const mhpc_config* cfg, const 
     if (cfg->sph) {
         A(c->svx, n); A(c->svy, n); A(c->svz, n); A(c->se, n); A(c->srho, n); A(c->sp, n); A(c->scs, n);
         A(c->sbal, n);
-        A(c->ra, 3 * n);  // (one block: also the gather's scratch)
+        // records of the pair sums, one block: also the gather's scratch.  The band
+        // repair's arrays share it (band_h0 with rb, the events, 32 bytes a particle,
+        // with rc): they live within a neighbour search, whose change of h makes the
+        // records stale (rec_form).
+        A(c->ra, 2 * n + std::max<size_t>(1024, n));
         c->rb = c->ra + n;
         c->rc = c->rb + n;
         A(c->smat, n);
@@ -629,9 +633,9 @@ int mhpc_ctx_create(mhpc_ctx** out, int capacity, const mhpc_config* cfg, const 
         // band repair events: a round changes a few pairs per out-of-band particle
         // (room for 4 per particle: a round that needs more is skipped and counted)
         c->band_cap = (int)std::min<size_t>(2147483000, std::max<size_t>(4096, 4 * n));
-        A(c->band_ev, c->band_cap);
+        c->band_ev = reinterpret_cast<int2*>(c->rc);
+        c->band_h0 = reinterpret_cast<double*>(c->rb);
         A(c->band_ctr, kBandCtr);
-        A(c->band_h0, n);
         A(c->nb_appended, n);
     }
     // mhpc_potential: the potential (when the caller passes no buffer) and the

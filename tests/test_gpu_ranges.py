@@ -402,6 +402,22 @@ def test_pair_sums_fp32_large(cuda):
         assert np.abs(a - b).max() <= 2e-5 * np.abs(a).max()
 
 
+def test_sph_context_memory(cuda):
+    """Device memory of an SPH context of 4,000,000 particles with lists of 8:
+    610 bytes a particle before the pair sums had records (96 bytes in place of
+    56), which the arrays of the band repair share.  5 bytes a particle of slack
+    for the allocator's 2 MB pages."""
+    n = 4_000_000
+    cfg = sph_cfg(max_num_interactions=8)
+    mat, ctx = material(), ctypes.c_void_p()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    _lib.check(_lib.load().mhpc_ctx_create(ctypes.byref(ctx), n, ctypes.byref(cfg), ctypes.byref(mat), 1), "create")
+    used = before - torch.cuda.mem_get_info()[0]
+    _lib.check(_lib.load().mhpc_ctx_destroy(ctx), "destroy")
+    assert used <= 615 * n, used / n
+
+
 # ------------------------------------------------------------ neighbour lists
 @pytest.mark.parametrize("avg_h", [0, 1])
 @pytest.mark.parametrize("scale,offset", [(1.0, 0.0), (1e-20, 0.0), (1e-14, 3e-15), (1e20, 0.0), (1.0, 1e6), (1.0, -3e3)])
