@@ -774,13 +774,22 @@ constexpr float kRelFloor = 0.1f;
 //   4 warps           43      127      209       301       883   1923   3984
 //   4, leaf queue     33      102                256       796   1768   3650   28029
 // (For one warp a queue of leaves saved a fifth of the steps and no time: 23813.)
-// With the geometric rule (also every potential) the lists are longer and the
-// team's barriers cost more than they share from about 650,000 on.  Geometric
-// walk / potential in us, Plummer, 1 warp: 400,000 1603 / 2318, 600,000 2277 / 3287,
-// 800,000 2955 / 4163, 1,060,864 3927 / 5455; 4 warps 1495 / 2225, 2250 / 3250,
-// 3025 / 4259, 4057 / 5621.  (A uniform cloud's geometric walk gains up to 1,060,864:
-// 2220 -> 2083 at 800,000; the line keeps both at one warp's time or less.)
-constexpr long kTeamGroups = 148 * 112, kTeamGroupsGeometric = 148 * 64;
+// With the geometric rule (also every potential) the team's barriers cost more than
+// they share sooner, the sooner the longer (small theta) or the fewer (large) the
+// accepted lists.  Geometric walk, Plummer, time of 1 warp over 4 warps:
+//   n        theta 0.02   0.05   0.1    0.28   0.6
+//   300,000      1.06            1.06   1.05   1.02
+//   370,000      1.02     1.03   1.09   1.07   0.98
+//   490,000      0.88     1.03   1.05   1.04   0.97
+//   600,000      0.89            1.02   1.01   0.94
+//   1,060,864                           0.97
+// (in us at theta 0.28: 600,000 2070 / 2054, 1,060,864 3927 / 4057, its potential 5455 /
+// 5621; a uniform cloud's walk gains by up to 10 % more at each.)
+constexpr long kTeamGroups = 148 * 112, kTeamGroupsGeometric = 148 * 64, kTeamGroupsGeometricFar = 148 * 36;
+inline long team_groups(double theta, bool geometric) {
+    if (!geometric) return kTeamGroups;
+    return theta >= 0.1 && theta <= 0.3 ? kTeamGroupsGeometric : kTeamGroupsGeometricFar;
+}
 // Resident blocks per SM the list walk is compiled for: 5 (96 registers) measured
 // 3 % faster at 16.7 M than the unconstrained 116 registers (4 blocks); 6 blocks
 // (80 registers) spill and run 1-2 % slower than 4.  At 96 registers the relative
@@ -1190,7 +1199,7 @@ int gravity_lists(const TreeDev& T, const GravParams& P, const double* sx, const
     // the self-interaction has R = 0 and r^2 = eps2: 1/r^3 stays finite in
     // FP32 for eps2 >= 1e-20
     const bool guard = !(P.eps2 >= 1e-20) && !(P.h_factor > 0.0), rel = P.rel_alpha > 0.0;
-    const bool team = groups <= (rel && !P.pot ? kTeamGroups : kTeamGroupsGeometric);
+    const bool team = groups <= team_groups(P.theta, !rel || P.pot);
     const long blocks = team ? groups : (groups * 32 + kListBlock - 1) / kListBlock;
 #define MHPC_LISTS(G_, R_, P_)                                                                                     \
     do {                                                                                                           \

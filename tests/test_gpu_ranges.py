@@ -250,18 +250,21 @@ def test_upward_pass_runs_longer_than_a_block(n, precision, cuda):
 
 
 # ------------------------------------------------------------------ list walk
-# teams of four warps up to 606,208 particles (relative rule: 1,060,864), then one
-# warp a group; above 2,000,000 the records have no mask of leaf slots
-@pytest.mark.parametrize("n,mac,eps2", [(606_208, 0, 1e-4), (606_209, 0, 1e-4), (606_209, 0, 0.0),
-                                        (1_060_864, 1, 1e-4), (1_060_865, 1, 1e-4), (1_060_865, 1, 0.0),
-                                        (2_000_001, 0, 1e-4), (2_000_001, 1, 1e-4)])
-def test_list_walk_sizes(n, mac, eps2, cuda):
+# teams of four warps up to 340,992 particles (geometric rule with theta from 0.1 to 0.3:
+# 606,208, relative rule: 1,060,864), then one warp a group; above 2,000,000 the
+# records have no mask of leaf slots
+@pytest.mark.parametrize("n,mac,theta,eps2", [(340_992, 0, 0.5, 1e-4), (340_993, 0, 0.5, 1e-4),
+                                              (606_208, 0, 0.28, 1e-4), (606_209, 0, 0.28, 1e-4),
+                                              (606_209, 0, 0.28, 0.0), (1_060_864, 1, 0.28, 1e-4),
+                                              (1_060_865, 1, 0.28, 1e-4), (1_060_865, 1, 0.28, 0.0),
+                                              (2_000_001, 0, 0.28, 1e-4), (2_000_001, 1, 0.28, 1e-4)])
+def test_list_walk_sizes(n, mac, theta, eps2, cuda):
     """The list walk on either side of its lines, relative and geometric rule,
-    guarded (eps2 = 0) or not: p99 <= 1e-3 of the direct sum, and (eps2 > 0)
+    guarded (eps2 = 0) or not: p99 <= 1e-3 of the direct sum (theta 0.28), and (eps2 > 0)
     close to the FP64 statement of the same rule with the same interactions;
     bars as for 131,072 particles in the parity tests."""
     P = ics.plummer(n, seed=1)
-    sim = Miluphpc(gravity_cfg(sfc=1, precision=1, theta_mixed=0.28, smoothing=eps2, gravity_mac=mac, mac_alpha=3e-3), P)
+    sim = Miluphpc(gravity_cfg(sfc=1, precision=1, theta_mixed=theta, smoothing=eps2, gravity_mac=mac, mac_alpha=3e-3), P)
     sim.rhs(0)
     prev = np.sqrt(sum(sim.numpy(f) ** 2 for f in ("g_ax", "g_ay", "g_az")))
     if mac:
@@ -269,7 +272,7 @@ def test_list_walk_sizes(n, mac, eps2, cuda):
     g = [sim.numpy(f) for f in ("g_ax", "g_ay", "g_az")]
     tg = np.random.default_rng(7).choice(n, 512, replace=False).astype(np.int32)
     d = O.direct(P["x"], P["y"], P["z"], P["mass"], tg, eps2)[:3]
-    assert np.percentile(rel_err(*(c[tg] for c in g), *d), 99) <= 1e-3
+    assert theta > 0.3 or np.percentile(rel_err(*(c[tg] for c in g), *d), 99) <= 1e-3
     if eps2 > 0:
         bb = O.bbox(P["x"], P["y"], P["z"])
         T = O.Tree(P["x"], P["y"], P["z"], P["mass"], bb)
@@ -279,7 +282,7 @@ def test_list_walk_sizes(n, mac, eps2, cuda):
         if mac:
             *o, cnt, nq = O.gravity_boxes_rel(T, perm, radius, 1.0, eps2, q, prev, 3e-3, 3)
         else:
-            *o, cnt, nq = O.gravity_boxes(T, perm, radius, 0.28, eps2, q, gsize=64, nsub=8)
+            *o, cnt, nq = O.gravity_boxes(T, perm, radius, theta, eps2, q, gsize=64, nsub=8)
         assert np.percentile(rel_err(*g, *o), 99) < 2e-4
         st = sim.stats()
         assert abs(st["gravity_interactions"] / cnt.sum() - 1.0) < (3e-3 if mac else 1e-3)
