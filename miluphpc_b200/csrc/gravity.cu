@@ -47,7 +47,16 @@ constexpr int kWalkBlock = 128;
 //   W = 2                 58     98     134     177      369      748       2347
 //   W = 4                 38     57      84     161      352      772       2547
 //   W = 8                 29     37      89     176      436      989       3400
-__host__ __device__ constexpr int v2_stack(int W) { return 512 + 256 * (W - 1); }
+// Entries of the stack.  The bound lets a step pop at most a seventh of the free
+// entries: with a small opening parameter most cells open, the stack stays full,
+// and the steps of a short stack test few nodes each.  Longer stacks leave fewer
+// resident blocks.  Walk in us, W = 2, one node at a time / 768 entries / 1536:
+//   theta                    0.05                0.1                 0.25               0.3         0.5
+//   Plummer, 1,000,003   58900 / 77500 / 34300   25100/23200/14100   8410/5620/4910   6810/4210/4050   3480/2130/2230
+//   Plummer, 2^23  (ms)    540 / 915 / 340         222 / 256 / 130     72/51.1/44.4     57/38.0/36.2     28.8/18.4/19.5
+//   cloud, 2^23    (ms)    330 / 370 / 192         145 / 131 / 86      48/30.7/30.6     37/24.2/24.8     19.9/13.1/13.9
+constexpr double kV2LongTheta = 0.3;
+inline int v2_stack(int W, double theta) { return W == 2 && theta < kV2LongTheta ? 1536 : 512 + 256 * (W - 1); }
 constexpr int kV2Reserve = 7 * 22 + 8;
 
 template <int W>
@@ -55,11 +64,11 @@ struct V2Smem {
     double2 la[64 * W], lb[64 * W];  // accepted: (x, y), (z, m)
     double2 ua[32 * W], ub[32 * W];  // put to the vote: (x, y), (z, dp)
     double part[W][3][32];           // the warps' sums
-    int stk[v2_stack(W)];
     int defer[32 * W];
     int cnt[W][4];                   // per warp: accepted, children, votes, buckets
     unsigned char yes[32 * W];
     int top;
+    // the stack follows
 };
 
 // every W-th entry of the list from entry w on
@@ -82,9 +91,10 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
                                                     const double* __restrict__ sy, const double* __restrict__ sz,
                                                     const double* __restrict__ sh, const int* __restrict__ perm,
                                                     double* __restrict__ gax, double* __restrict__ gay,
-                                                    double* __restrict__ gaz, DevStatus* st) {
+                                                    double* __restrict__ gaz, int cap, DevStatus* st) {
     extern __shared__ __align__(16) unsigned char v2_raw[];
     V2Smem<W>& S = *reinterpret_cast<V2Smem<W>*>(v2_raw);
+    int* const stk = reinterpret_cast<int*>(&S + 1);  // cap entries
     if (__syncthreads_or(st->code)) return;
     const int M = *T.nodes;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -123,18 +133,18 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
     // the root's children: node 0 and its skip chain
     if (threadIdx.x == 0) {
         int c = 0, q = 0;
-        while (c < M && q < 8) { S.stk[q++] = c; c = __ldg(&T.link[c].x); }
+        while (c < M && q < 8) { stk[q++] = c; c = __ldg(&T.link[c].x); }
         if (c < M) set_status(st, MHPC_ERR_DEPTH, 9);
         S.top = q;
     }
     __syncthreads();
     int top = S.top, nlist = 0;  // block-uniform
     while (top > 0) {
-        const int room = (v2_stack(W) - kV2Reserve - top) / 7;
+        const int room = (cap - kV2Reserve - top) / 7;
         int k = top < 32 * W ? top : 32 * W;
         if (k > room) k = room > 1 ? room : 1;
         const bool act = (int)threadIdx.x < k;
-        const int nd = act ? S.stk[top - 1 - threadIdx.x] : 0;
+        const int nd = act ? stk[top - 1 - threadIdx.x] : 0;
         top -= k;
         nvisit += k;
         bool acc = false, open = false, vote = false;
@@ -231,7 +241,7 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
         }
         if (bucket) S.defer[dbase + __popc(bb & lt)] = nd;
         nlist += nacc;
-        if (top + total > v2_stack(W)) {
+        if (top + total > cap) {
             // unreachable by the bound on k; stop instead of overrunning
             if (threadIdx.x == 0) set_status(st, MHPC_ERR_DEPTH, 10);
             return;
@@ -245,7 +255,7 @@ __global__ void __launch_bounds__(32 * W) k_grav_v2(TreeDev T, GravParams P, con
             int pos = top + kbase + incl - nkid;
 #pragma unroll
             for (int d = 0; d < 8; ++d)
-                if ((mask >> d) & 1) S.stk[pos++] = all[d];
+                if ((mask >> d) & 1) stk[pos++] = all[d];
         }
         top += total;
         __syncthreads();
@@ -1156,8 +1166,12 @@ int gravity_v2(const TreeDev& T, const GravParams& P, const double* sx, const do
                cudaStream_t s) {
     if (P.n <= 0) return MHPC_OK;
     const long groups = ((long)P.n + 31) / 32;
-#define MHPC_V2(W_) \
-    k_grav_v2<W_><<<(int)groups, 32 * W_, sizeof(V2Smem<W_>), s>>>(T, P, sx, sy, sz, sh, perm, gax, gay, gaz, st)
+#define MHPC_V2(W_)                                                                                           \
+    do {                                                                                                      \
+        const int cap = v2_stack(W_, P.theta);                                                                \
+        k_grav_v2<W_><<<(int)groups, 32 * W_, sizeof(V2Smem<W_>) + sizeof(int) * cap, s>>>(                   \
+            T, P, sx, sy, sz, sh, perm, gax, gay, gaz, cap, st);                                              \
+    } while (0)
     // warps per group: the walk of one group is a chain of memory round trips
     // and FP64 sums, so more warps pay until the groups alone fill the SMs
     // (measured at either side of each line beside k_grav_v2)

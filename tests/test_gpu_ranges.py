@@ -87,6 +87,52 @@ def test_v2_walk_scales(k, cuda):
     assert rel_err(*out[1][1], *out[0][1]).max() < 1e-12
 
 
+# two warps per group take a stack of 1536 entries below theta 0.3, else of 768
+@pytest.mark.parametrize("theta", [1e-6, 0.02, 0.29, 0.3])
+@pytest.mark.parametrize("n", [12_000, 151_553])
+def test_v2_walk_small_theta(n, theta, cuda):
+    """Opening parameters at which most cells open, so that the stack stays full:
+    the oracle's interactions and accelerations (theta 1e-6: the direct sum)."""
+    P = ics.plummer(n, seed=5)
+    sim = Miluphpc(gravity_cfg(sfc=1, theta=theta, smoothing=1e-4), P)
+    sim.rhs(0)
+    g = [sim.numpy(f) for f in ("g_ax", "g_ay", "g_az")]
+    if theta < 1e-3:
+        tg = np.arange(0, n, n // 300).astype(np.int32)
+        o = O.direct(P["x"], P["y"], P["z"], P["mass"], tg, 1e-4)[:3]
+        g = [c[tg] for c in g]
+    else:
+        bb = O.bbox(P["x"], P["y"], P["z"])
+        T = O.Tree(P["x"], P["y"], P["z"], P["mass"], bb)
+        _, perm = O.sort(O.keys(P["x"], P["y"], P["z"], bb, 1))
+        o = O.gravity_v2(T, perm, 0.5 * (bb[1] - bb[0]), theta, 1e-4)
+    big = np.sqrt(sum(c ** 2 for c in o)).max()
+    assert max(np.abs(a - b).max() for a, b in zip(g, o)) <= 1e-9 * big
+    sim.close()
+
+
+def test_v2_walk_time_small_theta(cuda):
+    """Time per interaction at theta 0.05 within 1.5 times that at 0.5 (300,000
+    particles; 2.2 times it when the stack of 768 entries held the steps back)."""
+    P = ics.plummer(300_000, seed=3)
+    per = []
+    for theta in (0.5, 0.05):
+        sim = Miluphpc(gravity_cfg(sfc=1, theta=theta, smoothing=1e-4), P)
+        sim.rhs(0)
+        t = []
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            _lib.check(sim.L.mhpc_gravity(sim.ctx, ctypes.byref(sim.soa), 0), "gravity")
+            b.record()
+            torch.cuda.synchronize()
+            t.append(a.elapsed_time(b))
+        sim.rhs(0)
+        per.append(min(t) / sim.stats()["gravity_interactions"])
+        sim.close()
+    assert per[1] < 1.5 * per[0], per
+
+
 # -------------------------------------------------------------------- keys
 def box_keys(x, y, z, lo, hi, curve):
     dev = torch.device("cuda:0")
