@@ -795,7 +795,7 @@ constexpr float kRelFloor = 0.1f;
 //   1,060,864                           0.97
 // (in us at theta 0.28: 600,000 2070 / 2054, 1,060,864 3927 / 4057, its potential 5455 /
 // 5621; a uniform cloud's walk gains by up to 10 % more at each.)
-constexpr long kTeamGroups = 148 * 112, kTeamGroupsGeometric = 148 * 64, kTeamGroupsGeometricFar = 148 * 36;
+constexpr long kTeamGroups = kLeafMaskN / kListGroup, kTeamGroupsGeometric = 148 * 64, kTeamGroupsGeometricFar = 148 * 36;
 inline long team_groups(double theta, bool geometric) {
     if (!geometric) return kTeamGroups;
     return theta >= 0.1 && theta <= 0.3 ? kTeamGroupsGeometric : kTeamGroupsGeometricFar;

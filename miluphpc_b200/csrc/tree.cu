@@ -541,14 +541,20 @@ constexpr int kUpHand = 1024;
 // eight lanes, where a cell's time is its round trips: 54 us at 1,000, 57 at 20,011,
 // 68 at 100,003, 148 at 300,000.  (Without them a cell has too little to share:
 // 78 us against 55 at 131,072.)
-// (8 positions, above 2,000,000 particles, leave out the mask of leaf slots: no
-// walk of that size asks for it, and it cost 100 us at 2^24.)
+// Above, the lines lie where a wave of resident blocks (444) ends: 444 ranges of 1024
+// are 454,656 particles, of 2048 909,312.  4 / 8 positions, Plummer with walk records
+// (8 without the leaf mask / with it), cloud with boxes: 400,000 138 / 152 / 160, 87 /
+// 99; 500,000 194 / 162 / 172, 123 / 104; 850,000 236 / 199 / 208, 161 / 139;
+// 1,000,000 278 / 283 / 298, 193 / 207; 1,300,000 323 / 302 / 318, 222 / 224; 2,000,000
+// 458 / 407 / 430, 319 / 305.
+// (The mask of leaf slots costs 4-5 % of the pass, 100 us at 2^24; above kLeafMaskN no
+// walk asks for it.)
 constexpr int kWideN = 200000;
 inline int up_per(int n) {
     if (n <= 8192) return 4;
     if (n <= 65536) return 1;
     if (n <= 200000) return 2;
-    return n <= 2000000 ? 4 : 8;
+    return n <= 454656 || (n > 909312 && n <= kLeafMaskN) ? 4 : 8;
 }
 
 __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
@@ -745,7 +751,7 @@ __device__ __forceinline__ void upward_chunk(const TreeDev& T, Leaf&& leaf_fn, C
     }
 }
 
-template <int kUpPer, bool kWide>
+template <int kUpPer, bool kWide, bool kLeafMask>
 __global__ void __launch_bounds__(kUpBlock, 3) k_upward(TreeDev T, const double* __restrict__ sx,
                                                      const double* __restrict__ sy, const double* __restrict__ sz,
                                                      const double* __restrict__ sm, int want_quad, int want_box,
@@ -756,11 +762,10 @@ __global__ void __launch_bounds__(kUpBlock, 3) k_upward(TreeDev T, const double*
     upward_chunk<kUpPer, kWide>(
         T, [&](int a, int leaf) { leaf_moments(T, a, leaf, sx, sy, sz, sm, want_quad, want_box, edge0, inv_theta); },
         [&](int p, bool local) {
-            cell_moments<kWide ? 1 : 4, (kUpPer < 8)>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta,
-                                                      local);
+            cell_moments<kWide ? 1 : 4, kLeafMask>(T, p, cell_kids(T, p), want_quad, want_box, edge0, inv_theta, local);
         },
         [&](bool act, int p, bool local) {
-            cell_moments_wide<(kUpPer < 8)>(T, act, p, want_quad, want_box, edge0, inv_theta, local);
+            cell_moments_wide<kLeafMask>(T, act, p, want_quad, want_box, edge0, inv_theta, local);
         });
 }
 
@@ -814,17 +819,19 @@ int tree_build(TreeDev& T, const uint64_t* skey, void* scan_scratch, DevStatus* 
 int tree_upward(TreeDev& T, const double* sx, const double* sy, const double* sz, const double* sm,
                 int want_quad, int want_box, const long long* ord, double theta, DevStatus* st, cudaStream_t s) {
     const double inv_theta = want_quad ? 1.0 / theta : 0.0;
-#define MHPC_UP(P_, W_)                                                                                                \
-    k_upward<P_, W_><<<(T.n + P_ * kUpBlock - 1) / (P_ * kUpBlock), kUpBlock, 0, s>>>(T, sx, sy, sz, sm, want_quad, \
+#define MHPC_UP(P_, W_, M_)                                                                                            \
+    k_upward<P_, W_, M_><<<(T.n + P_ * kUpBlock - 1) / (P_ * kUpBlock), kUpBlock, 0, s>>>(T, sx, sy, sz, sm, want_quad, \
                                                                                      want_box, ord, inv_theta, st)
     if (want_quad && T.n <= kWideN) {
-        MHPC_UP(1, true);
+        MHPC_UP(1, true, true);
     } else {
         switch (up_per(T.n)) {
-            case 1: MHPC_UP(1, false); break;
-            case 2: MHPC_UP(2, false); break;
-            case 4: MHPC_UP(4, false); break;
-            default: MHPC_UP(8, false); break;
+            case 1: MHPC_UP(1, false, true); break;
+            case 2: MHPC_UP(2, false, true); break;
+            case 4: MHPC_UP(4, false, true); break;
+            default:
+                if (T.n <= kLeafMaskN) MHPC_UP(8, false, true);
+                else MHPC_UP(8, false, false);
         }
     }
 #undef MHPC_UP

@@ -15,6 +15,9 @@
 
 // info word of nd_link.y: bits 0-7 level, bit 8 leaf flag
 #define ND_LEAF 0x100
+// Largest number of particles whose walk records tell which child slots hold
+// leaves (the list walk's teams, which read it, end there).
+constexpr int kLeafMaskN = 148 * 112 * 64;
 
 struct TreeDev {
     int n;              // particles

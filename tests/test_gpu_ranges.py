@@ -228,10 +228,12 @@ def test_sort_scratch_serves_smaller_n(cuda):
 
 
 # ------------------------------------------------------------- upward pass
-# 4 positions per thread up to 8,192, 1 up to 65,536, 2 up to 200,000, 4 up to 2,000,000,
-# then 8; with walk records (precision 1) eight lanes per cell up to 200,000; nodes are
-# counted in one block up to 16,384
-@pytest.mark.parametrize("n", [1, 2, 5, 8192, 8193, 16_384, 16_385, 65_536, 65_537, 200_000, 200_001, 2_000_001])
+# 4 positions per thread up to 8,192, 1 up to 65,536, 2 up to 200,000, 4 up to 454,656, 8 up to
+# 909,312, 4 up to 1,060,864, then 8; with walk records (precision 1) eight lanes per cell up
+# to 200,000, and no mask of leaf slots above 1,060,864; nodes are counted in one block up
+# to 16,384
+@pytest.mark.parametrize("n", [1, 2, 5, 8192, 8193, 16_384, 16_385, 65_536, 65_537, 200_000, 200_001, 454_656, 454_657,
+                               909_312, 909_313, 1_060_864, 1_060_865, 2_000_001])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_upward_pass_sizes(n, precision, cuda):
     """The cells' masses and centres of mass are bit-equal to the oracle's
@@ -250,9 +252,9 @@ def test_upward_pass_sizes(n, precision, cuda):
     sim.close()
 
 
-# a block's range is 1024 sorted particles up to 8,192 and from 200,001 on, 2048 above
-# 2,000,000; its queue of hand-offs holds 1024
-@pytest.mark.parametrize("n", [8_000, 300_001, 2_000_001])
+# a block's range is 1024 sorted particles up to 8,192 and from 200,001 to 454,656, 2048
+# up to 909,312 and from 1,060,865 on; its queue of hand-offs holds 1024
+@pytest.mark.parametrize("n", [8_000, 20_000, 300_001, 500_001, 2_000_001])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_upward_pass_runs_longer_than_a_block(n, precision, cuda):
     """Runs of identical positions longer than a block's range: a block inside one
@@ -297,7 +299,7 @@ def test_upward_pass_runs_longer_than_a_block(n, precision, cuda):
 
 # ------------------------------------------------------------------ list walk
 # teams of four warps up to 340,992 particles (geometric rule with theta from 0.1 to 0.3:
-# 606,208, relative rule: 1,060,864), then one warp a group; above 2,000,000 the
+# 606,208, relative rule: 1,060,864), then one warp a group; above 1,060,864 the
 # records have no mask of leaf slots
 @pytest.mark.parametrize("n,mac,theta,eps2", [(340_992, 0, 0.5, 1e-4), (340_993, 0, 0.5, 1e-4),
                                               (606_208, 0, 0.28, 1e-4), (606_209, 0, 0.28, 1e-4),
