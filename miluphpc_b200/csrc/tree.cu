@@ -288,11 +288,14 @@ __device__ __forceinline__ void leaf_moments(const TreeDev& T, int a, int leaf, 
 // a load behind each slot's test waits for the one before it.  With `local`
 // the first pass over the children also brings their quadrupoles into L1 for
 // the second.
+// A bucket's particles are summed one after the other too (order), kBucketBatch
+// loads at a time.
 // kLeafMask: the record also tells which slots hold leaves, for the list walk's
 // teams; a walk that finds no such slot takes leaves as nodes.
 template <int kB, bool kLeafMask>
 __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids& K, int want_quad, int want_box,
                                              double edge0, double inv_theta, bool local) {
+    constexpr int kBucketBatch = kB == 1 ? 2 : 4;
     double m = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
     float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
     float4 hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
@@ -309,9 +312,21 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
     const int2 lkp = __ldg(&T.link[p]);
     const int end = lkp.x;
     if (K.mask & 0x100) {
-        for (int c = p + 1; c < end; c = __ldg(&T.link[c].x)) {
-            add_com(ld_up_d4(&T.com[c], local));
-            if (want_box) add_box(ld_up(&T.bmin[c], local), ld_up(&T.bmax[c], local));
+        // a shared-key bucket: its children are the consecutive leaves p + 1 ... end - 1
+        for (int c0 = p + 1; c0 < end; c0 += kBucketBatch) {
+            double4 cc[kBucketBatch];
+#pragma unroll
+            for (int k = 0; k < kBucketBatch; ++k) cc[k] = ld_up_d4(&T.com[min(c0 + k, end - 1)], local);
+#pragma unroll
+            for (int k = 0; k < kBucketBatch; ++k)
+                if (c0 + k < end) add_com(cc[k]);
+            if (want_box) {
+#pragma unroll
+                for (int k = 0; k < kBucketBatch; ++k) {
+                    const int c = min(c0 + k, end - 1);
+                    add_box(ld_up(&T.bmin[c], local), ld_up(&T.bmax[c], local));
+                }
+            }
         }
     } else {
 #pragma unroll
@@ -372,9 +387,15 @@ __device__ __forceinline__ void cell_moments(const TreeDev& T, int p, const Kids
             }
         };
         if (K.mask & 0x100) {
-            for (int c = p + 1; c < end; c = __ldg(&T.link[c].x))
-                add_quad(ld_up_d4(&T.com[c], local), ld_up(T.wrec + 4 * (size_t)c + 2, local),
-                         ld_up(T.wrec + 4 * (size_t)c + 3, local));
+            const float4 leaf = make_float4(0.f, 0.f, __int_as_float(ND_LEAF), 0.f);
+            for (int c0 = p + 1; c0 < end; c0 += kBucketBatch) {
+                double4 cc[kBucketBatch];
+#pragma unroll
+                for (int k = 0; k < kBucketBatch; ++k) cc[k] = ld_up_d4(&T.com[min(c0 + k, end - 1)], local);
+#pragma unroll
+                for (int k = 0; k < kBucketBatch; ++k)
+                    if (c0 + k < end) add_quad(cc[k], leaf, leaf);
+            }
         } else {
             constexpr int kQ = kB > 2 ? kB / 2 : kB;
 #pragma unroll
@@ -781,7 +802,8 @@ __global__ void __launch_bounds__(kUpBlock, 4) k_hmax(TreeDev T, const double* _
             float m = 0.f;
             if (km & 0x100) {
                 const int end = __ldg(&T.link[p].x);
-                for (int c = p + 1; c < end; c = __ldg(&T.link[c].x)) m = fmaxf(m, ld_up(&T.hmax[c], local));
+#pragma unroll 4
+                for (int c = p + 1; c < end; ++c) m = fmaxf(m, ld_up(&T.hmax[c], local));
             } else {
                 const Kids K = cell_kids(T, p);
                 float v[8];
