@@ -39,8 +39,9 @@ constexpr int kWalkBlock = 128;
 // every W-th entry in FP64, and the warps' sums are added at the end.  The
 // stack bound is the list walk's (below): a pop of k nodes pushes at most 8k,
 // and k leaves room for a depth-first descent.
-// Bound: FP64 pipe (20 instructions an entry and warp) and, below ~500
-// groups, the round trips of the traversal.  Walk in us, Plummer theta 0.5:
+// Bound: issue (68 % of the slots at 131,072 particles, FP64 pipe 48 % busy) and the
+// fixed latency of the FP64 chains; below ~500 groups the round trips of the
+// traversal and the barriers.  Walk in us, Plummer theta 0.5:
 //   n                  1,000  4,000  20,011  50,000  131,072  300,000  1,000,000
 //   one node at a time   190               262               800
 //   W = 1                 93    170     223     267      418      793       2326

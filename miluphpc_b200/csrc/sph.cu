@@ -71,8 +71,8 @@ constexpr int kMaxCuts = 3;
 // 1.3e-6 H^2, and a pair farther apart cannot come within that of H^2 while
 // R < 1e5 H.  The walk and the box tests are conservative too, so each
 // neighbour set equals the brute-force set.
-// Bound: issue and fixed latency (58 % of the issue slots, 18 active warps per
-// SM).  List walk in us with FP64 tests and grown boxes / now: Sedov lattice of
+// Bound: issue (64 to 72 % of the slots, ALU pipe 52 to 58 %) and fixed latency, 23
+// warps active of the 28 resident per SM.  List walk in us with FP64 tests and grown boxes / now: Sedov lattice of
 // 262,144 particles 258 / 203, of 2,097,152 1693 / 1303; all walks of a cloud step,
 // 2^20 particles 2229 / 1500, 2^23 16600 / 10500.  Of the 1303: the tree walk 334,
 // staging the candidates 180, pair tests and list writes 790.
@@ -523,9 +523,9 @@ __global__ void k_vh_init(int n, const double* __restrict__ h, double* hnew, int
 // End of a sweep on lists: every iterating particle takes its new h, and the
 // particles that have not stopped form the next list (in any order: every
 // particle's update and pair edits depend on it alone, and the appended lists
-// are sorted at the end); the lists are re-walked when they are truncated (a
-// count above maxnb) or when the sweep's pair changes overflowed the event
-// buffer (nothing was edited).
+// are sorted at the end); the lists are re-walked once a count was above maxnb
+// (ctr[2] stays set: every sweep from then on) or when the sweep's pair changes
+// overflowed the event buffer (nothing was edited).
 __global__ void k_vh_commit(const int* __restrict__ list, const int* __restrict__ list_count,
                             const double* __restrict__ hnew, double* h, const int* __restrict__ done, int* next,
                             int* next_count, int* ctr) {

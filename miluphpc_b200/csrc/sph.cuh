@@ -144,9 +144,12 @@ int sph_apply_h_changes(const TreeDev& T, const SphParams& P, const double* x, c
 // after each sweep the pairs changed by the new h are edited into the lists
 // (sph_apply_h_changes), so the next sweep's counts are exact without a walk,
 // and the lists at the end are those of the final h (the list walk of the
-// right-hand side is not needed).  Lists that pass maxnb during the
-// iteration, or an event-buffer overflow, fall back to a full list walk after
-// that sweep.  Uses B.hnew and B.ctr[0..3]; T.hmax stays an upper bound
+// right-hand side is not needed).  An event-buffer overflow falls back to a
+// full list walk after that sweep, a list that passes maxnb to one after that
+// and every later sweep: such an iteration moves many h far, and its walks cost
+// less than its pair edits (2^20 cloud started at 1.6 / 2.2 / 3 times its h: 13.4 / 17.1 /
+// 23.5 ms; with the edits back once all lists fit again 20.8 / 24.3 / 36.7).
+// Uses B.hnew and B.ctr[0..3]; T.hmax stays an upper bound
 // (grow-only) of the current h.  Without sort_lists the lists with appends stay
 // marked and unsorted (sph_band_fixup, run next, sorts them with its own).
 int sph_variable_h_lists(const TreeDev& T, const SphParams& P, const double* x, const double* y, const double* z,

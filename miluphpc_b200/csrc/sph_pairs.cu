@@ -421,6 +421,10 @@ __global__ void __launch_bounds__(kBlock) k_balsara(SphParams P, SphSorted S, co
 // and, in FP64, the roots and divisions.  Density / forces in us, Sedov lattice,
 // with one array per field and every division in the loop, and now: 262,144
 // particles FP64 185 / 497 -> 113 / 291; 2,097,152 FP32 773 / 1271 -> 494 / 909.
+// The records and the lanes per particle need neighbours to pay for: from 17 on
+// density and forces together are faster throughout, with 6 (h = 1.3 spacings) up to a
+// fifth slower (2,097,152 FP64: cubic spline 500 -> 431, with h_bar 511 -> 555, Wendland
+// C2 498 -> 604).
 template <bool MIXED, int KERNEL, bool AVG, int T>
 __global__ void __launch_bounds__(kBlock) k_forces(SphParams P, SphSorted S, const int* __restrict__ nbr,
                                                    const int* __restrict__ noi, const int* __restrict__ perm,

@@ -698,10 +698,10 @@ def test_coincident_particles(cuda):
 
 @pytest.mark.parametrize("precision", [0, 1])
 def test_upward_pass_long_shared_key_runs(precision, cuda):
-    """Three runs of 2600 identical positions: each shared-key bucket spans more
-    than one block's range of 2048 sorted particles, so the one-launch upward
-    pass completes it by counted hand-offs from several blocks, and a block
-    inside the run queues more hand-offs than its shared-memory queue holds.
+    """Three runs of 2600 identical positions: each shared-key bucket spans many
+    blocks' ranges of 256 sorted particles, so the one-launch upward pass
+    completes it by counted hand-offs from several blocks (ranges of 1024 and
+    2048, whose hand-offs overflow a block's queue, in the range tests).
     Every cell's mass and centre of mass equal the sums over its particles
     (contiguous in sorted order: the keys with the cell's prefix)."""
     n = 24_000
